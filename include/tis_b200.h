@@ -190,7 +190,9 @@ typedef struct tis_params {
   int32_t launch_threads;          /* threads per CTA: 128, 256, 512, or 1024 (mixed, one CTA per replica) */
   int32_t launch_group;            /* threads per bead in the force gather: 1, 2, 4 or 8 */
   int32_t launch_ctas;             /* CTAs per replica: 1, or 2 (a cluster: mixed precision, 512 threads,
-                                      no periodic box, no Ewald, >= 64 beads) */
+                                      no periodic box, no Ewald, >= 64 beads); 4, 8 or 16: the replica's
+                                      beads and items split over that many (any precision and box), which
+                                      the library also chooses by itself (2 to 16) where that is faster */
   int32_t launch_noise_sweep;      /* two CTAs: 1 draws the noise in the bonded sweep, 2 in the update */
   int32_t launch_order;            /* 1: replicas launched in context order, 2: largest first */
   const char *launch_table;        /* NULL: tuned_launch.tsv next to the library */
@@ -211,7 +213,8 @@ typedef struct tis_status_t {
   int32_t last_error;              /* last TIS_E_* returned */
   int32_t exv_pairs_max;           /* largest exv half list among replicas */
   int32_t ele_pairs_max;           /* largest ele half list among replicas */
-  int32_t ctas_per_lane;           /* CTAs (one cluster) that tis_step gives each replica: 1 or 2 */
+  int32_t ctas_per_lane;           /* 2: pairs of CTAs that each hold the whole replica (launch_ctas 2);
+                                      1: one CTA, or replicas split over larger clusters */
   int32_t threads_per_cta;         /* the launch configuration in use (see tis_params.launch_*) */
   int32_t group;                   /* threads per bead in the force gather, 0: per-replica rule */
   int32_t noise_sweep;

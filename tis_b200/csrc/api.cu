@@ -24,6 +24,7 @@
 
 #include "../../include/tis_b200.h"
 #include "common.cuh"
+#include "split_plan.cuh"
 
 namespace tis {
 size_t smem_bytes_host(int N, int nq, int nslot, int ninc, bool periodic, bool skin, int real_size, int nunit,
@@ -33,6 +34,14 @@ cudaError_t lane_kernel_launch_pair(int nlane, size_t smem, cudaStream_t st, con
 size_t smem_base_host(int N, int nq, int nslot, int ninc, bool periodic, bool skin, int real_size, int nunit,
                       bool dbuf);
 cudaError_t lane_kernel_launch(bool mixed, int grid, int block, size_t smem, cudaStream_t st, const KArgs &a);
+cudaError_t split_setup_mixed(int nsplit, int nt, size_t smem, int *clusters);
+cudaError_t split_launch_mixed(int nlane, int nt, size_t smem, cudaStream_t st, const KArgs &a);
+cudaError_t split_setup_fp64(int nsplit, int nt, size_t smem, int *clusters);
+cudaError_t split_launch_fp64(int nlane, int nt, size_t smem, cudaStream_t st, const KArgs &a);
+cudaError_t split_setup_mixed_box(int nsplit, int nt, size_t smem, int *clusters);
+cudaError_t split_launch_mixed_box(int nlane, int nt, size_t smem, cudaStream_t st, const KArgs &a);
+cudaError_t split_setup_fp64_box(int nsplit, int nt, size_t smem, int *clusters);
+cudaError_t split_launch_fp64_box(int nlane, int nt, size_t smem, cudaStream_t st, const KArgs &a);
 cudaError_t energy_kernel_launch(int grid, int max_nmp, cudaStream_t st, const KArgs &a);
 cudaError_t energy_pair_launch(int nlane, int max_nmp, cudaStream_t st, const KArgs &a, const KArgs &b);
 cudaError_t noise_launch(cudaStream_t st, KArgs a, long long istep0, int nstep, double *out);
@@ -165,6 +174,13 @@ struct tis_ctx {
   std::vector<int> h_order;          // launch order of the lanes (order 2: largest first)
   DBuf<int> d_order;
   size_t smem2 = 0;
+  int nsplit = 0, split_nt = 0;      // lanes split over a cluster of nsplit CTAs of split_nt threads (0: none)
+  int split_least = 0, n_split = 0;  // those of at least this many beads: the first n_split of h_order
+  cudaStream_t stream2 = nullptr;    // the other lanes' launches run beside them
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  DBuf<int> slot_pos;
+  SplitPlan sp{};
+  DBuf<unsigned char> split_blob;    // constant shared-memory part of each CTA, per topology
   // tis_run: the recorded period (nstep steps [+ exchange]) and its launches
   cudaGraphExec_t g_exec = nullptr;
   cudaEvent_t g_ev0 = nullptr, g_ev1 = nullptr;   // recorded around the period's steps
@@ -376,6 +392,29 @@ void ewald_table(double L, double alpha, double hmax, std::vector<int8_t> &hv, s
 
 // --------------------------------------------------------------------- init
 namespace {
+// How many clusters of nr CTAs of the split kernel the GPU holds at once (0:
+// none); asked once per process, device and kernel variant (its registers
+// allow one CTA per SM, so neither the threads nor the shared memory of a
+// context change it).
+int split_clusters(int nr, bool mixed, bool periodic) {
+  static std::mutex mu;
+  static std::map<std::array<int, 4>, int> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  const std::array<int, 4> key{dev, nr, mixed, periodic};
+  const auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  auto setup = periodic ? (mixed ? split_setup_mixed_box : split_setup_fp64_box)
+                        : (mixed ? split_setup_mixed : split_setup_fp64);
+  int n = 0, m = 0;
+  if (setup(nr, 256, 227 * 1024, &n) != cudaSuccess || setup(nr, 512, 227 * 1024, &m) != cudaSuccess) {
+    cudaGetLastError();
+    n = m = 0;
+  }
+  return known[key] = std::min(n, m);
+}
+
 // the whole ladder of a context that holds only some of its replicas
 struct Ladder {
   int nall;
@@ -447,6 +486,7 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
   std::vector<int> u_lunit, u_class;
   std::vector<double> rneigh2;
   std::vector<int> bd_idx, ba_idx, st_idx, hb_idx, hb_site, site_val, site_ptr, site_hb, inc_ptr, inc_slot, q_bead;
+  std::vector<int> slot_pos;
   std::vector<double> bd_nat, bd_coef, ba_nat, ba_coef, st_nat, st_coef, hb_nat, hb_coef, hb_nd2;
   std::vector<double> st_hsTm_all;
   std::vector<uint8_t> hb_tert;
@@ -710,9 +750,14 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
       for (int q2 = 0; q2 < 6; ++q2) inc[t.idtrna_hb2mp[6 * b + q2] - 1].push_back(d.slot_hb + 6 * b + q2);
     int ip = (int)inc_slot.size();
     const int ip0 = ip;
+    d.sp0 = (int)slot_pos.size();
+    slot_pos.resize(slot_pos.size() + d.nslot, 0);
     for (int i = 0; i < t.nmp; ++i) {
       inc_ptr.push_back(ip);
-      for (int sl : inc[i]) inc_slot.push_back(sl);
+      for (size_t q = 0; q < inc[i].size(); ++q) {
+        inc_slot.push_back(inc[i][q]);
+        slot_pos[d.sp0 + inc[i][q]] = ip - ip0 + (int)q;
+      }
       ip += (int)inc[i].size();
     }
     inc_ptr.push_back(ip);
@@ -917,19 +962,207 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     c->sweep = cfg.sweep;
     c->launch_source = source;
     c->smem2 = c->pair ? smem2 : 0;
+    // Lanes split over clusters of nr CTAs (split_kernel), unless the caller
+    // or the environment chose a configuration; launch_ctas 4, 8 or 16 asks
+    // for it.  least: the fewest beads of a lane that is split.
+    auto try_split = [&](int nr, int least, bool lists, int &clusters) {
+      TopDesc mx{};   // the largest counts
+      int mq = 0;
+      for (auto &d : c->tops) {
+        if (d.nmp < least) continue;
+        const int own = split_own(d.nmp, nr);
+        d.sp_ninc = 0;
+        for (int r = 0; r < nr; ++r) {
+          const int b0 = std::min(d.nmp, r * own), b1 = std::min(d.nmp, b0 + own);
+          d.sp_ninc = std::max(d.sp_ninc, inc_ptr[d.inc0 + b1] - inc_ptr[d.inc0 + b0]);
+        }
+        mx.nmp = std::max(mx.nmp, d.nmp); mx.nst = std::max(mx.nst, d.nst); mx.nhb = std::max(mx.nhb, d.nhb);
+        mx.nba = std::max(mx.nba, d.nba); mx.nbd = std::max(mx.nbd, d.nbd); mx.nsite = std::max(mx.nsite, d.nsite);
+        mx.nunit = std::max(mx.nunit, d.nunit); mx.sp_ninc = std::max(mx.sp_ninc, d.sp_ninc);
+        if (p.i_ele != TIS_ELE_NONE) mq = std::max(mq, d.nq);
+      }
+      const bool ewald = p.i_ele == TIS_ELE_EWALD;
+      const SplitPlan sp = split_plan(mx, mq, nr, periodic, skin, ewald, real_size, 227 * 1024);
+      // (Debye-Hueckel rows may list every charge; without room for the lists
+      // the kernel reads the rows' bits, ~4x slower)
+      if (sp.total > 227 * 1024 || (lists && !ewald && sp.ecap < (unsigned)sp.rows * mq)) return false;
+      // 256 threads (with twice the registers) while a CTA's warps have a
+      // few work items each, 512 above
+      const int nt = sp.own <= 32 ? 256 : 512;
+      clusters = split_clusters(nr, mixed, periodic);
+      if (clusters < 1) return false;
+      c->nsplit = nr;
+      c->split_nt = nt;
+      c->sp = sp;
+      return true;
+    };
+    if (!c->bdhi && maxN < (periodic ? 2044 : 65532)) {
+      int clusters = 0, best = 0, best_least = 0;
+      if (p.launch_ctas >= 4) {
+        for (int nr = std::min(p.launch_ctas, SPLIT_MAX); nr >= 2 && !best; nr /= 2)
+          if (try_split(nr, 0, false, clusters)) best = nr;
+      } else if (source != 2) {
+        // The split with the least estimated time of a step of the whole
+        // context: nr CTAs for every lane, or for the lanes of a batch that
+        // have at least `least` beads, the others on one CTA beside them.
+        // From timings on B200 (chains of 26 to 1,199 beads, 1 to 64 lanes),
+        // microseconds: a lane on one CTA takes t1(N), on nr CTAs c + w(N) /
+        // nr, and lanes that do not fit at once take turns.  A ladder context
+        // decides for the whole ladder, so a replica moves the same whichever
+        // ranks hold it.
+        auto t1 = [&](double n) {
+          return mixed ? 6.0 + 0.010 * n + (cfg.threads >= 1024 ? 0.8e-4 : 1.3e-4) * n * n : 10.0 + 0.02 * n + 1.9e-4 * n * n;
+        };
+        auto tn = [&](double n, int nr) {
+          const double w = mixed ? 0.010 * n + 1.1e-4 * n * n : 0.02 * n + 1.6e-4 * n * n;
+          return (nr == 16 ? 7.0 : 6.0) + n / 300.0 + w / nr;
+        };
+        const double scale = lad ? (double)lad->nall / nlane : 1.0, sms = std::max(nsm, 1);
+        auto total = [&](int nr, int least, int places) {   // nr 0: every lane on one CTA
+          double work = 0.0, longest = 0.0;
+          int n_split = 0;
+          for (int l = 0; l < nlane; ++l) {
+            const double n = c->lane_nmp[l];
+            const bool sp = nr && c->lane_nmp[l] >= least;
+            const double t = sp ? tn(n, nr) : t1(n);
+            work += t * (sp ? nr : 1);
+            longest = std::max(longest, t);
+            n_split += sp;
+          }
+          if (c->ntop == 1) return longest * std::ceil(nlane * scale / (nr ? places : sms));   // equal lanes: whole rounds
+          const double turns = n_split > places || nlane > sms ? 0.25 * longest : 0.0;
+          return std::max(longest, std::max(work * scale / sms, n_split ? work * n_split / nlane / (places * nr) : 0.0) + turns);
+        };
+        double time = total(0, 0, 0);
+        std::vector<int> from{0};
+        if (c->ntop > 1 && p.i_ele != TIS_ELE_EWALD)
+          for (int n : {150, 240, 320, 450, 600, 800, 1000})
+            if (n > minN && n <= maxN) from.push_back(n);
+        for (int least : from)
+          for (int nr = 16; nr >= 2; nr /= 2) {
+            if (std::max(minN, least) < 4 * nr || !try_split(nr, least, true, clusters)) continue;
+            const double x = total(nr, least, clusters);
+            if (x < time) { time = x; best = nr; best_least = least; }
+          }
+      }
+      c->nsplit = 0;
+      if (best) {
+        try_split(best, best_least, false, clusters);
+        c->split_least = best_least;
+        c->pair = false;
+      }
+    }
     // replicas largest first: a CTA that frees its SM takes the next one
     std::vector<int> order(nlane);
     for (int l = 0; l < nlane; ++l) order[l] = l;
     if (c->order == 2)
       std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return c->lane_nmp[x] > c->lane_nmp[y]; });
+    if (c->nsplit) {   // the split lanes first, then the others
+      std::stable_partition(order.begin(), order.end(), [&](int l) { return c->lane_nmp[l] >= c->split_least; });
+      for (int l = 0; l < nlane; ++l) c->n_split += c->lane_nmp[l] >= c->split_least;
+    }
     c->h_order = order;
+  }
+
+  std::vector<unsigned char> split_blob;
+  if (c->nsplit) {
+    const int nr = c->nsplit;
+    auto build = [&](auto real) {
+      typedef decltype(real) Real;
+      for (auto &d : c->tops) {
+        const SplitPlan &pl = c->sp;
+        const int N = d.nmp, own = split_own(N, nr), OS = pl.own;
+        if (N < c->split_least) continue;
+        std::vector<int> base(SPLIT_MAX + 1, 0);
+        for (int r = 0; r <= nr; ++r) base[r] = inc_ptr[d.inc0 + std::min(N, r * own)] - inc_ptr[d.inc0];
+        d.sp_blob = (long long)split_blob.size();
+        split_blob.resize(split_blob.size() + pl.comm + (size_t)nr * (pl.stat - pl.comm), 0);
+        // CTA and place of slot k of a bead
+        auto word = [&](int k, int bead) {
+          const int r = bead / own;
+          return (uint32_t)r << 24 | (uint32_t)(slot_pos[d.sp0 + k] - base[r]);
+        };
+        unsigned char *B0 = &split_blob[(size_t)d.sp_blob];
+        uint32_t *tcu = (uint32_t *)(B0 + pl.tcu);
+        Real *re = (Real *)(B0 + pl.RE);
+        for (int i = 0; i < N; ++i) {
+          const int b = d.bead0 + i;
+          tcu[i] = (uint32_t)(uint8_t)b_type[b] | (uint32_t)(uint8_t)b_class[b] << 8 | (uint32_t)(uint16_t)b_unit[b] << 16;
+          re[2 * i] = (Real)b_radius[b]; re[2 * i + 1] = (Real)b_eps[b];
+        }
+        if (p.i_ele != TIS_ELE_NONE)
+          for (int k = 0; k < d.nq; ++k) ((int *)(B0 + pl.qb))[k] = q_bead[d.q0 + k];
+        std::memcpy(B0 + pl.base, base.data(), base.size() * sizeof(int));
+        std::memcpy(B0 + pl.rn2, &rneigh2[d.rn0], 8 * (size_t)d.nunit * d.nunit);
+        for (int r = 0; r < nr; ++r) {
+          unsigned char *B = B0 + (size_t)r * (pl.stat - pl.comm);   // offsets from pl.comm on
+          const int lo = std::min(N, r * own), hi = std::min(N, lo + own);
+          double *C = (double *)(B + pl.C);
+          for (int i = lo; i < hi; ++i) {
+            const int b = d.bead0 + i, li = i - lo;
+            C[li] = b_c2[b]; C[OS + li] = b_c3[b]; C[2 * OS + li] = b_c4[b]; C[3 * OS + li] = b_rcmass[b];
+            ((Real *)(B + pl.scr))[li] = (Real)(b_screen[b] * (1.0 + 1.0e-4) + 1.0e-3);
+          }
+          for (int i = lo; i <= hi; ++i) ((int *)(B + pl.iptr))[i - lo] = inc_ptr[d.inc0 + i] - inc_ptr[d.inc0 + lo];
+          for (int k0 = split_share(d.nbd, nr, r), k = k0; k < split_share(d.nbd, nr, r + 1); ++k) {
+            const int *m = &bd_idx[2 * (size_t)(d.bd0 + k)];
+            ((uint32_t *)(B + pl.bdi))[k - k0] = (uint32_t)m[0] | (uint32_t)m[1] << 16;
+            for (int q = 0; q < 2; ++q) ((uint32_t *)(B + pl.bdd))[2 * (k - k0) + q] = word(2 * k + q, m[q]);
+            Real *cf = (Real *)(B + pl.bdc) + 2 * (k - k0);
+            cf[0] = (Real)bd_nat[d.bd0 + k]; cf[1] = (Real)bd_coef[d.bd0 + k];
+          }
+          for (int k0 = split_share(d.nba, nr, r), k = k0; k < split_share(d.nba, nr, r + 1); ++k) {
+            const int *m = &ba_idx[3 * (size_t)(d.ba0 + k)];
+            uint32_t *ix = (uint32_t *)(B + pl.bai) + 2 * (k - k0);
+            ix[0] = (uint32_t)m[0] | (uint32_t)m[1] << 16; ix[1] = (uint32_t)m[2];
+            for (int q = 0; q < 3; ++q) ((uint32_t *)(B + pl.bad))[3 * (k - k0) + q] = word(d.slot_ba + 3 * k + q, m[q]);
+            Real *cf = (Real *)(B + pl.bac) + 2 * (k - k0);
+            cf[0] = (Real)ba_nat[d.ba0 + k]; cf[1] = (Real)ba_coef[d.ba0 + k];
+          }
+          for (int k0 = split_share(d.nst, nr, r), k = k0; k < split_share(d.nst, nr, r + 1); ++k) {
+            const int *m = &st_idx[7 * (size_t)(d.st0 + k)];
+            uint32_t *ix = (uint32_t *)(B + pl.sti) + 4 * (k - k0);
+            for (int q = 0; q < 7; ++q) {
+              ix[q / 2] |= (uint32_t)m[q] << (16 * (q & 1));
+              ((uint32_t *)(B + pl.std_))[7 * (k - k0) + q] = word(d.slot_st + 7 * k + q, m[q]);
+            }
+            Real *cf = (Real *)(B + pl.stc) + 6 * (k - k0);
+            for (int q = 0; q < 3; ++q) {
+              cf[q] = (Real)st_nat[3 * (size_t)(d.st0 + k) + q];
+              cf[3 + q] = (Real)st_coef[3 * (size_t)(d.st0 + k) + q];
+            }
+          }
+          for (int k0 = split_share(d.nhb, nr, r), k = k0; k < split_share(d.nhb, nr, r + 1); ++k) {
+            const int *m = &hb_idx[6 * (size_t)(d.hb0 + k)];
+            uint32_t *ix = (uint32_t *)(B + pl.hbi) + 3 * (k - k0);
+            for (int q = 0; q < 6; ++q) {
+              ix[q / 2] |= (uint32_t)m[q] << (16 * (q & 1));
+              ((uint32_t *)(B + pl.hbd))[6 * (k - k0) + q] = word(d.slot_hb + 6 * k + q, m[q]);
+              const int site = hb_site[6 * (size_t)(d.hb0 + k) + q];
+              ((uint32_t *)(B + pl.hbs))[6 * (k - k0) + q] =
+                  site < 0 ? 0xffffffffu : (uint32_t)site | (uint32_t)std::min(std::max(site_val[d.site0 + site], 0), 254) << 24;
+            }
+            Real *cf = (Real *)(B + pl.hbc) + 13 * (k - k0);
+            for (int q = 0; q < 6; ++q) cf[q] = (Real)hb_nat[6 * (size_t)(d.hb0 + k) + q];
+            for (int q = 0; q < 7; ++q) cf[6 + q] = (Real)hb_coef[7 * (size_t)(d.hb0 + k) + q];
+          }
+        }
+      }
+    };
+    if (p.precision == TIS_PREC_MIXED) build(0.0f);
+    else build(0.0);
   }
 
   // ---- device
   CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   CK(cudaEventCreate(&c->ev0));
   CK(cudaEventCreate(&c->ev1));
-  if (!c->bdhi) CK(lane_kernel_set_smem(p.precision == TIS_PREC_MIXED, (int)smem, (int)c->smem2));
+  if (c->n_split > 0 && c->n_split < nlane) {
+    CK(cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
+  }
+  if (!c->bdhi && c->n_split < nlane) CK(lane_kernel_set_smem(p.precision == TIS_PREC_MIXED, (int)smem, (int)c->smem2));
   CK(c->d_order.upload(c->h_order));
   CK(c->d_tops.upload(c->tops));
   CK(c->d_lanes.upload(c->lanes));
@@ -957,6 +1190,8 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
   if (pmf_on) { CK(c->pmf_e.upload(pmf_e)); CK(c->pmf_f.upload(pmf_f)); }
   CK(c->site_val.upload(site_val)); CK(c->site_ptr.upload(site_ptr)); CK(c->site_hb.upload(site_hb));
   CK(c->inc_ptr.upload(inc_ptr)); CK(c->inc_slot.upload(inc_slot)); CK(c->q_bead.upload(q_bead));
+  CK(c->slot_pos.upload(slot_pos));
+  CK(c->split_blob.upload(split_blob));
   CK(c->lab_Td.upload(lab_T)); CK(c->lab_coef.upload(lab_coef)); CK(c->lab_cdist.upload(lab_cdist));
   CK(c->lab_beta.upload(lab_beta)); CK(c->lab_rele2.upload(lab_rele2));
   CK(c->lab_u0off.upload(lab_u0off)); CK(c->lab_u0.upload(lab_u0));
@@ -1089,7 +1324,7 @@ extern "C" void tis_destroy(tis_ctx *c) {
   c->bd_idx.free(); c->ba_idx.free(); c->st_idx.free(); c->hb_idx.free(); c->hb_site.free();
   c->tst_idx.free(); c->tst_nat.free(); c->tst_coef.free(); c->stx_ptr.free(); c->stx_tst.free();
   c->site_val.free(); c->site_ptr.free(); c->site_hb.free(); c->inc_ptr.free(); c->inc_slot.free();
-  c->q_bead.free();
+  c->q_bead.free(); c->slot_pos.free(); c->split_blob.free();
   c->bd_nat.free(); c->bd_coef.free(); c->ba_nat.free(); c->ba_coef.free(); c->st_nat.free(); c->st_coef.free();
   c->hb_nat.free(); c->hb_coef.free(); c->hb_nd2.free(); c->hb_tert.free(); c->b_qkind.free(); c->lab_zp.free(); c->pmf_e.free(); c->pmf_f.free();
   c->lab_Td.free(); c->lab_coef.free(); c->lab_cdist.free(); c->lab_beta.free(); c->lab_rele2.free();
@@ -1111,6 +1346,9 @@ extern "C" void tis_destroy(tis_ctx *c) {
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->tev0) cudaEventDestroy(c->tev0);
   if (c->tev1) cudaEventDestroy(c->tev1);
+  if (c->ev_fork) cudaEventDestroy(c->ev_fork);
+  if (c->ev_join) cudaEventDestroy(c->ev_join);
+  if (c->stream2) cudaStreamDestroy(c->stream2);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -1313,6 +1551,10 @@ KArgs make_args(tis_ctx *c, int mode, int nsteps, int only_lane) {
   a.lane_nsteps = nullptr;
   a.step_k = 0;
   a.lane_order = (c->order == 2 && only_lane < 0) ? c->d_order.p : nullptr;
+  a.nsplit = c->nsplit;
+  a.slot_pos = c->slot_pos.p;
+  a.split_blob = c->split_blob.p;
+  a.sp = c->sp;
   return a;
 }
 
@@ -1327,10 +1569,37 @@ int ewald_recip(tis_ctx *c, KArgs &a, bool forces) {
   return TIS_OK;
 }
 
+// The lane kernels for every lane, or for a.only_lane.  A batch of which
+// some lanes are split runs them beside the others on a second stream.
 int launch_lane(tis_ctx *c, const KArgs &a) {
-  ++c->launches;
-  CK(lane_kernel_launch(c->par.precision == TIS_PREC_MIXED, a.only_lane >= 0 ? 1 : a.nlane, c->threads, c->smem,
-                        c->stream, a));
+  const bool mixed = c->par.precision == TIS_PREC_MIXED;
+  const bool one = a.only_lane >= 0;
+  const int n_split = !c->nsplit ? 0 : (one ? (c->lane_nmp[a.only_lane] >= c->split_least ? 1 : 0) : c->n_split);
+  const int n_single = (one ? 1 : a.nlane) - n_split;
+  const bool both = n_split > 0 && n_single > 0;
+  if (both) {
+    CK(cudaEventRecord(c->ev_fork, c->stream));
+    CK(cudaStreamWaitEvent(c->stream2, c->ev_fork, 0));
+  }
+  if (n_split > 0) {
+    KArgs s = a;
+    s.smem_total = (int)c->sp.total;
+    if (both) s.lane_order = c->d_order.p;
+    auto run = a.periodic ? (mixed ? split_launch_mixed_box : split_launch_fp64_box)
+                          : (mixed ? split_launch_mixed : split_launch_fp64);
+    ++c->launches;
+    CK(run(n_split, c->split_nt, c->sp.total, c->stream, s));
+  }
+  if (n_single > 0) {
+    KArgs s = a;
+    if (both) s.lane_order = c->d_order.p + n_split;
+    ++c->launches;
+    CK(lane_kernel_launch(mixed, n_single, c->threads, c->smem, both ? c->stream2 : c->stream, s));
+  }
+  if (both) {
+    CK(cudaEventRecord(c->ev_join, c->stream2));
+    CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+  }
   return TIS_OK;
 }
 

@@ -47,6 +47,9 @@ struct TopDesc {
   int nslot;        // 2 nbd + 3 nba + 7 nst + 6 ntst + 6 nhb
   int slot_ba, slot_st, slot_tst, slot_hb;   // slot bases inside a lane (bonds start at 0)
   int nlabel;       // labels that belong to this topology
+  int sp0;          // slot_pos[sp0 + slot]: place of a bonded slot in the topology's incidence lists
+  int sp_ninc;      // lanes split over a cluster: the most incidence entries a CTA's beads have
+  long long sp_blob;// and their constant shared memory: the common part at split_blob[sp_blob], then each CTA's own
 };
 
 // per-lane descriptor
@@ -92,6 +95,30 @@ enum KMode {
   KM_XSTEP = 5,        // first half of one step: trigger, rebuild, x update
   KM_VSTEP = 6,        // second half of one step: forces (+ f_ext), v / a update
   KM_VXSTEP = 7,       // KM_VSTEP, then the KM_XSTEP of the next step
+};
+
+constexpr int SPLIT_MAX = 16;    // split_kernel: CTAs per lane at most
+constexpr int SPLIT_MISC = 16;   // its flag words before the unit table
+
+// Byte offsets of a CTA's shared memory, the same for every lane and CTA of a
+// context (distributed shared memory addresses a peer's copy by offset; as a
+// kernel argument they are constants of the address arithmetic, which the
+// short loops of a step are mostly made of).  The first `stat` bytes are
+// constant for a context: the host lays them out once per topology, a part
+// common to its CTAs (up to `comm`) and a part per CTA (split_blob), and the
+// kernel copies them in as they are.
+struct SplitPlan {
+  int own, rows;           // beads (a multiple of 4) and charged rows of a CTA (at most)
+  unsigned ecap;           // partner-list entries of a CTA's charged rows that fit
+  int nst, nhb, nba, nbd;  // bonded items of a CTA (at most)
+  int np;                  // beads, rounded up to a multiple of 4 (component stride of the positions)
+  // constant
+  unsigned tcu, RE, qb, base, rn2, comm, C, scr, iptr, bdi, bdd, bdc, bai, bad, bac, sti, std_, stc, hbi, hbd, hbc, hbs;
+  unsigned stat;
+  // state and scratch
+  unsigned X, P, Q, A4, L3, V, DD, C1, u0, NZ, exF, dhF, NR4, near, ncnt, mexv, mele, slots, exc, hbf, red, img, misc;
+  unsigned eoff, elist;
+  unsigned total;
 };
 
 // Kernel arguments (all device pointers).
@@ -226,6 +253,10 @@ struct KArgs {
                            // moves the lane (KM_XSTEP / KM_VSTEP); null: every lane takes nsteps
   int step_k;              // KM_XSTEP / KM_VSTEP: index of this step within the call
   const int *lane_order;   // lane of each CTA (or cluster) of a launch over every lane; null: in order
+  int nsplit;              // split_kernel: CTAs (one cluster) per lane
+  const int *slot_pos;     // see TopDesc::sp0
+  const unsigned char *split_blob;
+  SplitPlan sp;
 };
 
 #ifdef __CUDACC__

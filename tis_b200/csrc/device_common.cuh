@@ -18,10 +18,13 @@ static __device__ unsigned long long g_phase[128];
 #else
 #define PHASE_ALL(k, t0) do { if (blockIdx.x == 0) { atomicAdd(&g_phase[k], (unsigned long long)(clock64() - (t0))); atomicAdd(&g_phase[(k) + 16], 1ull); } } while (0)
 #endif
+// per-warp spans by kind of work of CTA 0: total at 32 + k, count at 48 + k
+#define PHASE_KIND(k, t0) do { if (blockIdx.x == 0 && (threadIdx.x & 31) == 0) { const int k_ = (k); atomicAdd(&g_phase[32 + k_], (unsigned long long)(clock64() - (t0))); atomicAdd(&g_phase[48 + k_], 1ull); } } while (0)
 // per-warp spans of the first two CTAs: slots base + 16 blockIdx.x + warp
 #define PHASE_WARP(base, t0) do { if (blockIdx.x < 2 && (threadIdx.x & 31) == 0) atomicAdd(&g_phase[(base) + 16 * blockIdx.x + (threadIdx.x >> 5)], (unsigned long long)(clock64() - (t0))); } while (0)
 #else
 #define PHASE_WARP(base, t0) do {} while (0)
+#define PHASE_KIND(k, t0) do {} while (0)
 #define PHASE_ALL(k, t0) do {} while (0)
 #define PHASE_T0(v) do {} while (0)
 #define PHASE_ADD(k, t0) do {} while (0)
@@ -76,7 +79,7 @@ template <> struct V4<double> { typedef double4 T; };
 constexpr size_t MASK_SMEM_MAX = 64 * 1024;    // bit matrices kept in shared memory up to this size
 
 // MISC_EXCESS, MISC_NEAR_DISP and MISC_DMAX have a second copy (+1) for odd
-// steps: the two-CTA kernel sets a flag for the next step while the current
+// steps: the cluster kernels set a flag for the next step while the current
 // one is read.
 enum { MISC_EXCESS = 0, MISC_CLAMP = 2, MISC_NEXV = 3, MISC_NELE = 4, MISC_NAN = 5,
        MISC_REBUILT = 6, MISC_NEAR_BAD = 7, MISC_NEAR_DISP = 8, MISC_PMF = 10, MISC_CHUNK = 11,
@@ -350,8 +353,8 @@ __device__ __forceinline__ void put_slot(const SlotDst &d, size_t k, int bead, R
   p[0] = fx; p[1] = fy; p[2] = fz;
 }
 
-template <typename Real>
-__device__ __forceinline__ R3<Real> dvec(const Smem<Real> &s, int i, int j) {   // x_j - x_i (unwrapped)
+template <typename Real, typename S>
+__device__ __forceinline__ R3<Real> dvec(const S &s, int i, int j) {   // x_j - x_i (unwrapped)
   return R3<Real>{(Real)(s.X[j] - s.X[i]), (Real)(s.Y[j] - s.Y[i]), (Real)(s.Z[j] - s.Z[i])};
 }
 
@@ -370,11 +373,11 @@ template <typename Real> __device__ __forceinline__ Real wrap_pi(Real d) {
 }
 
 // force_bond.F90:41-56
-template <typename Real>
-__device__ void term_bond(const KArgs &a, const TopDesc &T, const Smem<Real> &s, const SlotDst &slots, int k) {
+template <typename Real, typename S, typename Dst>
+__device__ void term_bond(const KArgs &a, const TopDesc &T, const S &s, const Dst &slots, int k) {
   const int *mp = a.bd_idx + 2 * (size_t)(T.bd0 + k);
   const int m[2] = {ldro(mp), ldro(mp + 1)};
-  R3<Real> v = dvec(s, m[0], m[1]);
+  R3<Real> v = dvec<Real>(s, m[0], m[1]);
   Real dist = sqrt(v.x * v.x + v.y * v.y + v.z * v.z);
   Real dd = dist - (Real)ldro(a.bd_nat + T.bd0 + k);
   Real f = (Real)ldro(a.bd_coef + T.bd0 + k) * ((Real)-2.0 * fdiv(dd, dist));
@@ -382,19 +385,13 @@ __device__ void term_bond(const KArgs &a, const TopDesc &T, const Smem<Real> &s,
   put_slot<Real>(slots, 2 * k + 1, m[1], f * v.x, f * v.y, f * v.z);
 }
 
-// force_bangle.F90:103-147
+// force_bangle.F90:103-147: the forces of one angle's beads
 template <typename Real>
-__device__ void term_angle(const KArgs &a, const TopDesc &T, const Smem<Real> &s, const SlotDst &slots, int k) {
-  const size_t sb = T.slot_ba + 3 * (size_t)k;
-  const Real cf = (Real)ldro(a.ba_coef + T.ba0 + k);
-  const int *mp = a.ba_idx + 3 * (size_t)(T.ba0 + k);
-  const int m[3] = {ldro(mp), ldro(mp + 1), ldro(mp + 2)};
+__device__ __forceinline__ void angle_force(R3<Real> v21, R3<Real> v32, Real nat, Real cf, R3<Real> *f3) {
   if (cf < (Real)1.0e-6) {
-    put_slot<Real>(slots, sb, m[0], 0, 0, 0); put_slot<Real>(slots, sb + 1, m[1], 0, 0, 0);
-    put_slot<Real>(slots, sb + 2, m[2], 0, 0, 0);
+    f3[0] = f3[1] = f3[2] = R3<Real>{0, 0, 0};
     return;
   }
-  R3<Real> v21 = dvec(s, m[0], m[1]), v32 = dvec(s, m[1], m[2]);
   Real c11 = dot(v21, v21), c22 = dot(v32, v32), c21 = dot(v32, v21);
   Real co = -c21 * frsq(c11 * c22);
   if (co > (Real)1) co = 1; else if (co < (Real)-1) co = -1;
@@ -411,23 +408,35 @@ __device__ void term_angle(const KArgs &a, const TopDesc &T, const Smem<Real> &s
     th = acos(co);
     t3 = c11 * c22 - c21 * c21;
   }
-  Real dba = th - (Real)ldro(a.ba_nat + T.ba0 + k);
+  Real dba = th - nat;
   if (t3 <= (Real)1) t3 = 1;
   Real f = (Real)2 * cf * dba * frsq(t3);
   Real a1 = fdiv(c21, c11), a2 = fdiv(c21, c22);
   R3<Real> f21{f * (v21.x * a1 - v32.x), f * (v21.y * a1 - v32.y), f * (v21.z * a1 - v32.z)};
   R3<Real> f32{f * (v32.x * a2 - v21.x), f * (v32.y * a2 - v21.y), f * (v32.z * a2 - v21.z)};
-  put_slot<Real>(slots, sb, m[0], -f21.x, -f21.y, -f21.z);
-  put_slot<Real>(slots, sb + 1, m[1], f21.x - f32.x, f21.y - f32.y, f21.z - f32.z);
-  put_slot<Real>(slots, sb + 2, m[2], f32.x, f32.y, f32.z);
+  f3[0] = R3<Real>{-f21.x, -f21.y, -f21.z};
+  f3[1] = R3<Real>{f21.x - f32.x, f21.y - f32.y, f21.z - f32.z};
+  f3[2] = f32;
+}
+
+template <typename Real, typename S, typename Dst>
+__device__ void term_angle(const KArgs &a, const TopDesc &T, const S &s, const Dst &slots, int k) {
+  const size_t sb = T.slot_ba + 3 * (size_t)k;
+  const Real cf = (Real)ldro(a.ba_coef + T.ba0 + k);
+  const int *mp = a.ba_idx + 3 * (size_t)(T.ba0 + k);
+  const int m[3] = {ldro(mp), ldro(mp + 1), ldro(mp + 2)};
+  R3<Real> f[3];
+  angle_force<Real>(dvec<Real>(s, m[0], m[1]), dvec<Real>(s, m[1], m[2]), (Real)ldro(a.ba_nat + T.ba0 + k), cf, f);
+#pragma unroll
+  for (int p = 0; p < 3; ++p) put_slot<Real>(slots, sb + p, m[p], f[p].x, f[p].y, f[p].z);
 }
 
 // st_status of secondary stack k (force_dtrna_stack_nlocal.F90:83-92): off
 // when an exclusive tertiary stack of it is within 10 A of its native
 // distance; FP64 in the reference's operation order, so the decision is the
 // reference's
-template <typename Real>
-__device__ __forceinline__ bool stack_excluded(const KArgs &a, const TopDesc &T, const Smem<Real> &s, int k) {
+template <typename Real, typename S>
+__device__ __forceinline__ bool stack_excluded(const KArgs &a, const TopDesc &T, const S &s, int k) {
   if (T.ntst == 0) return false;
   for (int e = a.stx_ptr[T.stx0 + k]; e < a.stx_ptr[T.stx0 + k + 1]; ++e) {
     const int t = a.stx_tst[e];
@@ -443,8 +452,8 @@ __device__ __forceinline__ bool stack_excluded(const KArgs &a, const TopDesc &T,
 
 // force_dtrna_stack_nlocal.F90:60-263: tertiary stack k into its six slots,
 // FP64 in both paths for the reason given at term_stack
-template <typename Real>
-__device__ void term_tstack(const KArgs &a, const TopDesc &T, const Smem<Real> &s, const SlotDst &slots, int k) {
+template <typename Real, typename S, typename Dst>
+__device__ void term_tstack(const KArgs &a, const TopDesc &T, const S &s, const Dst &slots, int k) {
   const int *m = a.tst_idx + 6 * (size_t)(T.tst0 + k);
   const double *nat = a.tst_nat + 6 * (size_t)(T.tst0 + k);
   const double *cf = a.tst_coef + 7 * (size_t)(T.tst0 + k);
@@ -562,8 +571,8 @@ __device__ void term_tstack(const KArgs &a, const TopDesc &T, const Smem<Real> &
 // dihedrals run through a nearly straight triple: their cross products of
 // nearly parallel bond vectors, and force terms that cancel, are resolved by
 // FP32 only to ~1e-4 (measured on a C4 chain).
-template <typename Real>
-__device__ void term_stack64(const KArgs &a, const TopDesc &T, const Smem<Real> &s, const SlotDst &slots, int k, double u0) {
+template <typename Real, typename S, typename Dst>
+__device__ void term_stack64(const KArgs &a, const TopDesc &T, const S &s, const Dst &slots, int k, double u0) {
   const int *mp = a.st_idx + 7 * (size_t)(T.st0 + k);
   const int m[7] = {ldro(mp), ldro(mp + 1), ldro(mp + 2), ldro(mp + 3), ldro(mp + 4), ldro(mp + 5), ldro(mp + 6)};
   const double *natp = a.st_nat + 3 * (size_t)(T.st0 + k), *cfp = a.st_coef + 3 * (size_t)(T.st0 + k);
@@ -634,8 +643,8 @@ __device__ void term_stack64(const KArgs &a, const TopDesc &T, const Smem<Real> 
 // path evaluates it as written; the mixed path in FP32 unless one of the
 // dihedrals' triples is within ~2 degrees of straight (sin^2 < 1e-3), which
 // goes to term_stack64
-template <typename Real>
-__device__ void term_stack(const KArgs &a, const TopDesc &T, const Smem<Real> &s, const SlotDst &slots, int k, double u0) {
+template <typename Real, typename S, typename Dst>
+__device__ void term_stack(const KArgs &a, const TopDesc &T, const S &s, const Dst &slots, int k, double u0) {
   const int *mp = a.st_idx + 7 * (size_t)(T.st0 + k);
   const int m[7] = {ldro(mp), ldro(mp + 1), ldro(mp + 2), ldro(mp + 3), ldro(mp + 4), ldro(mp + 5), ldro(mp + 6)};
   if (stack_excluded<Real>(a, T, s, k)) {
@@ -647,11 +656,11 @@ __device__ void term_stack(const KArgs &a, const TopDesc &T, const Smem<Real> &s
   const double *natp = a.st_nat + 3 * (size_t)(T.st0 + k), *cfp = a.st_coef + 3 * (size_t)(T.st0 + k);
   const double nat[3] = {ldro(natp), ldro(natp + 1), ldro(natp + 2)};
   const double cf[3] = {ldro(cfp), ldro(cfp + 1), ldro(cfp + 2)};
-  R3<Real> v21 = dvec(s, m[0], m[1]);
-  R3<Real> v34 = dvec(s, m[3], m[2]);
-  R3<Real> v54 = dvec(s, m[3], m[4]);
-  R3<Real> v56 = dvec(s, m[5], m[4]);
-  R3<Real> v76 = dvec(s, m[5], m[6]);
+  R3<Real> v21 = dvec<Real>(s, m[0], m[1]);
+  R3<Real> v34 = dvec<Real>(s, m[3], m[2]);
+  R3<Real> v54 = dvec<Real>(s, m[3], m[4]);
+  R3<Real> v56 = dvec<Real>(s, m[5], m[4]);
+  R3<Real> v76 = dvec<Real>(s, m[5], m[6]);
   if constexpr (sizeof(Real) == 4) {
     const R3<Real> c1 = crs(v34, v54), c2 = crs(v54, v56), c3 = crs(v76, v56);
     const Real l54 = dot(v54, v54), l56 = dot(v56, v56);
@@ -715,8 +724,8 @@ __device__ void term_stack(const KArgs &a, const TopDesc &T, const Smem<Real> &s
 
 // force_dtrna_hbond15.F90:91-353 (one hbond of the neighbour list).
 // Returns the energy; active = |d| <= hb_cutoff_dist.
-template <typename Real>
-__device__ double term_hbond(const KArgs &a, const TopDesc &T, const Smem<Real> &s, const SlotDst &slots, int k, bool &active) {
+template <typename Real, typename S, typename Dst>
+__device__ double term_hbond(const KArgs &a, const TopDesc &T, const S &s, const Dst &slots, int k, bool &active) {
   const int *mp = a.hb_idx + 6 * (size_t)(T.hb0 + k);
   const int m[6] = {ldro(mp), ldro(mp + 1), ldro(mp + 2), ldro(mp + 3), ldro(mp + 4), ldro(mp + 5)};
   const double *natp = a.hb_nat + 6 * (size_t)(T.hb0 + k), *cfp = a.hb_coef + 7 * (size_t)(T.hb0 + k);
@@ -850,10 +859,14 @@ __device__ double term_hbond(const KArgs &a, const TopDesc &T, const Smem<Real> 
   return ene;
 }
 
-// force_dtrna_hbond15.F90:373-509, run by one thread of the lane
-template <typename Real>
+// force_dtrna_hbond15.F90:373-509, run by one thread of the lane; on_del is
+// called with every hydrogen bond it turns off
+struct NoDel {
+  __device__ void operator()(int) const {}
+};
+template <typename Real, typename Del = NoDel>
 __device__ void prune_hbonds(const KArgs &a, int lane, const LaneDesc &L, const TopDesc &T, long long istep,
-                             double beta, bool zero_energy, int *exc) {
+                             double beta, bool zero_energy, int *exc, Del on_del = Del()) {
   uint8_t *hbf = a.hb_flag + L.hb0;
   double *ene = a.hb_ene + L.hb0;
   const int ns = T.nsite;
@@ -894,6 +907,7 @@ __device__ void prune_hbonds(const KArgs &a, int lane, const LaneDesc &L, const 
       if (rnd < ratio) idel = jhb;
     }
     hbf[idel] &= ~2;
+    on_del(idel);
     if (zero_energy) ene[idel] = 0.0;
     const int *sites = a.hb_site + 6 * (size_t)(T.hb0 + idel);
     for (int i = 0; i < 3; ++i) {

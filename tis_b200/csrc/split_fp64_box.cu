@@ -1,0 +1,23 @@
+// split_fp64_box.cu -- split_kernel for FP64 lanes in a periodic box (one unit
+// per variant: they compile side by side).
+#include "split_launch.cuh"
+
+namespace tis {
+
+cudaError_t split_launch_fp64_box(int nlane, int nt, size_t smem, cudaStream_t st, const KArgs &a) {
+  return nt == 256 ? split_run<double, 256, true>(nlane, smem, st, a) : split_run<double, 512, true>(nlane, smem, st, a);
+}
+
+cudaError_t split_setup_fp64_box(int nsplit, int nt, size_t smem, int *clusters) {
+  return nt == 256 ? split_prepare<double, 256, true>(nsplit, smem, clusters) : split_prepare<double, 512, true>(nsplit, smem, clusters);
+}
+
+#ifdef TIS_PHASE_TIMING
+extern "C" int tis_phase_read_fp64_box(unsigned long long *out) {
+  static const unsigned long long zero[128] = {};
+  const int e = (int)cudaMemcpyFromSymbol(out, g_phase, sizeof(zero));
+  return e ? e : (int)cudaMemcpyToSymbol(g_phase, zero, sizeof(zero));
+}
+#endif
+
+} // namespace tis

@@ -1,0 +1,83 @@
+// split_plan.cuh -- shared-memory layout of a lane split over a cluster
+// (split_kernel.cuh), shared with the host, which lays out the constant part.
+#pragma once
+#include "common.cuh"
+
+namespace tis {
+
+constexpr int SG = 8;            // threads per bead (update phase, exv lists)
+constexpr int SP_NEAR = 8;       // near-list entries per thread of a bead's group
+constexpr int SP_IMG = 11;       // pair entries: bead in the low bits, periodic image above (periodic lanes: N < 2048)
+
+// threads of a warp that share one charged row: short rows take few
+__host__ __device__ inline int split_row_lanes(int nq, bool ewald) {
+  return (ewald || nq <= 64) ? 8 : (nq <= 160 ? 16 : 32);
+}
+
+// own beads of a CTA for a lane of N beads
+__host__ __device__ inline int split_own(int N, int nr) { return ((N + nr - 1) / nr + 3) & ~3; }
+
+// T: the largest counts of the context's topologies
+inline SplitPlan split_plan(const TopDesc &T, int nq, int nr, bool periodic, bool skin, bool ewald, int real,
+                            unsigned limit) {
+  SplitPlan p;
+  const int N = T.nmp;
+  p.own = split_own(N, nr);
+  p.rows = (nq + nr - 1) / nr;
+  p.nst = (T.nst + nr - 1) / nr; p.nhb = (T.nhb + nr - 1) / nr;
+  p.nba = (T.nba + nr - 1) / nr; p.nbd = (T.nbd + nr - 1) / nr;
+  p.np = (N + 3) & ~3;
+  const unsigned n = p.np, o = p.own, W = (N + 31) / 32, R = real;
+  unsigned b = 0;
+  auto take = [&](unsigned bytes) { const unsigned at = b; b = (b + bytes + 15u) & ~15u; return at; };
+  p.tcu = take(4 * n);                    // type | class << 8 | unit << 16
+  p.RE = take(2 * R * n);                 // exv radius, sqrt(eps)
+  p.qb = take(4 * nq);
+  p.base = take(4 * (SPLIT_MAX + 1));
+  p.rn2 = take(8 * T.nunit * T.nunit);
+  p.comm = b;
+  p.C = take(32 * o);                     // rlan_const(2..4), 1 / m of the own beads
+  p.scr = take(R * o);                    // exv screen radius
+  p.iptr = take(4 * (o + 1));
+  p.bdi = take(4 * p.nbd); p.bdd = take(8 * p.nbd); p.bdc = take(2 * R * p.nbd);
+  p.bai = take(8 * p.nba); p.bad = take(12 * p.nba); p.bac = take(2 * R * p.nba);
+  p.sti = take(16 * p.nst); p.std_ = take(28 * p.nst); p.stc = take(6 * R * p.nst);
+  p.hbi = take(12 * p.nhb); p.hbd = take(24 * p.nhb); p.hbc = take(13 * R * p.nhb); p.hbs = take(24 * p.nhb);
+  p.stat = b;
+  p.X = take(24 * n);
+  p.P = periodic ? take(24 * n) : p.X;
+  p.Q = periodic ? take(24 * n) : p.X;
+  p.A4 = take(4 * R * (n + 4));           // and a bead far away without charge (entry np)
+  p.L3 = real == 4 ? take(12 * n) : 0;
+  p.V = take((skin ? 72 : 48) * o);       // v, a, [dxyz]
+  p.DD = skin ? take(8 * o) : 0;
+  p.C1 = take(8 * o);
+  p.u0 = take(8 * p.nst);
+  p.NZ = take(24 * o); p.exF = take(24 * o); p.dhF = take(24 * o);
+  p.NR4 = take(16 * o);
+  p.near = take(2 * SG * SP_NEAR * o); p.ncnt = take(SG * o);
+  p.mexv = take(4 * W * o); p.mele = take(4 * W * p.rows);
+  p.slots = take(3 * R * T.sp_ninc);
+  p.exc = take(4 * T.nsite); p.hbf = take(p.nhb);
+  p.red = take(8 * (64 + 2 * SPLIT_MAX) + 8 * SPLIT_MAX);   // reductions; then the CTAs' displacement maxima, 2 parities
+  p.img = periodic ? take(4 * R * 27) : 0;
+  p.misc = take(4 * (SPLIT_MISC + T.nunit * T.nunit + 8));
+  // partner lists of the charged rows: room for the longest possible ones, or
+  // what is left of the shared memory (Debye-Hueckel rows fill theirs, the
+  // 20 A rows of an ion box need a fraction)
+  const unsigned eb = 2 * split_row_lanes(nq, ewald), most = p.rows * ((nq + eb - 1) / eb * eb);
+  p.eoff = take(4 * (p.rows + 1));
+  const unsigned left = b < limit ? (limit - b) / 32 * 16 : 0;
+  p.ecap = most < left ? most : left;
+  p.elist = take(2 * p.ecap);
+  p.total = b;
+  return p;
+}
+
+// CTA r's share of n items divided by index
+__host__ __device__ inline int split_share(int n, int nr, int r) {
+  const int per = (n + nr - 1) / nr;
+  return per * r < n ? per * r : n;
+}
+
+} // namespace tis
