@@ -136,3 +136,22 @@ def test_batch_with_some_lanes_split(tis_lib):
         assert np.abs(x[lo:lo + s["nmp"]] - orc.get_state()[0].reshape(-1, 3)).max() < POS_TOL[0]
         orc.close()
     eng.close()
+
+
+@pytest.mark.parametrize("ctas,precision", [(2, 1), (4, 0), (8, 0), (16, 0), (8, 1)])
+def test_near_lists_follow_beads_of_other_ctas(tis_lib, ctas, precision):
+    """A dense chain over 300 steps, many near-list recordings: a contact with
+    a bead that another CTA moves must not be missed.  Against one CTA per
+    replica with the same noise (FP64: the same sums in another order; mixed:
+    FP32 rounding, amplified over the run)."""
+    s = synth.set_friction(synth.dt15_chain(40, 5, min_dist=2.8, confine=12.0), 0.5)
+    par = synth.dt15_params(ionic_strength=0.15, n_step_neighbor=0, precision=precision)
+    out = []
+    for c in (1, ctas):
+        eng = Engine([s], dict(par, launch_ctas=c), [400.0])
+        eng.set_state(s["xyz"])
+        eng.time_integral_pre()
+        eng.step(300)
+        out.append(eng.get_state()[0])
+        eng.close()
+    assert np.abs(out[0] - out[1]).max() < {0: 1e-6, 1: 1e-2}[precision]

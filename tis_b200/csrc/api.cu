@@ -187,9 +187,9 @@ struct tis_ctx {
   long long g_nstep = -1, g_launches = 0;
   int g_exchange = -1;
   // Ewald
-  int nk = 0, hmax = 0, nqblk = 1, nq_max = 0;
-  DBuf<int8_t> ew_h;
-  DBuf<double> ew_coef, ew_tab, ew_S, f_ext;
+  int ew_ncol = 0, hmax = 0, nq_max = 0;
+  DBuf<char4> ew_col;
+  DBuf<double> ew_w, ew_S, f_ext;
   // Brownian dynamics with hydrodynamic interactions
   bool bdhi = false;
   int max_nmp = 0;
@@ -348,44 +348,30 @@ int env_int(const char *name) {
   return e ? std::atoi(e) : 0;
 }
 
-// Reciprocal vectors of mloop_ewld.F90:56-156: every integer h != 0 with
-// |h| <= hmax in (x, y, z) loop order, comb-sorted by |h|^2 with the
-// reference's gap rule, and C(k) = 2 pi / L^3 exp(-k^2 / 4 alpha^2) / k^2
-// for k = 2 pi h / L.
-void ewald_table(double L, double alpha, double hmax, std::vector<int8_t> &hv, std::vector<double> &coef) {
+// Reciprocal vectors of mloop_ewld.F90:56-156, every integer h != 0 with |h|
+// <= hmax, as columns (hx, hy) of the half space hx > 0 or hx = 0 and hy >= 0
+// (longest first), and the weights of their pairs +-hz from C(k) = 2 pi / L^3
+// exp(-k^2 / 4 alpha^2) / k^2, k = 2 pi h / L (see KArgs::ew_w).
+void ewald_columns(double L, double alpha, double hmax, std::vector<char4> &col, std::vector<double> &w) {
   const int lmax = (int)std::ceil(hmax);
-  const double hmax2 = hmax * hmax;
-  std::vector<int> hh;
-  std::vector<double> h2;
-  for (int ix = -lmax; ix <= lmax; ++ix)
-    for (int iy = -lmax; iy <= lmax; ++iy)
-      for (int iz = -lmax; iz <= lmax; ++iz) {
-        if (ix == 0 && iy == 0 && iz == 0) continue;
-        const double r2 = (double)ix * ix + (double)iy * iy + (double)iz * iz;
-        if (r2 <= hmax2) { hh.push_back(ix); hh.push_back(iy); hh.push_back(iz); h2.push_back(r2); }
-      }
-  const int n = (int)h2.size();
-  int gap = n;
-  bool swapped = false;
-  while (gap > 1 || swapped) {
-    gap = (gap * 10) / 13;
-    if (gap < 1) gap = 1;
-    else if (gap == 9 || gap == 10) gap = 11;
-    swapped = false;
-    for (int i = 0; i + gap < n; ++i)
-      if (h2[i] > h2[i + gap]) {
-        std::swap(h2[i], h2[i + gap]);
-        for (int d = 0; d < 3; ++d) std::swap(hh[3 * i + d], hh[3 * (i + gap) + d]);
-        swapped = true;
-      }
-  }
-  const double f = 2.0 * F_PI / L;
-  hv.resize(3 * (size_t)n);
-  coef.resize(n);
-  for (int i = 0; i < n; ++i) {
-    for (int d = 0; d < 3; ++d) hv[3 * i + d] = (int8_t)hh[3 * i + d];
-    coef[i] = 2.0 * F_PI / (L * L * L) * std::exp(-(f * f) * h2[i] / (4.0 * alpha * alpha)) / ((f * f) * h2[i]);
-  }
+  const double hmax2 = hmax * hmax, f = 2.0 * F_PI / L;
+  for (int ix = 0; ix <= lmax; ++ix)
+    for (int iy = -lmax; iy <= lmax; ++iy) {
+      if ((ix == 0 && iy < 0) || (double)(ix * ix + iy * iy) > hmax2) continue;
+      int mz = 0;
+      while ((double)(ix * ix + iy * iy + (mz + 1) * (mz + 1)) <= hmax2) ++mz;
+      col.push_back(make_char4((char)ix, (char)iy, (char)mz, 0));
+    }
+  std::stable_sort(col.begin(), col.end(), [](const char4 &x, const char4 &y) { return x.z > y.z; });
+  const size_t n = col.size();
+  w.assign((size_t)EW_H * n, 0.0);
+  for (size_t k = 0; k < n; ++k)
+    for (int h = 0; h <= col[k].z; ++h) {
+      const double h2 = (double)(col[k].x * col[k].x + col[k].y * col[k].y + h * h);
+      if (h2 == 0.0) continue;
+      const double c = 2.0 * F_PI / (L * L * L) * std::exp(-(f * f) * h2 / (4.0 * alpha * alpha)) / ((f * f) * h2);
+      w[h * n + k] = (h ? 2.0 : 1.0) * c * (col[k].x == 0 && col[k].y == 0 ? 0.5 : 1.0);
+    }
 }
 
 }  // namespace
@@ -468,8 +454,7 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     return TIS_E_ARG;
   }
   if (p.i_ele == TIS_ELE_EWALD) {
-    // mloop_ewld.F90 uses psize(1) for a cubic box; the per-charge tables
-    // hold |h| <= 11
+    // mloop_ewld.F90 uses psize(1) for a cubic box; the column sums hold |h| <= 11
     if (p.i_periodic != 1 || p.psize[0] != p.psize[1] || p.psize[0] != p.psize[2] || !(p.ewld_hmax > 0.0) ||
         std::ceil(p.ewld_hmax) > 11.0 || !(p.ewld_alpha > 0.0)) {
       tis_destroy(c);
@@ -824,7 +809,7 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
   }
   size_t mask_off = 0, slot_off = 0;
   long long mirror_off = 0;
-  int hb_off = 0, site_off = 0, state_off = 0, ew_off = 0;
+  int hb_off = 0, site_off = 0, state_off = 0;
   long long bd_off = 0, bdp_off = 0, bd32_off = 0, bdw_off = 0;
   int lane = 0;
   for (int k = 0; k < ntop; ++k) {
@@ -842,8 +827,6 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
       L.hb0 = hb_off;
       L.site0 = site_off;
       L.unif0 = 0;
-      L.ew0 = ew_off;
-      ew_off += d.nq;
       L.bd0 = bd_off;
       L.bdp0 = bdp_off;
       L.bd32 = bd32_off;
@@ -976,16 +959,30 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
           const int b0 = std::min(d.nmp, r * own), b1 = std::min(d.nmp, b0 + own);
           d.sp_ninc = std::max(d.sp_ninc, inc_ptr[d.inc0 + b1] - inc_ptr[d.inc0 + b0]);
         }
-        mx.nmp = std::max(mx.nmp, d.nmp); mx.nst = std::max(mx.nst, d.nst); mx.nhb = std::max(mx.nhb, d.nhb);
-        mx.nba = std::max(mx.nba, d.nba); mx.nbd = std::max(mx.nbd, d.nbd); mx.nsite = std::max(mx.nsite, d.nsite);
+        mx.nmp = std::max(mx.nmp, d.nmp); mx.nsite = std::max(mx.nsite, d.nsite);
         mx.nunit = std::max(mx.nunit, d.nunit); mx.sp_ninc = std::max(mx.sp_ninc, d.sp_ninc);
+        // bonded items go with the owner of their first bead
+        auto most = [&](const std::vector<int> &idx, int first, int n, int width) {
+          std::vector<int> m(nr, 0);
+          for (int k = 0; k < n; ++k) ++m[idx[(size_t)width * (first + k)] / own];
+          return *std::max_element(m.begin(), m.end());
+        };
+        mx.nst = std::max(mx.nst, most(st_idx, d.st0, d.nst, 7)); mx.nhb = std::max(mx.nhb, most(hb_idx, d.hb0, d.nhb, 6));
+        mx.nba = std::max(mx.nba, most(ba_idx, d.ba0, d.nba, 3)); mx.nbd = std::max(mx.nbd, most(bd_idx, d.bd0, d.nbd, 2));
+        mx.ntst = std::max(mx.ntst, most(tst_idx, d.tst0, d.ntst, 6));
         if (p.i_ele != TIS_ELE_NONE) mq = std::max(mq, d.nq);
       }
       const bool ewald = p.i_ele == TIS_ELE_EWALD;
-      const SplitPlan sp = split_plan(mx, mq, nr, periodic, skin, ewald, real_size, 227 * 1024);
-      // (Debye-Hueckel rows may list every charge; without room for the lists
-      // the kernel reads the rows' bits, ~4x slower)
-      if (sp.total > 227 * 1024 || (lists && !ewald && sp.ecap < (unsigned)sp.rows * mq)) return false;
+      // Debye-Hueckel rows may list every charge; the short rows of an ion box
+      // get four times their share of a uniform box
+      int row = mq;
+      if (ewald) {
+        const double rc = p.cutoff_ele + p.neigh_margin;
+        row = (int)std::min<double>(mq, 64.0 + 4.0 * mq * (4.0 / 3.0 * F_PI * rc * rc * rc) / (p.psize[0] * p.psize[1] * p.psize[2]));
+      }
+      const SplitPlan sp = split_plan(mx, mq, row, nr, periodic, skin, ewald, real_size, 227 * 1024);
+      // (without room for the lists the kernel reads the rows' bits, ~4x slower)
+      if (sp.total > 227 * 1024 || (lists && sp.ecap < (unsigned)sp.rows * row)) return false;
       // 256 threads (with twice the registers) while a CTA's warps have a
       // few work items each, 512 above
       const int nt = sp.own <= 32 ? 256 : 512;
@@ -1033,17 +1030,25 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
           const double turns = n_split > places || nlane > sms ? 0.25 * longest : 0.0;
           return std::max(longest, std::max(work * scale / sms, n_split ? work * n_split / nlane / (places * nr) : 0.0) + turns);
         };
-        double time = total(0, 0, 0);
+        const double time = total(0, 0, 0);
         std::vector<int> from{0};
         if (c->ntop > 1 && p.i_ele != TIS_ELE_EWALD)
           for (int n : {150, 240, 320, 450, 600, 800, 1000})
             if (n > minN && n <= maxN) from.push_back(n);
+        // best estimate first (as if clusters could use every SM), until one fits
+        struct Option { double time; int least, nr; };
+        std::vector<Option> options;
         for (int least : from)
-          for (int nr = 16; nr >= 2; nr /= 2) {
-            if (std::max(minN, least) < 4 * nr || !try_split(nr, least, true, clusters)) continue;
-            const double x = total(nr, least, clusters);
-            if (x < time) { time = x; best = nr; best_least = least; }
-          }
+          for (int nr = 16; nr >= 2; nr /= 2)
+            if (std::max(minN, least) >= 4 * nr) options.push_back({total(nr, least, std::max(1, nsm / nr)), least, nr});
+        std::stable_sort(options.begin(), options.end(), [](const Option &x, const Option &y) { return x.time < y.time; });
+        double least_time = time;
+        for (const Option &o : options) {
+          if (o.time >= least_time) break;
+          if (!try_split(o.nr, o.least, true, clusters)) continue;
+          const double x = total(o.nr, o.least, clusters);
+          if (x < least_time) { least_time = x; best = o.nr; best_least = o.least; }
+        }
       }
       c->nsplit = 0;
       if (best) {
@@ -1104,48 +1109,56 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
             ((Real *)(B + pl.scr))[li] = (Real)(b_screen[b] * (1.0 + 1.0e-4) + 1.0e-3);
           }
           for (int i = lo; i <= hi; ++i) ((int *)(B + pl.iptr))[i - lo] = inc_ptr[d.inc0 + i] - inc_ptr[d.inc0 + lo];
-          for (int k0 = split_share(d.nbd, nr, r), k = k0; k < split_share(d.nbd, nr, r + 1); ++k) {
-            const int *m = &bd_idx[2 * (size_t)(d.bd0 + k)];
-            ((uint32_t *)(B + pl.bdi))[k - k0] = (uint32_t)m[0] | (uint32_t)m[1] << 16;
-            for (int q = 0; q < 2; ++q) ((uint32_t *)(B + pl.bdd))[2 * (k - k0) + q] = word(2 * k + q, m[q]);
-            Real *cf = (Real *)(B + pl.bdc) + 2 * (k - k0);
+          int *cnt = (int *)(B + pl.cnt);
+          // items in topology order, those whose first bead this CTA owns
+          auto items = [&](const std::vector<int> &idx, int first, int n, int width, int &count, auto put) {
+            count = 0;
+            for (int k = 0; k < n; ++k) {
+              const int *m = &idx[(size_t)width * (first + k)];
+              if (m[0] >= lo && m[0] < hi) put(count++, k, m);
+            }
+          };
+          items(bd_idx, d.bd0, d.nbd, 2, cnt[4], [&](int i, int k, const int *m) {
+            ((uint32_t *)(B + pl.bdi))[i] = (uint32_t)m[0] | (uint32_t)m[1] << 16;
+            for (int q = 0; q < 2; ++q) ((uint32_t *)(B + pl.bdd))[2 * i + q] = word(2 * k + q, m[q]);
+            Real *cf = (Real *)(B + pl.bdc) + 2 * i;
             cf[0] = (Real)bd_nat[d.bd0 + k]; cf[1] = (Real)bd_coef[d.bd0 + k];
-          }
-          for (int k0 = split_share(d.nba, nr, r), k = k0; k < split_share(d.nba, nr, r + 1); ++k) {
-            const int *m = &ba_idx[3 * (size_t)(d.ba0 + k)];
-            uint32_t *ix = (uint32_t *)(B + pl.bai) + 2 * (k - k0);
+          });
+          items(ba_idx, d.ba0, d.nba, 3, cnt[3], [&](int i, int k, const int *m) {
+            uint32_t *ix = (uint32_t *)(B + pl.bai) + 2 * i;
             ix[0] = (uint32_t)m[0] | (uint32_t)m[1] << 16; ix[1] = (uint32_t)m[2];
-            for (int q = 0; q < 3; ++q) ((uint32_t *)(B + pl.bad))[3 * (k - k0) + q] = word(d.slot_ba + 3 * k + q, m[q]);
-            Real *cf = (Real *)(B + pl.bac) + 2 * (k - k0);
+            for (int q = 0; q < 3; ++q) ((uint32_t *)(B + pl.bad))[3 * i + q] = word(d.slot_ba + 3 * k + q, m[q]);
+            Real *cf = (Real *)(B + pl.bac) + 2 * i;
             cf[0] = (Real)ba_nat[d.ba0 + k]; cf[1] = (Real)ba_coef[d.ba0 + k];
-          }
-          for (int k0 = split_share(d.nst, nr, r), k = k0; k < split_share(d.nst, nr, r + 1); ++k) {
-            const int *m = &st_idx[7 * (size_t)(d.st0 + k)];
-            uint32_t *ix = (uint32_t *)(B + pl.sti) + 4 * (k - k0);
+          });
+          items(st_idx, d.st0, d.nst, 7, cnt[1], [&](int i, int k, const int *m) {
+            ((int *)(B + pl.stk))[i] = k;
+            uint32_t *ix = (uint32_t *)(B + pl.sti) + 4 * i;
             for (int q = 0; q < 7; ++q) {
               ix[q / 2] |= (uint32_t)m[q] << (16 * (q & 1));
-              ((uint32_t *)(B + pl.std_))[7 * (k - k0) + q] = word(d.slot_st + 7 * k + q, m[q]);
+              ((uint32_t *)(B + pl.std_))[7 * i + q] = word(d.slot_st + 7 * k + q, m[q]);
             }
-            Real *cf = (Real *)(B + pl.stc) + 6 * (k - k0);
+            Real *cf = (Real *)(B + pl.stc) + 6 * i;
             for (int q = 0; q < 3; ++q) {
               cf[q] = (Real)st_nat[3 * (size_t)(d.st0 + k) + q];
               cf[3 + q] = (Real)st_coef[3 * (size_t)(d.st0 + k) + q];
             }
-          }
-          for (int k0 = split_share(d.nhb, nr, r), k = k0; k < split_share(d.nhb, nr, r + 1); ++k) {
-            const int *m = &hb_idx[6 * (size_t)(d.hb0 + k)];
-            uint32_t *ix = (uint32_t *)(B + pl.hbi) + 3 * (k - k0);
+          });
+          items(tst_idx, d.tst0, d.ntst, 6, cnt[2], [&](int i, int k, const int *) { ((int *)(B + pl.tsk))[i] = k; });
+          items(hb_idx, d.hb0, d.nhb, 6, cnt[0], [&](int i, int k, const int *m) {
+            ((int *)(B + pl.hbk))[i] = k;
+            uint32_t *ix = (uint32_t *)(B + pl.hbi) + 3 * i;
             for (int q = 0; q < 6; ++q) {
               ix[q / 2] |= (uint32_t)m[q] << (16 * (q & 1));
-              ((uint32_t *)(B + pl.hbd))[6 * (k - k0) + q] = word(d.slot_hb + 6 * k + q, m[q]);
+              ((uint32_t *)(B + pl.hbd))[6 * i + q] = word(d.slot_hb + 6 * k + q, m[q]);
               const int site = hb_site[6 * (size_t)(d.hb0 + k) + q];
-              ((uint32_t *)(B + pl.hbs))[6 * (k - k0) + q] =
+              ((uint32_t *)(B + pl.hbs))[6 * i + q] =
                   site < 0 ? 0xffffffffu : (uint32_t)site | (uint32_t)std::min(std::max(site_val[d.site0 + site], 0), 254) << 24;
             }
-            Real *cf = (Real *)(B + pl.hbc) + 13 * (k - k0);
+            Real *cf = (Real *)(B + pl.hbc) + 13 * i;
             for (int q = 0; q < 6; ++q) cf[q] = (Real)hb_nat[6 * (size_t)(d.hb0 + k) + q];
             for (int q = 0; q < 7; ++q) cf[6 + q] = (Real)hb_coef[7 * (size_t)(d.hb0 + k) + q];
-          }
+          });
         }
       }
     };
@@ -1273,18 +1286,16 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     CK(cudaMemset(c->d_not_spd.p, 0, nlane * sizeof(int)));
   }
   if (p.i_ele == TIS_ELE_EWALD) {
-    std::vector<int8_t> h;
-    std::vector<double> coef;
-    ewald_table(p.psize[0], p.ewld_alpha, p.ewld_hmax, h, coef);
-    c->nk = (int)coef.size();
+    std::vector<char4> col;
+    std::vector<double> w;
+    ewald_columns(p.psize[0], p.ewld_alpha, p.ewld_hmax, col, w);
+    c->ew_ncol = (int)col.size();
     c->hmax = (int)std::ceil(p.ewld_hmax);
-    c->nqblk = std::min(16, std::max(1, (c->nq_max + 63) / 64));
-    CK(c->ew_h.upload(h));
-    CK(c->ew_coef.upload(coef));
-    CK(c->ew_tab.alloc(std::max<size_t>((size_t)ew_off * 3 * (c->hmax + 1) * 2, 1)));
-    CK(c->ew_S.alloc(std::max<size_t>((size_t)nlane * c->nqblk * c->nk * 2, 1)));
-    CK(c->f_ext.alloc(n3 * EW_F_SPLIT));
-    CK(cudaMemset(c->f_ext.p, 0, n3 * EW_F_SPLIT * 8));
+    CK(c->ew_col.upload(col));
+    CK(c->ew_w.upload(w));
+    CK(c->ew_S.alloc((size_t)nlane * EW_H * c->ew_ncol * 4));
+    CK(c->f_ext.alloc(n3));
+    CK(cudaMemset(c->f_ext.p, 0, n3 * 8));
   }
   c->clamp_seen.assign(nlane, 0);
   *out = c;
@@ -1334,7 +1345,7 @@ extern "C" void tis_destroy(tis_ctx *c) {
   c->out_force.free(); c->out_energy.free(); c->scale.free();
   c->mask.free(); c->site_exc.free(); c->mirror.free(); c->hb_flag.free();
   c->hb_ene.free(); c->hb_flag2.free(); c->hb_ene2.free(); c->site_exc2.free(); c->slots.free(); c->noise.free(); c->unif.free(); c->lane_n.free(); c->d_order.free();
-  c->ew_h.free(); c->ew_coef.free(); c->ew_tab.free(); c->ew_S.free(); c->f_ext.free();
+  c->ew_col.free(); c->ew_w.free(); c->ew_S.free(); c->f_ext.free();
   c->fene_idx.free(); c->wca_idx.free(); c->bd_ptr.free(); c->bd_ent.free(); c->fene_cls.free(); c->wca_cls.free(); c->b_hrad.free(); c->d_not_spd.free();
   c->fene_nat.free(); c->fene_coef.free(); c->fene_d2.free(); c->wca_nat.free(); c->wca_coef.free();
   c->bd_D64.free(); c->bd_z.free(); c->bd_E32.free(); c->bd_W32.free();
@@ -1481,9 +1492,9 @@ KArgs make_args(tis_ctx *c, int mode, int nsteps, int only_lane) {
     a.ewld_alpha = p.ewld_alpha;
     a.ewld_beta = 2.0 * p.ewld_alpha / std::sqrt(F_PI);
     a.ewld_self = -p.ewld_alpha / std::sqrt(F_PI);
-    a.nk = c->nk; a.hmax = c->hmax; a.nqblk = c->nqblk;
-    for (int d = 0; d < 3; ++d) a.two_pi_L[d] = 2.0 * F_PI / p.psize[0];
-    a.ew_h = c->ew_h.p; a.ew_coef = c->ew_coef.p; a.ew_tab = c->ew_tab.p; a.ew_S = c->ew_S.p;
+    a.hmax = c->hmax; a.ew_ncol = c->ew_ncol;
+    a.two_pi_L = 2.0 * F_PI / p.psize[0];
+    a.ew_col = c->ew_col.p; a.ew_w = c->ew_w.p; a.ew_S = c->ew_S.p;
   }
   a.f_ext = nullptr;
   a.fene_idx = c->fene_idx.p; a.fene_nat = c->fene_nat.p; a.fene_coef = c->fene_coef.p; a.fene_d2 = c->fene_d2.p;
@@ -1558,12 +1569,12 @@ KArgs make_args(tis_ctx *c, int mode, int nsteps, int only_lane) {
   return a;
 }
 
-// Ewald reciprocal space for the lanes of `a` (tables, structure factors
-// and, when `forces`, the per-charge forces in f_ext, which the next lane
-// launch adds to each bead's sum).  No-op without Ewald.
+// Ewald reciprocal space for the lanes of `a` (structure factors and, when
+// `forces`, the per-charge forces in f_ext, which the next lane launch adds to
+// each bead's sum).  No-op without Ewald.
 int ewald_recip(tis_ctx *c, KArgs &a, bool forces) {
   if (c->par.i_ele != TIS_ELE_EWALD) return TIS_OK;
-  c->launches += (forces ? 3 : 2) + (c->nqblk > 1 ? 1 : 0);
+  c->launches += forces ? 2 : 1;
   if (forces) a.f_ext = c->f_ext.p;   // written by the force kernel, read by the lane kernel
   CK(ewald_recip_launch(c->stream, a, c->nq_max, forces));
   return TIS_OK;

@@ -19,8 +19,8 @@ namespace tis {
 constexpr int MAX_THREADS = 1024;
 constexpr int N_ETYPE = 25;   // E_TYPE%MAX
 constexpr int CHMAX = 1024;   // electrostatic row chunks per lane (at least one per charged bead)
-constexpr int EW_F_SPLIT = 4; // k ranges of the reciprocal-space forces: f_ext holds one (3, nbead_total)
-                              // plane of partial forces per range, added in range order
+constexpr int EW_H = 12;      // Ewald: hz = 0 .. 11 of a column (hx, hy) of reciprocal vectors
+constexpr int EW_COLS = 192;  // columns of the half space at most (189 for |h| <= 11)
 // HI_TENSOR (const_index.F90:39-45)
 constexpr int TIS_HI_RPY_DEV = 1, TIS_HI_RPY_OVER_DEV = 2, TIS_HI_ERMAK_OVER_DEV = 3, TIS_HI_ZUK_RPY_DEV = 4;
 
@@ -62,7 +62,6 @@ struct LaneDesc {
   int hb0;          // hb flags / status / energies (nhb each)
   int site0;        // per-lane hbond-site excess counters (nsite ints)
   int unif0;        // injected uniform stream (n_uniform per lane)
-  int ew0;          // Ewald: first charge of this lane in the per-lane charge tables
   long long bd0;    // Brownian-HI: first element of this lane's (3N)^2 diffusion / Cholesky matrices
   long long bdp0;   // Brownian-HI, tensor cores: first float of this lane's TF32 panel planes
   long long bd32;   // Brownian-HI, mixed precision: first float of this lane's FP32 D and L (rows padded to 4)
@@ -110,10 +109,10 @@ constexpr int SPLIT_MISC = 16;   // its flag words before the unit table
 struct SplitPlan {
   int own, rows;           // beads (a multiple of 4) and charged rows of a CTA (at most)
   unsigned ecap;           // partner-list entries of a CTA's charged rows that fit
-  int nst, nhb, nba, nbd;  // bonded items of a CTA (at most)
+  int nst, nhb, nba, nbd, nts;   // bonded items of a CTA (at most)
   int np;                  // beads, rounded up to a multiple of 4 (component stride of the positions)
   // constant
-  unsigned tcu, RE, qb, base, rn2, comm, C, scr, iptr, bdi, bdd, bdc, bai, bad, bac, sti, std_, stc, hbi, hbd, hbc, hbs;
+  unsigned tcu, RE, qb, base, rn2, comm, C, scr, iptr, cnt, stk, hbk, tsk, bdi, bdd, bdc, bai, bad, bac, sti, std_, stc, hbi, hbd, hbc, hbs;
   unsigned stat;
   // state and scratch
   unsigned X, P, Q, A4, L3, V, DD, C1, u0, NZ, exF, dhF, NR4, near, ncnt, mexv, mele, slots, exc, hbf, red, img, misc;
@@ -141,14 +140,13 @@ struct KArgs {
   // Ewald (force_ele_coulomb_ewld.F90, mloop_ewld.F90)
   double ewld_alpha, ewld_beta;   // alpha, 2 alpha / sqrt(pi)
   double ewld_self;               // -alpha / sqrt(pi)
-  int nk;                         // reciprocal vectors, all +-h with |h| <= hmax
-  int hmax;                       // ceil(hmax): per-dimension table length - 1
-  int nqblk;                      // charge blocks of the structure-factor partial sums
-  double two_pi_L[3];             // 2 pi / L
-  const int8_t *ew_h;             // (nk, 3) integer h
-  const double *ew_coef;          // (nk) 2 pi / L^3 exp(-k^2 / 4 alpha^2) / k^2
-  double *ew_tab;                 // (q, 3, hmax + 1) of (cos, sin)(2 pi h x / L), per lane's charges
-  double *ew_S;                   // (lane, nqblk, nk, 2) partial sums of q cos, q sin
+  int hmax;                       // ceil(hmax)
+  int ew_ncol;                    // columns (hx, hy) of the half space of reciprocal vectors
+  double two_pi_L;                // 2 pi / L
+  const char4 *ew_col;            // (ncol) hx, hy, largest hz; longest columns first
+  const double *ew_w;             // (EW_H, ncol) weight of +-hz: 2 C(k) (hz = 0: C(k)), C(k) = 2 pi / L^3
+                                  // exp(-k^2 / 4 alpha^2) / k^2; half for the column (0, 0)
+  double *ew_S;                   // (lane, EW_H, ncol, 4) structure-factor sums of +-hz
   double *f_ext;                  // (3, nbead_total) force added to each bead's sum, or null
   // Brownian dynamics with hydrodynamic interactions (time_integral.F90:429-457)
   const int *fene_idx; const double *fene_nat, *fene_coef, *fene_d2;   // force_fene.F90

@@ -20,11 +20,14 @@ static __device__ unsigned long long g_phase[128];
 #endif
 // per-warp spans by kind of work of CTA 0: total at 32 + k, count at 48 + k
 #define PHASE_KIND(k, t0) do { if (blockIdx.x == 0 && (threadIdx.x & 31) == 0) { const int k_ = (k); atomicAdd(&g_phase[32 + k_], (unsigned long long)(clock64() - (t0))); atomicAdd(&g_phase[48 + k_], 1ull); } } while (0)
+// spans of thread 0 of the first 16 CTAs
+#define PHASE_CTA(base, t0) do { if (threadIdx.x == 0 && blockIdx.x < 16) atomicAdd(&g_phase[(base) + blockIdx.x], (unsigned long long)(clock64() - (t0))); } while (0)
 // per-warp spans of the first two CTAs: slots base + 16 blockIdx.x + warp
 #define PHASE_WARP(base, t0) do { if (blockIdx.x < 2 && (threadIdx.x & 31) == 0) atomicAdd(&g_phase[(base) + 16 * blockIdx.x + (threadIdx.x >> 5)], (unsigned long long)(clock64() - (t0))); } while (0)
 #else
 #define PHASE_WARP(base, t0) do {} while (0)
 #define PHASE_KIND(k, t0) do {} while (0)
+#define PHASE_CTA(base, t0) do {} while (0)
 #define PHASE_ALL(k, t0) do {} while (0)
 #define PHASE_T0(v) do {} while (0)
 #define PHASE_ADD(k, t0) do {} while (0)
@@ -385,13 +388,19 @@ __device__ void term_bond(const KArgs &a, const TopDesc &T, const S &s, const Ds
   put_slot<Real>(slots, 2 * k + 1, m[1], f * v.x, f * v.y, f * v.z);
 }
 
-// force_bangle.F90:103-147: the forces of one angle's beads
-template <typename Real>
-__device__ __forceinline__ void angle_force(R3<Real> v21, R3<Real> v32, Real nat, Real cf, R3<Real> *f3) {
+// force_bangle.F90:103-147
+template <typename Real, typename S, typename Dst>
+__device__ void term_angle(const KArgs &a, const TopDesc &T, const S &s, const Dst &slots, int k) {
+  const size_t sb = T.slot_ba + 3 * (size_t)k;
+  const Real cf = (Real)ldro(a.ba_coef + T.ba0 + k);
+  const int *mp = a.ba_idx + 3 * (size_t)(T.ba0 + k);
+  const int m[3] = {ldro(mp), ldro(mp + 1), ldro(mp + 2)};
   if (cf < (Real)1.0e-6) {
-    f3[0] = f3[1] = f3[2] = R3<Real>{0, 0, 0};
+    put_slot<Real>(slots, sb, m[0], 0, 0, 0); put_slot<Real>(slots, sb + 1, m[1], 0, 0, 0);
+    put_slot<Real>(slots, sb + 2, m[2], 0, 0, 0);
     return;
   }
+  R3<Real> v21 = dvec<Real>(s, m[0], m[1]), v32 = dvec<Real>(s, m[1], m[2]);
   Real c11 = dot(v21, v21), c22 = dot(v32, v32), c21 = dot(v32, v21);
   Real co = -c21 * frsq(c11 * c22);
   if (co > (Real)1) co = 1; else if (co < (Real)-1) co = -1;
@@ -408,27 +417,15 @@ __device__ __forceinline__ void angle_force(R3<Real> v21, R3<Real> v32, Real nat
     th = acos(co);
     t3 = c11 * c22 - c21 * c21;
   }
-  Real dba = th - nat;
+  Real dba = th - (Real)ldro(a.ba_nat + T.ba0 + k);
   if (t3 <= (Real)1) t3 = 1;
   Real f = (Real)2 * cf * dba * frsq(t3);
   Real a1 = fdiv(c21, c11), a2 = fdiv(c21, c22);
   R3<Real> f21{f * (v21.x * a1 - v32.x), f * (v21.y * a1 - v32.y), f * (v21.z * a1 - v32.z)};
   R3<Real> f32{f * (v32.x * a2 - v21.x), f * (v32.y * a2 - v21.y), f * (v32.z * a2 - v21.z)};
-  f3[0] = R3<Real>{-f21.x, -f21.y, -f21.z};
-  f3[1] = R3<Real>{f21.x - f32.x, f21.y - f32.y, f21.z - f32.z};
-  f3[2] = f32;
-}
-
-template <typename Real, typename S, typename Dst>
-__device__ void term_angle(const KArgs &a, const TopDesc &T, const S &s, const Dst &slots, int k) {
-  const size_t sb = T.slot_ba + 3 * (size_t)k;
-  const Real cf = (Real)ldro(a.ba_coef + T.ba0 + k);
-  const int *mp = a.ba_idx + 3 * (size_t)(T.ba0 + k);
-  const int m[3] = {ldro(mp), ldro(mp + 1), ldro(mp + 2)};
-  R3<Real> f[3];
-  angle_force<Real>(dvec<Real>(s, m[0], m[1]), dvec<Real>(s, m[1], m[2]), (Real)ldro(a.ba_nat + T.ba0 + k), cf, f);
-#pragma unroll
-  for (int p = 0; p < 3; ++p) put_slot<Real>(slots, sb + p, m[p], f[p].x, f[p].y, f[p].z);
+  put_slot<Real>(slots, sb, m[0], -f21.x, -f21.y, -f21.z);
+  put_slot<Real>(slots, sb + 1, m[1], f21.x - f32.x, f21.y - f32.y, f21.z - f32.z);
+  put_slot<Real>(slots, sb + 2, m[2], f32.x, f32.y, f32.z);
 }
 
 // st_status of secondary stack k (force_dtrna_stack_nlocal.F90:83-92): off

@@ -1,183 +1,161 @@
 // ewald_kernel.cu -- reciprocal-space Ewald sums on the device, FP64
 // (force_ele_coulomb_ewld.F90:62-84 forces, energy_ele_coulomb_ewld.F90:75-89
-// energy, k table of mloop_ewld.F90:56-156).
+// energy, k vectors of mloop_ewld.F90:56-156).
 //
 // For a charge at x, e^{i k.x} with k = 2 pi (hx, hy, hz) / L factorises
-// into e^{i 2 pi hx x / L} e^{i 2 pi hy y / L} e^{i 2 pi hz z / L}.  A first
-// kernel tabulates (cos, sin)(2 pi h x_d / L) for h = 0..hmax per charge and
-// dimension (negative h by conjugation), so every (k, charge) term costs two
-// complex products instead of a sincos:
+// into e^{i 2 pi hx x / L} e^{i 2 pi hy y / L} e^{i 2 pi hz z / L} = (a + i b)
+// (c + i d), with (c, d) of -hz the conjugate of hz's.  The vectors are taken
+// by columns (hx, hy) of the half space hx > 0, or hx = 0 and hy >= 0 (-k adds
+// the same force and energy as k, so sums over it are doubled; the column
+// (0, 0) holds both k and -k and weighs half).  For the pair +-hz of a column
+// the four sums over the charges
+//   P = sum q a c   Q = sum q b d   R = sum q a d   T = sum q b c
+// give both structure factors, S(+-hz) = (P -+ Q) + i (T +- R): four products
+// a charge for two vectors, and as many for their force on a charge.
 //
-//   ewald_tab_kernel    per charge: 3 (hmax + 1) sincos
-//   ewald_sk_kernel     per k and charge block: partial S_c(k) = sum q cos,
-//                       S_s(k) = sum q sin (charges in ascending order)
-//   ewald_sk_sum_kernel S(k) = the charge-block partials summed in block order
-//   ewald_force_kernel  per charge (one warp) and k range (EW_F_SPLIT of
-//                       them): partial F = sum_k coef 2 C(k) q (sin S_c -
-//                       cos S_s) k, added by the lane kernel in range order
-//   ewald_energy_kernel per lane: coef (sum_k C(k) (S_c^2 + S_s^2) + self)
+//   ewald_sk_kernel     one block per column: threads over the charges, the
+//                       column's sums in registers, one reduction at the end
+//   ewald_force_kernel  one block per few charges: a thread per column keeps
+//                       its sums, weighted, in registers for all of them
+//   ewald_energy_kernel per lane: coef (sum_k C(k) |S(k)|^2 + self)
+//
+// A table of the charges' exponentials, structure factors per block of 64
+// charges with a kernel that adds them, and forces by k range of one vector
+// at a time took 8.9 + 14.6 + 5.4 + 19.5 us for 641 charges and 4,168 vectors
+// (four launches; 8.8 + 9.8 + 3.2 + 12.7 us for 165 charges): ten times the
+// FP64 work of the column form and four dependent launches.
 //
 // All sums run in a fixed order, so the results do not depend on scheduling.
+#include <algorithm>
+
 #include "device_common.cuh"
 
 namespace tis {
 
-constexpr int EW_SK_THREADS = 256;   // k vectors per structure-factor block
-constexpr int EW_SK_QCHUNK = 64;     // charges staged in shared memory at a time
+constexpr int EW_SK_THREADS = 128;
+constexpr int EW_F_MAXQ = 8;   // charges of a force block at most
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-// table entry for integer h (negative h: complex conjugate)
-__device__ __forceinline__ double2 tab_get(const double2 *t, int h) {
-  const double2 v = t[h < 0 ? -h : h];
-  return make_double2(v.x, h < 0 ? -v.y : v.y);
-}
-
-// grid (ceil(nq / 128), nlane): tab[(ew0 + kq) * 3 + d][h] = (cos, sin)(2 pi h x_d / L)
-__global__ void __launch_bounds__(128) ewald_tab_kernel(KArgs a) {
-  const int lane = (a.only_lane >= 0) ? a.only_lane : (int)blockIdx.y;
-  if (lane >= a.nlane) return;
-  const LaneDesc L = a.lanes[lane];
-  const TopDesc T = a.tops[L.top];
-  const int kq = blockIdx.x * blockDim.x + threadIdx.x;
-  if (kq >= T.nq) return;
-  const int bead = a.q_bead[T.q0 + kq];
-  const double *p = a.pxyz + 3 * (size_t)(L.state0 + bead);
-  const int H = a.hmax + 1;
-  double2 *t = (double2 *)a.ew_tab + (size_t)(L.ew0 + kq) * 3 * H;
-  for (int d = 0; d < 3; ++d) {
-    const double th = a.two_pi_L[d] * p[d];
-    for (int h = 0; h < H; ++h) {
-      double sn, cs;
-      sincos((double)h * th, &sn, &cs);
-      t[d * H + h] = make_double2(cs, sn);
-    }
-  }
-}
-
-// grid (ceil(nk / 256), nqblk, nlane)
+// grid (columns, lanes): S[(lane 12 + h) ncol + col] = (P, Q, R, T) of +-h
 __global__ void __launch_bounds__(EW_SK_THREADS) ewald_sk_kernel(KArgs a) {
-  const int lane = (a.only_lane >= 0) ? a.only_lane : (int)blockIdx.z;
-  if (lane >= a.nlane) return;
-  const LaneDesc L = a.lanes[lane];
-  const TopDesc T = a.tops[L.top];
-  const int H = a.hmax + 1;
-  const int k = blockIdx.x * EW_SK_THREADS + threadIdx.x;
-  const bool kv = k < a.nk;
-  int hx = 0, hy = 0, hz = 0;
-  if (kv) { hx = a.ew_h[3 * k]; hy = a.ew_h[3 * k + 1]; hz = a.ew_h[3 * k + 2]; }
-  // charges of this block: [q_lo, q_hi)
-  const int per = (T.nq + a.nqblk - 1) / a.nqblk;
-  const int q_lo = blockIdx.y * per, q_hi = min(T.nq, q_lo + per);
-  __shared__ double2 tab[EW_SK_QCHUNK * 3 * 12];
-  __shared__ double qv[EW_SK_QCHUNK];
-  double sc = 0.0, ss = 0.0;
-  const double2 *gt = (const double2 *)a.ew_tab + (size_t)L.ew0 * 3 * H;
-  for (int q0 = q_lo; q0 < q_hi; q0 += EW_SK_QCHUNK) {
-    const int nqc = min(EW_SK_QCHUNK, q_hi - q0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < nqc * 3 * H; e += EW_SK_THREADS) tab[e] = gt[(size_t)q0 * 3 * H + e];
-    for (int e = threadIdx.x; e < nqc; e += EW_SK_THREADS)
-      qv[e] = a.b_charge[T.bead0 + a.q_bead[T.q0 + q0 + e]];
-    __syncthreads();
-    if (kv) {
-      for (int c = 0; c < nqc; ++c) {
-        const double2 *t = tab + c * 3 * H;
-        const double2 e = cmul(cmul(tab_get(t, hx), tab_get(t + H, hy)), tab_get(t + 2 * H, hz));
-        sc += qv[c] * e.x;
-        ss += qv[c] * e.y;
-      }
-    }
-  }
-  if (kv) {
-    double *S = a.ew_S + (((size_t)lane * a.nqblk + blockIdx.y) * a.nk + k) * 2;
-    S[0] = sc;
-    S[1] = ss;
-  }
-}
-
-// grid (ceil(nk / 256), nlane): S(k) = sum of the charge-block partials in
-// block order, stored in block 0's slot
-__global__ void __launch_bounds__(256) ewald_sk_sum_kernel(KArgs a) {
   const int lane = (a.only_lane >= 0) ? a.only_lane : (int)blockIdx.y;
   if (lane >= a.nlane) return;
-  const int k = blockIdx.x * 256 + threadIdx.x;
-  if (k >= a.nk) return;
-  double *S = a.ew_S + (size_t)lane * a.nqblk * a.nk * 2;
-  double sc = S[2 * (size_t)k], ss = S[2 * (size_t)k + 1];
-  for (int b = 1; b < a.nqblk; ++b) {
-    sc += S[((size_t)b * a.nk + k) * 2];
-    ss += S[((size_t)b * a.nk + k) * 2 + 1];
+  const LaneDesc L = a.lanes[lane];
+  const TopDesc T = a.tops[L.top];
+  const char4 col = a.ew_col[blockIdx.x];   // hx, hy, largest hz
+  const double hx = (double)col.x * a.two_pi_L, hy = (double)col.y * a.two_pi_L;
+  const int mz = col.z;
+  double P[EW_H], Q[EW_H], R[EW_H], U[EW_H];
+#pragma unroll
+  for (int h = 0; h < EW_H; ++h) P[h] = Q[h] = R[h] = U[h] = 0.0;
+  for (int k = threadIdx.x; k < T.nq; k += EW_SK_THREADS) {
+    const int bead = a.q_bead[T.q0 + k];
+    const double *x = a.pxyz + 3 * (size_t)(L.state0 + bead);
+    const double q = a.b_charge[T.bead0 + bead];
+    double sx, cx, sy, cy, s1, c1;
+    sincos(hx * x[0], &sx, &cx);
+    sincos(hy * x[1], &sy, &cy);
+    sincos(a.two_pi_L * x[2], &s1, &c1);
+    const double ca = q * (cx * cy - sx * sy), cb = q * (cx * sy + sx * cy);
+    P[0] += ca; U[0] += cb;
+    double c = c1, d = s1;
+#pragma unroll
+    for (int h = 1; h < EW_H; ++h) {
+      if (h > mz) break;
+      P[h] = fma(ca, c, P[h]); Q[h] = fma(cb, d, Q[h]); R[h] = fma(ca, d, R[h]); U[h] = fma(cb, c, U[h]);
+      const double c2 = c * c1 - d * s1;   // e^{i (h + 1) z}
+      d = fma(c, s1, d * c1);
+      c = c2;
+    }
   }
-  S[2 * (size_t)k] = sc;
-  S[2 * (size_t)k + 1] = ss;
+  constexpr int NWRP = EW_SK_THREADS / 32;
+  __shared__ double red[NWRP][4 * EW_H];
+  const int lid = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int h = 0; h < EW_H; ++h) {
+    if (h > mz) break;
+    double v[4] = {P[h], Q[h], R[h], U[h]};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+      if (lid == 0) red[warp][4 * h + q] = v[q];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 4 * (mz + 1)) {
+    double v = 0.0;
+    for (int w = 0; w < NWRP; ++w) v += red[w][threadIdx.x];
+    a.ew_S[(((size_t)lane * EW_H + (threadIdx.x >> 2)) * a.ew_ncol + blockIdx.x) * 4 + (threadIdx.x & 3)] = v;
+  }
 }
 
-constexpr int EW_F_KCHUNK = 512;     // k vectors staged in shared memory at a time
-
-// grid (ceil(nq / 8), EW_F_SPLIT, nlane), 256 threads: one warp per charge
-// over k range blockIdx.y; the CTA stages its 8 charges' tables and
-// (S_c, S_s, C(k), h) of EW_F_KCHUNK vectors at a time
-constexpr int EW_TAB_MAX = 3 * 16;   // 3 (hmax + 1) table entries per charge staged (hmax <= 15)
-__global__ void __launch_bounds__(256) ewald_force_kernel(KArgs a) {
-  const int lane = (a.only_lane >= 0) ? a.only_lane : (int)blockIdx.z;
+// grid (ceil(nq / per), lanes), one thread per column (rounded up to whole
+// warps): the forces of `per` charges
+__global__ void __launch_bounds__(EW_COLS) ewald_force_kernel(KArgs a, int per) {
+  const int lane = (a.only_lane >= 0) ? a.only_lane : (int)blockIdx.y;
   if (lane >= a.nlane) return;
   const LaneDesc L = a.lanes[lane];
   const TopDesc T = a.tops[L.top];
-  const int H = a.hmax + 1;
-  const int warp = threadIdx.x >> 5, lid = threadIdx.x & 31;
-  const int kq = blockIdx.x * 8 + warp;
-  const bool qv = kq < T.nq;
-  const int bead = qv ? a.q_bead[T.q0 + kq] : 0;
-  const double q = qv ? a.b_charge[T.bead0 + bead] : 0.0;
-  const double coefT = a.lab_coef[a.lstate[lane].label];
-  const double *S = a.ew_S + (size_t)lane * a.nqblk * a.nk * 2;
-  __shared__ double2 sT[8 * EW_TAB_MAX];
-  __shared__ double2 sS[EW_F_KCHUNK];
-  __shared__ double sC[EW_F_KCHUNK];
-  __shared__ char4 sH[EW_F_KCHUNK];
-  const bool staged = 3 * H <= EW_TAB_MAX;
-  const double2 *t = staged ? sT + warp * EW_TAB_MAX
-                            : (const double2 *)a.ew_tab + (size_t)(L.ew0 + (qv ? kq : 0)) * 3 * H;
-  if (staged && qv) {
-    const double2 *g = (const double2 *)a.ew_tab + (size_t)(L.ew0 + kq) * 3 * H;
-    for (int e = lid; e < 3 * H; e += 32) sT[warp * EW_TAB_MAX + e] = g[e];
-  }
-  const int ka = (int)((long long)a.nk * blockIdx.y / EW_F_SPLIT);
-  const int kb = (int)((long long)a.nk * (blockIdx.y + 1) / EW_F_SPLIT);
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  for (int k0 = ka; k0 < kb; k0 += EW_F_KCHUNK) {
-    const int nkc = min(EW_F_KCHUNK, kb - k0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < nkc; e += blockDim.x) {
-      const int k = k0 + e;
-      sS[e] = make_double2(S[2 * (size_t)k], S[2 * (size_t)k + 1]);
-      sC[e] = a.ew_coef[k];
-      sH[e] = make_char4(a.ew_h[3 * k], a.ew_h[3 * k + 1], a.ew_h[3 * k + 2], 0);
-    }
-    __syncthreads();
-    if (qv) {
-      for (int e = lid; e < nkc; e += 32) {
-        const char4 h = sH[e];
-        const double2 ex = cmul(cmul(tab_get(t, h.x), tab_get(t + H, h.y)), tab_get(t + 2 * H, h.z));
-        const double2 sk = sS[e];
-        // qs * scos - qc * ssin (force_ele_coulomb_ewld.F90:74-80)
-        const double dv = coefT * 2.0 * sC[e] * (q * ex.y * sk.x - q * ex.x * sk.y);
-        fx += dv * (a.two_pi_L[0] * h.x);
-        fy += dv * (a.two_pi_L[1] * h.y);
-        fz += dv * (a.two_pi_L[2] * h.z);
-      }
+  const int k0 = blockIdx.x * per, nk = min(per, T.nq - k0);
+  if (nk <= 0) return;
+  const int tid = threadIdx.x, lid = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  __shared__ double2 ex[EW_F_MAXQ][3][EW_H];   // (cos, sin)(2 pi h x_d / L) of the block's charges
+  __shared__ double red[EW_COLS / 32][EW_F_MAXQ][3];
+  for (int e = tid; e < nk * 3 * EW_H; e += blockDim.x) {
+    const int q = e / (3 * EW_H), d = (e / EW_H) % 3, h = e % EW_H;
+    if (h <= a.hmax) {
+      const double x = a.pxyz[3 * (size_t)(L.state0 + a.q_bead[T.q0 + k0 + q]) + d];
+      double sn, cs;
+      sincos((double)h * (a.two_pi_L * x), &sn, &cs);
+      ex[q][d][h] = make_double2(cs, sn);
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    fx += __shfl_xor_sync(0xffffffffu, fx, o);
-    fy += __shfl_xor_sync(0xffffffffu, fy, o);
-    fz += __shfl_xor_sync(0xffffffffu, fz, o);
+  // this column's weighted sums
+  const bool on = tid < a.ew_ncol;
+  const char4 col = on ? a.ew_col[tid] : make_char4(0, 0, -1, 0);
+  const int mz = col.z, mw = __reduce_max_sync(0xffffffffu, mz);
+  double p[EW_H], r[EW_H], s[EW_H], t[EW_H];
+#pragma unroll
+  for (int h = 0; h < EW_H; ++h) {
+    p[h] = r[h] = s[h] = t[h] = 0.0;
+    if (h <= mz) {
+      const double *S = a.ew_S + (((size_t)lane * EW_H + h) * a.ew_ncol + tid) * 4;
+      const double w = a.ew_w[h * a.ew_ncol + tid];
+      p[h] = w * S[0]; s[h] = -(w * S[1]); t[h] = w * S[2]; r[h] = w * S[3];
+    }
   }
-  if (qv && lid == 0) {
-    double *f = a.f_ext + 3 * ((size_t)blockIdx.y * a.nbead_total + L.state0 + bead);
-    f[0] = fx; f[1] = fy; f[2] = fz;
+  __syncthreads();
+  for (int q = 0; q < nk; ++q) {
+    const double2 vx = ex[q][0][col.x], vy0 = ex[q][1][abs(col.y)];
+    const double sy = col.y < 0 ? -vy0.y : vy0.y;
+    const double ca = vx.x * vy0.x - vx.y * sy, cb = fma(vx.x, sy, vx.y * vy0.x);
+    double g1 = p[0], g2 = -r[0], h1 = 0.0, h2 = 0.0;
+#pragma unroll
+    for (int h = 1; h < EW_H; ++h) {
+      if (h > mw) break;   // the warp's longest column (sums beyond a column's own are zero)
+      const double2 z = ex[q][2][h];
+      const double c = z.x, d = z.y, ch = (double)h * c, dh = (double)h * d;
+      g1 = fma(c, p[h], fma(d, t[h], g1));
+      g2 = fma(d, s[h], fma(-c, r[h], g2));
+      h1 = fma(ch, s[h], fma(dh, r[h], h1));
+      h2 = fma(dh, p[h], fma(-ch, t[h], h2));
+    }
+    const double dv = fma(cb, g1, ca * g2), dz = fma(cb, h1, ca * h2);
+    double f[3] = {dv * (double)col.x, dv * (double)col.y, dz};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      for (int o = 16; o > 0; o >>= 1) f[d] += __shfl_xor_sync(0xffffffffu, f[d], o);
+      if (lid == 0) red[warp][q][d] = f[d];
+    }
+  }
+  __syncthreads();
+  if (tid < 3 * nk) {
+    const int q = tid / 3, d = tid - 3 * q;
+    const int bead = a.q_bead[T.q0 + k0 + q];
+    double f = 0.0;
+    for (int w = 0; w < nw; ++w) f += red[w][q][d];
+    // dv of a vector: coef 2 C(k) q (sin S_c - cos S_s) (force_ele_coulomb_ewld.F90:74-80), twice for -k
+    const double coef = 4.0 * a.lab_coef[a.lstate[lane].label] * a.b_charge[T.bead0 + bead] * a.two_pi_L;
+    a.f_ext[3 * (size_t)(L.state0 + bead) + d] = coef * f;
   }
 }
 
@@ -189,11 +167,12 @@ __global__ void __launch_bounds__(256) ewald_energy_kernel(KArgs a) {
   const LaneDesc L = a.lanes[lane];
   const TopDesc T = a.tops[L.top];
   const int label = (a.elabel && a.elabel[lane] >= 0) ? a.elabel[lane] : a.lstate[lane].label;
-  const double *S = a.ew_S + (size_t)lane * a.nqblk * a.nk * 2;
   double ef = 0.0, qq = 0.0;
-  for (int k = threadIdx.x; k < a.nk; k += blockDim.x) {
-    const double sc = S[2 * (size_t)k], ss = S[2 * (size_t)k + 1];
-    ef += a.ew_coef[k] * (sc * sc + ss * ss);
+  for (int k = threadIdx.x; k < EW_H * a.ew_ncol; k += blockDim.x) {
+    const int h = k / a.ew_ncol, col = k - h * a.ew_ncol;
+    if (h > a.ew_col[col].z) continue;
+    const double *S = a.ew_S + ((size_t)lane * EW_H * a.ew_ncol + k) * 4;
+    ef += 2.0 * a.ew_w[k] * ((S[0] * S[0] + S[1] * S[1]) + (S[2] * S[2] + S[3] * S[3]));
   }
   for (int kq = threadIdx.x; kq < T.nq; kq += blockDim.x) {
     const double q = a.b_charge[T.bead0 + a.q_bead[T.q0 + kq]];
@@ -216,15 +195,17 @@ __global__ void __launch_bounds__(256) ewald_energy_kernel(KArgs a) {
   }
 }
 
-// Launches tab, structure factors and forces (into f_ext) for one lane
+// Launches structure factors and forces (into f_ext) for one lane
 // (only_lane >= 0) or every lane.  nq_max: largest charge count of a lane.
 cudaError_t ewald_recip_launch(cudaStream_t st, const KArgs &a, int nq_max, bool forces) {
   if (forces && !a.f_ext) return cudaErrorInvalidValue;
   const int nl = a.only_lane >= 0 ? 1 : a.nlane;
-  ewald_tab_kernel<<<dim3((nq_max + 127) / 128, nl), 128, 0, st>>>(a);
-  ewald_sk_kernel<<<dim3((a.nk + EW_SK_THREADS - 1) / EW_SK_THREADS, a.nqblk, nl), EW_SK_THREADS, 0, st>>>(a);
-  if (a.nqblk > 1) ewald_sk_sum_kernel<<<dim3((a.nk + 255) / 256, nl), 256, 0, st>>>(a);
-  if (forces) ewald_force_kernel<<<dim3((nq_max + 7) / 8, EW_F_SPLIT, nl), 256, 0, st>>>(a);
+  ewald_sk_kernel<<<dim3(a.ew_ncol, nl), EW_SK_THREADS, 0, st>>>(a);
+  if (forces && nq_max > 0) {
+    // as few charges a block as still fill the chip once
+    const int per = std::min(EW_F_MAXQ, std::max(1, (int)(((long long)nq_max * nl + 147) / 148)));
+    ewald_force_kernel<<<dim3((nq_max + per - 1) / per, nl), (a.ew_ncol + 31) / 32 * 32, 0, st>>>(a, per);
+  }
   return cudaGetLastError();
 }
 

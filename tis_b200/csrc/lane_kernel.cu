@@ -831,8 +831,7 @@ __device__ void force_pass(const KArgs &a, int lane, const LaneDesc &L, const To
     if (valid) {
       for (int d = g; d < 3; d += GA) {
         double f = d == 0 ? fx : (d == 1 ? fy : fz);
-        if (a.f_ext)   // the reciprocal-space partial forces, in k-range order
-          for (int p = 0; p < EW_F_SPLIT; ++p) f += a.f_ext[3 * ((size_t)p * a.nbead_total + L.state0 + i) + d];
+        if (a.f_ext) f += a.f_ext[3 * ((size_t)L.state0 + i) + d];   // the reciprocal-space force
         sink(i, d, f);
       }
     }
@@ -1033,7 +1032,11 @@ __global__ void __launch_bounds__(NT) lane_kernel(KArgs a) {
         const V av = s.A4N[i];
         const float ex = (float)av.x - s.NR4[i].x, ey = (float)av.y - s.NR4[i].y, ez = (float)av.z - s.NR4[i].z;
         const float e2 = ex * ex + ey * ey + ez * ez;
-        if (!(e2 <= NEAR_DISP_MAX * NEAR_DISP_MAX)) atomicMax(&s.misc[f_disp], 0x7f000000);
+        // both CTAs record anew: the other one's lists hold this bead too
+        if (!(e2 <= NEAR_DISP_MAX * NEAR_DISP_MAX)) {
+          atomicMax(&s.misc[f_disp], 0x7f000000);
+          atomicMax(&peer_ptr(s.misc, cu)[f_disp], 0x7f000000);
+        }
       }
     };
     // the first step's x update; the later ones run in the v / a update of

@@ -10,11 +10,13 @@
 //
 // Each CTA keeps the positions and pair parameters of every bead and owns a
 // contiguous block of beads: their velocities and accelerations, excluded-
-// volume rows and near lists, incidence slots and updates.  The charged rows
-// of the electrostatic list, the bonded items and the hydrogen bonds are
-// divided evenly by index instead, whatever beads they touch, so an ion box
-// (bonded terms on a few beads, charges on all) is balanced too; their
-// results go to the CTA that owns the bead through distributed shared memory.
+// volume rows and near lists, incidence slots and updates, and the bonded
+// items whose first bead is one of them (divided by index instead, most of
+// their results were remote stores of single values, and the barrier that
+// waits for them took 9.3 k of a 400-nt step's 36 k cycles).  The charged
+// rows of the electrostatic list are divided evenly, so an ion box (charges
+// on every bead) is balanced too.  Results for another CTA's bead go there
+// through distributed shared memory.
 //
 // One step is two phases between cluster barriers:
 //   sweep   bonded terms, electrostatic rows, exv near lists, noise: warps
@@ -27,8 +29,8 @@
 //           so the reads are contiguous and need no index), add the row sums
 //           and update v / a and x; then whole warps copy the block's new
 //           positions to the other CTAs, 16 bytes a thread (stores of single
-//           values cost ~2 cycles each on the SM-to-SM network: 15.8 k ->
-//           12.0 k cycles of the 400-nt update).
+//           values cost ~2 cycles each on the SM-to-SM network), and only
+//           the parts that the forces read (28 or 32 bytes a bead).
 // Positions are not double buffered: nothing reads them in the update phase.
 // A step whose lists must be rebuilt first does so from the old positions
 // between its two halves, with one more barrier.
@@ -83,7 +85,9 @@ __device__ __forceinline__ void put_word(Real *slots, int rank, uint32_t w, R3<R
   }
 }
 
-// shared memory of a CTA: every bead's positions and pair parameters
+// shared memory of a CTA: every bead's positions and pair parameters.  A4
+// (with L3) is what a step sends and reads; the FP64 X and P of the other
+// CTAs' beads are brought up to date only for a list build
 template <typename Real>
 struct SplitSmem {
   double *X, *Y, *Z, *PX, *PY, *PZ, *QX, *QY, *QZ;
@@ -92,6 +96,24 @@ struct SplitSmem {
   Real *RE;                // exv radius, sqrt(eps)
   uint32_t *tcu;           // type | class << 8 | unit << 16
 };
+
+// pxyz of any bead from the copies that every step refreshes
+template <typename Real>
+struct SplitCoord {
+  const Real *A4;          // component d of bead i at 4 i
+  const float *L3;
+  __device__ double operator[](int i) const {
+    if constexpr (sizeof(Real) == 4) return (double)A4[4 * i] + (double)L3[3 * i];
+    else return A4[4 * i];
+  }
+};
+template <typename Real>
+struct SplitView { SplitCoord<Real> PX, PY, PZ; };
+template <typename Real>
+__device__ __forceinline__ SplitView<Real> split_view(const SplitSmem<Real> &s) {
+  const Real *A = (const Real *)s.A4;
+  return SplitView<Real>{{A, s.L3}, {A + 1, s.L3 + 1}, {A + 2, s.L3 + 2}};
+}
 
 template <typename Real>
 __device__ __forceinline__ void split_pos(const SplitSmem<Real> &s, int i, double x, double y, double z) {
@@ -128,22 +150,41 @@ __device__ __forceinline__ double diff_img(double a, double b, double k, double 
 // the deviation from nat, and the derivative terms of the four beads, as
 // force_dtrna_stack.F90:92-150 and force_dtrna_hbond15.F90:205-340 write
 // them.  CAP: the hydrogen bonds' cap of nearly straight triples (maxc).
+//
+// Sums of products are written with their rounding (a b - c d = fma(a, b,
+// -rn(c d)) and so on): left to the compiler, the variants of the kernel fuse
+// one or the other product, and a lane's bits would depend on its number of
+// CTAs.
+__device__ __forceinline__ float mulr(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mulr(double a, double b) { return __dmul_rn(a, b); }
+// a b + c d of the integration: FP64 as the reference evaluates it (see mad2)
+template <typename Real> __device__ __forceinline__ double smad(double a, double b, double c, double d) {
+  return sizeof(Real) == 8 ? __dadd_rn(__dmul_rn(a, b), __dmul_rn(c, d)) : fma(a, b, __dmul_rn(c, d));
+}
+template <typename Real> __device__ __forceinline__ Real det2(Real a, Real b, Real c, Real d) { return fma(a, b, -mulr(c, d)); }
+template <typename Real> __device__ __forceinline__ Real sq3(Real x, Real y, Real z) { return fma(z, z, fma(y, y, mulr(x, x))); }
+template <typename Real> __device__ __forceinline__ Real sdot(R3<Real> a, R3<Real> b) {
+  return fma(a.z, b.z, fma(a.y, b.y, mulr(a.x, b.x)));
+}
+template <typename Real> __device__ __forceinline__ R3<Real> cross(R3<Real> a, R3<Real> b) {
+  return R3<Real>{det2(a.y, b.z, a.z, b.y), det2(a.z, b.x, a.x, b.z), det2(a.x, b.y, a.y, b.x)};
+}
 template <typename Real> struct Dih { R3<Real> a, b, c, d; Real e; bool straight; };
 template <typename Real, bool CAP>
 __device__ __forceinline__ Dih<Real> dihedral(R3<Real> u, R3<Real> w, R3<Real> z, Real nat, Real k, Real maxc) {
   Dih<Real> o;
-  const R3<Real> m = crs(u, w), n = crs(w, z);
-  const Real w2 = dot(w, w), uw = dot(u, w), zw = dot(z, w);
-  Real m2 = dot(m, m), n2 = dot(n, n);
+  const R3<Real> m = cross(u, w), n = cross(w, z);
+  const Real w2 = sdot(w, w), uw = sdot(u, w), zw = sdot(z, w);
+  Real m2 = sdot(m, m), n2 = sdot(n, n);
   if (CAP) {   // |cos| > maxc, compared as squares
-    const Real uw2 = dot(u, u) * w2, zw2 = dot(z, z) * w2, mc2 = maxc * maxc;
+    const Real uw2 = sdot(u, u) * w2, zw2 = sdot(z, z) * w2, mc2 = maxc * maxc;
     if (uw * uw > mc2 * uw2) m2 = uw2 * ((Real)1 - mc2);
     if (zw * zw > mc2 * zw2) n2 = zw2 * ((Real)1 - mc2);
     o.straight = false;
   } else {
     // mixed stacks: within ~2 degrees of straight FP32 is not enough (see term_stack)
     const Real lim = (Real)1e-3;
-    o.straight = sizeof(Real) == 4 && (m2 < lim * dot(u, u) * w2 || n2 < lim * w2 * dot(z, z));
+    o.straight = sizeof(Real) == 4 && (m2 < lim * sdot(u, u) * w2 || n2 < lim * w2 * sdot(z, z));
   }
   Real aw, ou, oz, im2, in2;   // |w|, uw / w2, zw / w2, 1 / m2, 1 / n2
   if constexpr (sizeof(Real) == 8) {
@@ -154,14 +195,14 @@ __device__ __forceinline__ Dih<Real> dihedral(R3<Real> u, R3<Real> w, R3<Real> z
   } else {
     aw = sqrt(w2); ou = fdiv(uw, w2); oz = fdiv(zw, w2); im2 = fdiv((Real)1, m2); in2 = fdiv((Real)1, n2);
   }
-  const Real d = wrap_pi(atan2(dot(u, n) * aw, dot(m, n)) - nat);
-  o.e = k * d * d;
+  const Real d = wrap_pi(atan2(sdot(u, n) * aw, sdot(m, n)) - nat);
+  o.e = mulr(mulr(k, d), d);
   const Real pre = (Real)2 * k * d * aw, gi = pre * im2, gl = -pre * in2;
   o.a = R3<Real>{gi * m.x, gi * m.y, gi * m.z};
   o.d = R3<Real>{gl * n.x, gl * n.y, gl * n.z};
   const Real b1 = (Real)-1 + ou, c1 = (Real)-1 + oz;
-  o.b = R3<Real>{b1 * o.a.x - oz * o.d.x, b1 * o.a.y - oz * o.d.y, b1 * o.a.z - oz * o.d.z};
-  o.c = R3<Real>{c1 * o.d.x - ou * o.a.x, c1 * o.d.y - ou * o.a.y, c1 * o.d.z - ou * o.a.z};
+  o.b = R3<Real>{det2(b1, o.a.x, oz, o.d.x), det2(b1, o.a.y, oz, o.d.y), det2(b1, o.a.z, oz, o.d.z)};
+  o.c = R3<Real>{det2(c1, o.d.x, ou, o.a.x), det2(c1, o.d.y, ou, o.a.y), det2(c1, o.d.z, ou, o.a.z)};
   return o;
 }
 __device__ __forceinline__ float invsqrt(float x) { return rsqrtf(x); }
@@ -181,6 +222,33 @@ template <typename Real> __device__ __forceinline__ R3<Real> sel3(bool c, R3<Rea
 template <typename Real> __device__ __forceinline__ R3<Real> shx3(R3<Real> a, int o) {
   return R3<Real>{__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o),
                   __shfl_xor_sync(0xffffffffu, a.z, o)};
+}
+
+// force_bangle.F90:103-147: the forces of one angle's beads (see term_angle)
+template <typename Real>
+__device__ __forceinline__ void split_angle(R3<Real> v21, R3<Real> v32, Real nat, Real cf, R3<Real> *f3) {
+  const Real c11 = sdot(v21, v21), c22 = sdot(v32, v32), c21 = sdot(v32, v21), rs = invsqrt(c11 * c22);
+  Real co = -c21 * rs;
+  if (co > (Real)1) co = 1; else if (co < (Real)-1) co = -1;
+  Real th, t3;
+  if (sizeof(Real) == 4 && fabs(co) > (Real)0.99) {
+    const R3<Real> cr = cross(v21, v32);
+    t3 = sdot(cr, cr);
+    th = atan2(sqrt(t3), -c21);
+  } else {
+    th = acos(co);
+    t3 = det2(c11, c22, c21, c21);
+  }
+  if (t3 <= (Real)1) t3 = 1;
+  const Real f = cf < (Real)1.0e-6 ? (Real)0 : (Real)2 * cf * (th - nat) * invsqrt(t3);
+  Real a1, a2;
+  if constexpr (sizeof(Real) == 8) { const Real r2 = rs * rs; a1 = c21 * c22 * r2; a2 = c21 * c11 * r2; }
+  else { a1 = fdiv(c21, c11); a2 = fdiv(c21, c22); }
+  const R3<Real> A{fma(v21.x, a1, -v32.x), fma(v21.y, a1, -v32.y), fma(v21.z, a1, -v32.z)};
+  const R3<Real> B{fma(v32.x, a2, -v21.x), fma(v32.y, a2, -v21.y), fma(v32.z, a2, -v21.z)};
+  f3[0] = mul3(-f, A);
+  f3[1] = mul3(f, R3<Real>{A.x - B.x, A.y - B.y, A.z - B.z});
+  f3[2] = mul3(f, B);
 }
 
 // asynchronous copies global -> shared, all in flight together
@@ -241,7 +309,9 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   uint8_t *hbf = (uint8_t *)(sm + pl.hbf);
   const double *rn2 = (double *)(sm + pl.rn2);
   double *red = (double *)(sm + pl.red), *redc = red + 64;
-  int *dmax = (int *)(redc + 2 * SPLIT_MAX);   // [parity][CTA]: largest dot_product(dxyz, dxyz), float bits rounded up
+  // [parity][CTA], float bits: largest dot_product(dxyz, dxyz), rounded up; largest squared displacement
+  // since the near lists were recorded
+  int2 *dmax = (int2 *)(redc + 2 * SPLIT_MAX);
   float4 *imgf = (float4 *)(sm + pl.img);
   double4 *imgd = (double4 *)(sm + pl.img);
   int *misc = (int *)(sm + pl.misc);
@@ -252,18 +322,16 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   const SplitDst<Real> dst{slots, a.slot_pos + T.sp0, base, magic};
   // this CTA's share of the charged rows and of each kind of bonded item
   const int kq_lo = min(NQ, rank * rows), nrow = min(NQ, kq_lo + rows) - kq_lo;
-  const int h0 = split_share(T.nhb, nr, rank), nh = split_share(T.nhb, nr, rank + 1) - h0;
-  const int st0 = split_share(T.nst, nr, rank), nst = split_share(T.nst, nr, rank + 1) - st0;
-  const int ts0 = split_share(T.ntst, nr, rank), nts = split_share(T.ntst, nr, rank + 1) - ts0;
-  const int nba = split_share(T.nba, nr, rank + 1) - split_share(T.nba, nr, rank);
-  const int nbd = split_share(T.nbd, nr, rank + 1) - split_share(T.nbd, nr, rank);
+  const unsigned char *comm = a.split_blob + T.sp_blob, *mine = comm + (size_t)rank * (pl.stat - pl.comm);
+  const int *cnt = (const int *)(mine + pl.cnt);   // bonded items of this CTA
+  const int nh = ldro(cnt), nst = ldro(cnt + 1), nts = ldro(cnt + 2), nba = ldro(cnt + 3), nbd = ldro(cnt + 4);
+  const int *hbk = (const int *)(sm + pl.hbk), *stk = (const int *)(sm + pl.stk), *tsk = (const int *)(sm + pl.tsk);
   const int label = st.label;
   const long long istep0 = st.istep;   // written by CTA 0 after the last cluster barrier
 
   // ---- load: every copy is asynchronous, so the arrays' latencies overlap
   const bool lists_new = a.mode == KM_NEIGHBOR || a.mode == KM_PRE;
   {
-    const unsigned char *comm = a.split_blob + T.sp_blob, *mine = comm + (size_t)rank * (pl.stat - pl.comm);
     for (unsigned q = 16 * tid; q < pl.stat; q += 16 * NT) acopy16(sm + q, (q < pl.comm ? comm : mine) + q);
     const size_t o = 3 * (size_t)L.state0;
     for (int q = tid; q < 3 * N; q += NT) {
@@ -277,9 +345,9 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
       acopy8(Vv + k, a.velo + g); acopy8(Av + k, a.accel + g);
       if (skin) acopy8(Dv + k, a.dxyz + g);
     }
-    const double *c1 = a.lab_c1 + a.lab_c1off[label] + lo, *u0 = a.lab_u0 + a.lab_u0off[label] + st0;
+    const double *c1 = a.lab_c1 + a.lab_c1off[label] + lo, *u0 = a.lab_u0 + a.lab_u0off[label];
     for (int li = tid; li < nown; li += NT) acopy8(C1 + li, c1 + li);
-    for (int k = tid; k < nst; k += NT) acopy8((double *)u0s + k, u0 + k);
+    for (int k = tid; k < nst; k += NT) acopy8((double *)u0s + k, u0 + ldro((const int *)(mine + pl.stk) + k));
     if (!lists_new) {
       const uint32_t *gm = a.mask + L.mask0;
       for (int k = tid; k < nown * W; k += NT) acopy4(mexv + k, gm + (size_t)lo * W + k);
@@ -292,9 +360,9 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     for (int k = tid; k < 3 * T.sp_ninc; k += NT) slots[k] = (Real)0;
     for (int k = tid; k < 3 * OS; k += NT) dhF[k] = 0.0;
     for (int k = tid; k < T.nsite; k += NT) exc[k] = 0;
-    for (int k = tid; k < nh; k += NT) hbf[k] = a.hb_flag[L.hb0 + h0 + k];
+    for (int k = tid; k < nh; k += NT) hbf[k] = a.hb_flag[L.hb0 + ldro((const int *)(mine + pl.hbk) + k)];
     if (tid < SPLIT_MISC) misc[tid] = tid == MISC_NEAR_BAD ? 1 : (tid == MISC_CHUNK ? NW : 0);
-    if (tid < 2 * SPLIT_MAX) dmax[tid] = 0;
+    if (tid < 2 * SPLIT_MAX) dmax[tid] = make_int2(0, 0);
     if (PER && tid < 27) {   // the shift of each image as multiples of the box
       const int c[3] = {tid % 3, (tid / 3) % 3, tid / 9};
       auto k = [](int q) { return q == 0 ? 0.0 : (q == 1 ? -1.0 : 1.0); };
@@ -324,6 +392,32 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
 
   const bool ewald = a.i_ele == 2, coul = a.i_ele == 3;
   const int LQ = split_row_lanes(NQ, ewald), RW = 32 / LQ;
+  // x_j - x_i of the bonded terms in W (nearest image when periodic: the
+  // chain's own, as its beads are close); in FP32 from the hi and lo parts,
+  // rounded once
+  auto rvec = [&](auto w, int i, int j) SPLIT_INL {
+    typedef decltype(w) Wt;
+    const V p = s.A4[i], q = s.A4[j];
+    if constexpr (sizeof(Wt) == 4) {
+      const float *l = s.L3 + 3 * i, *m = s.L3 + 3 * j;
+      auto d1 = [&](float x, float y, float lx, float ly, int d) SPLIT_INL {
+        const float t = y - x, bb = t - y, e = (y - (t - bb)) + (-x - bb) + (ly - lx);
+        if (!PER) return t + e;
+        const float h = (float)a.psizeh[d], k = t > h ? -1.0f : (t < -h ? 1.0f : 0.0f);
+        const float Lh = (float)a.psize[d], Ll = (float)(a.psize[d] - (double)Lh);
+        return fmaf(k, Lh, t) + fmaf(k, Ll, e);
+      };
+      return R3<Wt>{d1(p.x, q.x, l[0], m[0], 0), d1(p.y, q.y, l[1], m[1], 1), d1(p.z, q.z, l[2], m[2], 2)};
+    } else {
+      double x = (double)q.x - (double)p.x, y = (double)q.y - (double)p.y, z = (double)q.z - (double)p.z;
+      if constexpr (sizeof(Real) == 4) {
+        const float *l = s.L3 + 3 * i, *m = s.L3 + 3 * j;
+        x += (double)m[0] - (double)l[0]; y += (double)m[1] - (double)l[1]; z += (double)m[2] - (double)l[2];
+      }
+      if (PER) { pb1(x, a.psize[0], a.psizeh[0]); pb1(y, a.psize[1], a.psizeh[1]); pb1(z, a.psize[2], a.psizeh[2]); }
+      return R3<Wt>{x, y, z};
+    }
+  };
   // partner lists of the charged rows from their bit rows (with the image of
   // each pair when periodic): lane l expands words l, l + 32, ...
   // (called by the whole CTA; misc[MISC_ELIST]: they fit)
@@ -380,7 +474,24 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   // tests one own row, lane l bead 32 w + l, and writes its words by ballot;
   // mixed precision screens in FP32 and takes the FP64 test of the reference
   // only within the rounding of the screen
-  auto build = [&](long long is) SPLIT_INL {
+  auto build = [&](long long is, bool loaded) SPLIT_INL {
+    if (!loaded) {
+      // the FP64 positions of the other CTAs' beads (nobody moves beads now)
+      bool units = false;   // the unit prescreen sums unwrapped positions
+      if (PER)
+        for (int u = 0, n = 0; u < nu; ++u) { n += a.u_class[T.unit0 + u] != 4; units = n > 1; }
+      for (int i = tid; i < N; i += NT) {
+        const int r = (int)__umulhi((unsigned)i, magic);
+        if (r == rank) continue;
+        const double *P = cl.map_shared_rank(s.PX, r);
+        s.PX[i] = P[i]; s.PY[i] = P[np + i]; s.PZ[i] = P[2 * np + i];
+        if (PER && units) {
+          const double *X = cl.map_shared_rank(s.X, r);
+          s.X[i] = X[i]; s.Y[i] = X[np + i]; s.Z[i] = X[2 * np + i];
+        }
+      }
+      cl.sync();   // (the owners wrap theirs below)
+    }
     if (PER) {
       for (int i = tid; i < N; i += NT) {
         const double x = wrap1(s.PX[i], a.psize[0]), y = wrap1(s.PY[i], a.psize[1]), z = wrap1(s.PZ[i], a.psize[2]);
@@ -528,7 +639,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     if (nele) atomicAdd(&misc[MISC_NELE], nele);
     // hbond neighbour flags (neighbor_list_hb.F90:335-354)
     for (int k = tid; k < nh; k += NT) {
-      const int h = h0 + k, *m = a.hb_idx + 6 * (size_t)(T.hb0 + h);
+      const int h = hbk[k], *m = a.hb_idx + 6 * (size_t)(T.hb0 + h);
       const int m0 = ldro(m), m1 = ldro(m + 1);
       double v0 = __dsub_rn(s.PX[m0], s.PX[m1]), v1 = __dsub_rn(s.PY[m0], s.PY[m1]), v2 = __dsub_rn(s.PZ[m0], s.PZ[m1]);
       if (PER) { pb1(v0, a.psize[0], a.psizeh[0]); pb1(v1, a.psize[1], a.psizeh[1]); pb1(v2, a.psize[2], a.psizeh[2]); }
@@ -580,7 +691,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     const int i = lo + li;
     if (valid && g < 3) {
       const int q = g * OS + li;
-      const double dx = mad2<Real>(C4[li], Vv[q], a.tstep2, Av[q]);
+      const double dx = smad<Real>(C4[li], Vv[q], a.tstep2, Av[q]);
       const double nx = s.X[g * np + i] + dx;
       s.X[g * np + i] = nx;
       double p = nx;
@@ -591,18 +702,20 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
       if constexpr (sizeof(Real) == 4) s.L3[3 * i + g] = (float)(p - (double)h);
     }
     __syncwarp();
-    int bits = 0;
+    int bits = 0, nbits = 0;   // float bits, order-preserving for values >= 0
     if (valid && g == 0) {
       const V p = s.A4[i];
       const float4 r = NR4[li];
-      const float ex = (float)p.x - r.x, ey = (float)p.y - r.y, ez = (float)p.z - r.z;
-      if (!(ex * ex + ey * ey + ez * ez <= NEAR_DISP_MAX * NEAR_DISP_MAX)) misc[MISC_NEAR_DISP + par] = 1;
+      const float ex = (float)p.x - r.x, ey = (float)p.y - r.y, ez = (float)p.z - r.z, e2 = sq3(ex, ey, ez);
+      nbits = e2 >= 0.0f ? __float_as_int(e2) : 0x7f000000;   // (before the first recording NR4 holds anything)
       if (skin) {
         const double d2 = disp2(Dv[li], Dv[OS + li], Dv[2 * OS + li]);
         DD[li] = d2;
-        bits = __float_as_int(__double2float_ru(d2));   // order-preserving for d2 >= 0
+        bits = __float_as_int(__double2float_ru(d2));
       }
     }
+    nbits = __reduce_max_sync(0xffffffffu, nbits);
+    if (lid == 0) atomicMax(&misc[MISC_NEAR_DISP], nbits);
     if (skin) {
       bits = __reduce_max_sync(0xffffffffu, bits);
       if (lid == 0) atomicMax(&misc[MISC_DMAX], bits);
@@ -612,36 +725,30 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   // 16 bytes per thread, whole warps per CTA: scattered stores of single
   // values cost ~2 cycles each on the SM-to-SM network
   auto send = [&](int par) SPLIT_INL {
+    PHASE_T0(t_y);
     __syncthreads();
+    PHASE_ADD(13, t_y);
     constexpr int PV = sizeof(V) / 16;
-    const int n0 = own / 2, nA = own * PV, nL = sizeof(Real) == 4 ? own * 3 / 4 : 0, nX = PER ? 6 * n0 : 3 * n0;
-    const int avail = ((N + 3) & ~3) - lo;   // beads behind lo (a multiple of 4): the last block is shorter
-    const int m0 = min(n0, max(avail, 0) / 2), mA = min(nA, max(avail, 0) * PV), mL = min(nL, max(avail, 0) * 3 / 4);
+    const int avail = max(((N + 3) & ~3) - lo, 0);   // beads from lo on: the last block is shorter
+    const int nA = min(own, avail) * PV, nL = sizeof(Real) == 4 ? min(own, avail) * 3 / 4 : 0;
     const int per = max(1, NW / (nr - 1));
     for (int t = nown > 0 ? warp : 1 << 20; t < (nr - 1) * per; t += NW) {
       const int r = (rank + 1 + t % (nr - 1)) % nr, sub = t / (nr - 1);
       unsigned char *peer = cl.map_shared_rank(sm, r);
-      for (int q = sub * 32 + lid; q < nX; q += per * 32) {
-        const int c = q / n0, k = q - c * n0;
-        if (k < m0) {
-          const unsigned off = (c < 3 ? pl.X : pl.P) + 8 * ((c % 3) * np + lo) + 16 * k;
-          *(uint4 *)(peer + off) = *(const uint4 *)(sm + off);
-        }
-      }
-      for (int q = sub * 32 + lid; q < mA; q += per * 32) {
+      for (int q = sub * 32 + lid; q < nA; q += per * 32) {
         const unsigned off = pl.A4 + (unsigned)sizeof(V) * lo + 16 * q;
         *(uint4 *)(peer + off) = *(const uint4 *)(sm + off);
       }
-      for (int q = sub * 32 + lid; q < mL; q += per * 32) {
+      for (int q = sub * 32 + lid; q < nL; q += per * 32) {
         const unsigned off = pl.L3 + 12 * lo + 16 * q;
         *(uint4 *)(peer + off) = *(const uint4 *)(sm + off);
       }
     }
-    if (skin && warp == 0) {
-      const int bits = misc[MISC_DMAX];
+    if (warp == 0) {
+      const int2 m = make_int2(misc[MISC_DMAX], misc[MISC_NEAR_DISP]);
       __syncwarp();
-      if (lid == 0) misc[MISC_DMAX] = 0;
-      if (lid < nr) cl.map_shared_rank(dmax, lid)[par * SPLIT_MAX + rank] = bits;
+      if (lid == 0) { misc[MISC_DMAX] = 0; misc[MISC_NEAR_DISP] = 0; }
+      if (lid < nr) cl.map_shared_rank(dmax, lid)[par * SPLIT_MAX + rank] = m;
     }
   };
 
@@ -666,13 +773,13 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     const V pj = s.A4[j];
     Real sx, sy, sz;
     pair_diff(pi, pj, img, sx, sy, sz);
-    if (sx * sx + sy * sy + sz * sz > scr2) return;
+    if (sq3(sx, sy, sz) > scr2) return;
     Real wx = sx, wy = sy, wz = sz;
     if constexpr (sizeof(Real) == 4) {
       wx = sx + (s.L3[3 * j] - s.L3[3 * i]); wy = sy + (s.L3[3 * j + 1] - s.L3[3 * i + 1]);
       wz = sz + (s.L3[3 * j + 2] - s.L3[3 * i + 2]);
     }
-    const Real r2 = wx * wx + wy * wy + wz * wz;
+    const Real r2 = sq3(wx, wy, wz);
     const int ti = typ(i), ci = cls(i), tj = typ(j), cj = cls(j);
     const Real bix = s.RE[2 * i], bjx = s.RE[2 * j];
     // contact rule: 0 base-base / RNA-RNA, 1 phosphate-sugar, 2 radius sum (DT19: force_exv_dt15.F90:60-66)
@@ -681,20 +788,20 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     const Real dij = rule == 0 ? dist_rr : (rule == 1 ? dist_ps : bix + bjx);
     if (r2 > dij * dij) return;
     Real rinv = invsqrt(r2);
-    Real dr = r2 * rinv + ra - dij;
+    Real dr = fma(r2, rinv, ra) - dij;
     if (sizeof(Real) == 4 && dr < (Real)1.5) {
       // the steep part of the potential: distance and dr in FP64 (see lane_kernel.cu)
       const double ex = (double)sx + ((double)s.L3[3 * j] - (double)s.L3[3 * i]);
       const double ey = (double)sy + ((double)s.L3[3 * j + 1] - (double)s.L3[3 * i + 1]);
       const double ez = (double)sz + ((double)s.L3[3 * j + 2] - (double)s.L3[3 * i + 2]);
-      const double d64 = sqrt(ex * ex + ey * ey + ez * ez);
+      const double d64 = sqrt(sq3(ex, ey, ez));
       const double dij64 = rule == 0 ? a.exv_dist : (rule == 1 ? a.exv_dist_PS : (double)bix + (double)bjx);
       rinv = (Real)(1.0 / d64);
       dr = (Real)(d64 + a.exv_adjust - dij64);
     }
     const Real coef = s.RE[2 * i + 1] * s.RE[2 * j + 1];
     const Real ro2 = fdiv(ra2, dr * dr);
-    const Real ro4 = ro2 * ro2, ro8 = ro4 * ro4, ro14 = ro2 * ro4 * ro8;
+    const Real ro4 = ro2 * ro2, ro8 = mulr(ro4, ro4), ro14 = mulr(ro2 * ro4, ro8);
     Real f = fabs((Real)12 * coef * (ro14 - ro8) * dr * inv_ra2 * rinv);
     // DE_MAX clamp; each pair is visited from both beads and counted once
     if (f > (Real)50) { f = 50; nclamp += j > i; }
@@ -711,7 +818,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     const V pj = s.A4[j];
     Real x, y, z;
     pair_diff(pi, pj, PER ? e >> SP_IMG : 0, x, y, z);
-    const Real r2 = x * x + y * y + z * z;
+    const Real r2 = sq3(x, y, z);
     const Real ri = invsqrt(r2);
     const Real d = r2 * ri;
     Real f;
@@ -719,7 +826,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
       f = qci * pj.w * ri * ri * ri;   // force_ele_coulomb.F90:66-71 (no clamp)
     } else if constexpr (KIND == 2) {
       // force_ele_coulomb_ewld.F90:118-137 (no clamp); pairs past the cutoff add nothing
-      f = (r2 <= cut2) ? qci * pj.w * (erfc(ew_a * d) * ri + ew_b * exp(-ew_a2 * r2)) * ri * ri : (Real)0;
+      f = (r2 <= cut2) ? qci * pj.w * fma((Real)erfc(ew_a * d), ri, mulr(ew_b, (Real)exp(-ew_a2 * r2))) * ri * ri : (Real)0;
     } else {
       f = qci * pj.w * ri * ri * (ri + rcd) * fexp<Real>(-d * rcd);   // force_ele_DH.F90:72-117
       if (KIND == 3 && pmf_row && j != np && mg_p_pair(typ(i), typ(j)) && (double)d <= a.pmf_rmax) {
@@ -776,12 +883,11 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     }
   };
 
-  auto sweep = [&](long long istep, int noise_step, int par) SPLIT_INL {
+  auto sweep = [&](long long istep, int noise_step, int par, bool rec) SPLIT_INL {
     const int f_exc = MISC_EXCESS + par;
-    const bool rec = misc[MISC_NEAR_BAD] != 0 || misc[MISC_NEAR_DISP + par] != 0;
     // flags of the next step: their last readers passed the barrier before this sweep, and
     // they are set only behind the one after it
-    if (tid == 0) { misc[MISC_EXCESS + (par ^ 1)] = 0; misc[MISC_NEAR_DISP + (par ^ 1)] = 0; }
+    if (tid == 0) misc[MISC_EXCESS + (par ^ 1)] = 0;
     const int c_end = c_nz + (noise_step >= 0 ? n_nz : 0);
     int c = warp;
     PHASE_T0(t_s);
@@ -792,7 +898,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
       if (c >= c_ex && c < c_ba) {
         // exv of 32 / SG own beads, SG threads each: thread g takes the
         // partners j with j % SG == g, in ascending order.  A recording pass
-        // keeps those within the screen radius + NEAR_SKIN; later passes
+        // keeps those within the screen radius + SP_SKIN; later passes
         // visit only these (partners further off add nothing, so the sums
         // are the same bits)
         const int li = (c - c_ex) * (32 / SG) + lid / SG, i = lo + li;
@@ -808,7 +914,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
           uint32_t m = 0;
           do {
             if (scan) {   // the next (at most SP_NEAR) near partners from the row's bits
-              const Real nscr = sr + (Real)NEAR_SKIN, nscr2 = nscr * nscr;
+              const Real nscr = sr + (Real)SP_SKIN, nscr2 = nscr * nscr;
               for (n = 0; n < SP_NEAR;) {
                 while (m == 0 && w < W) m = mexv[li * W + w++] & (0x01010101u << g);
                 if (m == 0) { more = false; break; }
@@ -821,11 +927,11 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
                   Real cx = fabs(x), cy = fabs(y), cz = fabs(z);
                   cx = min(cx, (Real)fabs((Real)a.psize[0] - cx)); cy = min(cy, (Real)fabs((Real)a.psize[1] - cy));
                   cz = min(cz, (Real)fabs((Real)a.psize[2] - cz));
-                  if (cx * cx + cy * cy + cz * cz > nscr2 + (Real)0.1) continue;
+                  if (sq3(cx, cy, cz) > nscr2 + (Real)0.1) continue;
                   img = split_image(a, s, i, j);
                   pair_diff(pi, pj, img, x, y, z);
                 }
-                if (x * x + y * y + z * z <= nscr2) lst[n++] = (uint16_t)(PER ? (j | (img << SP_IMG)) : j);
+                if (sq3(x, y, z) <= nscr2) lst[n++] = (uint16_t)(PER ? (j | (img << SP_IMG)) : j);
               }
               if (rec && first) {
                 ncnt[li * SG + g] = (uint8_t)(more ? 0xFF : n);
@@ -856,18 +962,18 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
         const int m[7] = {(int)(ix.x & 0xffff), (int)(ix.x >> 16), (int)(ix.y & 0xffff), (int)(ix.y >> 16),
                           (int)(ix.z & 0xffff), (int)(ix.z >> 16), (int)(ix.w & 0xffff)};
         const double u0 = u0s[k];
-        const bool off = stack_excluded<Real>(a, T, s, st0 + k), live = k0 < nst;
+        const bool off = T.ntst > 0 && stack_excluded<Real>(a, T, split_view(s), stk[k]), live = k0 < nst;
         // the stack in W (nat and coef of its distance, then of this thread's
         // dihedral): forces of beads 0 / 1, 2 / 6, 3 / 5 and (thread 0) 4;
         // true when a triple is too straight for FP32
         auto stack = [&](bool mine, auto w, auto n0, auto k1, auto nat, auto kd) SPLIT_INL {
           typedef decltype(w) Wt;
-          const R3<Wt> v21 = dvec<Wt>(s, m[0], m[1]), v54 = dvec<Wt>(s, m[3], m[4]), v56 = dvec<Wt>(s, m[5], m[4]);
-          const R3<Wt> u = dvec<Wt>(s, role ? m[5] : m[3], role ? m[6] : m[2]);
+          const R3<Wt> v21 = rvec(Wt(), m[0], m[1]), v54 = rvec(Wt(), m[3], m[4]), v56 = rvec(Wt(), m[5], m[4]);
+          const R3<Wt> u = rvec(Wt(), role ? m[5] : m[3], role ? m[6] : m[2]);
           const Dih<Wt> o = dihedral<Wt, false>(u, sel3(role != 0, v56, v54), sel3(role != 0, v54, v56), nat, kd, (Wt)1);
           const int other = __shfl_xor_sync(0xffffffffu, (int)o.straight, 1);   // every lane takes part
           Wt dist, rdist;
-          length(dot(v21, v21), dist, rdist);
+          length(sdot(v21, v21), dist, rdist);
           const Wt dd = dist - n0;
           const Wt ediv = (Wt)1 + k1 * dd * dd + (o.e + __shfl_xor_sync(0xffffffffu, o.e, 1));
           const R3<Wt> fb = add3(o.b, shx3(o.d, 1)), fc = add3(o.c, shx3(o.c, 1));
@@ -888,7 +994,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
         const bool bad = stack(live, (Real)0, cf[0], cf[3], cf[1 + role], cf[4 + role]);
         if constexpr (sizeof(Real) == 4)
           if (__any_sync(0xffffffffu, bad)) {   // those in FP64, from the FP64 tables (see term_stack)
-            const double *nd = a.st_nat + 3 * (size_t)(T.st0 + st0 + k), *cd = a.st_coef + 3 * (size_t)(T.st0 + st0 + k);
+            const double *nd = a.st_nat + 3 * (size_t)(T.st0 + stk[k]), *cd = a.st_coef + 3 * (size_t)(T.st0 + stk[k]);
             stack(bad, 0.0, ldro(nd), ldro(cd), ldro(nd + 1 + role), ldro(cd + 1 + role));
           }
       } else if (c >= c_ba && c < c_bd) {
@@ -898,9 +1004,9 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
           const uint32_t *dw = (const uint32_t *)(sm + pl.bad) + 3 * k;
           const Real nat = ((const Real *)(sm + pl.bac))[2 * k], cf = ((const Real *)(sm + pl.bac))[2 * k + 1];
           const int m1 = (int)(ix.x >> 16);
-          const R3<Real> v21 = dvec<Real>(s, (int)(ix.x & 0xffff), m1), v32 = dvec<Real>(s, m1, (int)ix.y);
+          const R3<Real> v21 = rvec(Real(), (int)(ix.x & 0xffff), m1), v32 = rvec(Real(), m1, (int)ix.y);
           R3<Real> f[3];
-          angle_force<Real>(v21, v32, nat, cf, f);
+          split_angle<Real>(v21, v32, nat, cf, f);
 #pragma unroll
           for (int p = 0; p < 3; ++p) put_word(slots, rank, dw[p], f[p]);
         }
@@ -910,9 +1016,9 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
           const uint32_t ix = ((const uint32_t *)(sm + pl.bdi))[k];
           const uint32_t *dw = (const uint32_t *)(sm + pl.bdd) + 2 * k;
           const Real nat = ((const Real *)(sm + pl.bdc))[2 * k], cf = ((const Real *)(sm + pl.bdc))[2 * k + 1];
-          const R3<Real> v = dvec<Real>(s, (int)(ix & 0xffff), (int)(ix >> 16));
+          const R3<Real> v = rvec(Real(), (int)(ix & 0xffff), (int)(ix >> 16));
           Real dist, rdist;
-          length(v.x * v.x + v.y * v.y + v.z * v.z, dist, rdist);
+          length(sdot(v, v), dist, rdist);
           const Real f = cf * ((Real)-2.0 * ((dist - nat) * rdist));
           put_word(slots, rank, dw[0], mul3(-f, v));
           put_word(slots, rank, dw[1], mul3(f, v));
@@ -924,26 +1030,20 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
         // 8 hydrogen bonds (force_dtrna_hbond15.F90:91-353), four threads
         // each: one dihedral on each of threads 0..2, the angles on 0 and 1,
         // the distance on 2
-        const int k0 = (c << 3) + (lid >> 2), role = lid & 3, k = min(k0, nh - 1), h = h0 + k;
+        const int k0 = (c << 3) + (lid >> 2), role = lid & 3, k = min(k0, nh - 1), h = hbk[k];
         const uint32_t *ix = (const uint32_t *)(sm + pl.hbi) + 3 * k, *dw = (const uint32_t *)(sm + pl.hbd) + 6 * k;
         const Real *cf = (const Real *)(sm + pl.hbc) + 13 * k;   // nat (6), coef (7)
         const int m[6] = {(int)(ix[0] & 0xffff), (int)(ix[0] >> 16), (int)(ix[1] & 0xffff), (int)(ix[1] >> 16),
                           (int)(ix[2] & 0xffff), (int)(ix[2] >> 16)};
         const uint8_t f = k0 < nh ? hbf[k] : (uint8_t)0;
-        double w0 = s.PX[m[0]] - s.PX[m[1]], w1 = s.PY[m[0]] - s.PY[m[1]], w2 = s.PZ[m[0]] - s.PZ[m[1]];
-        if (PER) { pb1(w0, a.psize[0], a.psizeh[0]); pb1(w1, a.psize[1], a.psizeh[1]); pb1(w2, a.psize[2], a.psizeh[2]); }
-        const R3<Real> v12{(Real)w0, (Real)w1, (Real)w2};
+        const R3<Real> v12 = rvec(Real(), m[1], m[0]);
         Real a12, r12;
-        length(dot(v12, v12), a12, r12);
+        length(sdot(v12, v12), a12, r12);
         const Real d12 = a12 - cf[0];
         const bool act = (f & 1) && !(fabs((double)d12) > a.hb_cutoff_dist);
         Real e = 0;
         if (__any_sync(0xffffffffu, act)) {
-          auto dv = [&](int p, int q) SPLIT_INL {   // x_p - x_q with minimum image when periodic
-            double z0 = s.X[p] - s.X[q], z1 = s.Y[p] - s.Y[q], z2 = s.Z[p] - s.Z[q];
-            if (PER) { pb1(z0, a.psize[0], a.psizeh[0]); pb1(z1, a.psize[1], a.psizeh[1]); pb1(z2, a.psize[2], a.psizeh[2]); }
-            return R3<Real>{(Real)z0, (Real)z1, (Real)z2};
-          };
+          auto dv = [&](int p, int q) SPLIT_INL { return rvec(Real(), q, p); };   // x_p - x_q
           const Real MAXC = (Real)a.max_abscos;
           const R3<Real> v13 = dv(m[0], m[2]), v42 = dv(m[3], m[1]);
           const R3<Real> ve = dv(role == 1 ? m[4] : m[3], role == 1 ? m[2] : m[5]);   // v53 or v46
@@ -954,7 +1054,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
           Dih<Real> o = dihedral<Real, true>(u, w, z, cf[3 + min(role, 2)], cf[10 + min(role, 2)], MAXC);
           // angles 3-1=2 (vectors v13, v12) and 1=2-4 (v12, v42, opposite sign)
           const R3<Real> p = sel3(r1, v12, v13), q = sel3(r1, v42, v12);
-          const Real p2 = dot(p, p), q2 = dot(q, q), pq = dot(p, q);
+          const Real p2 = sdot(p, p), q2 = sdot(q, q), pq = sdot(p, q);
           Real apq, co, cp, cq;   // |p| |q|, the cosine, pq / p2, pq / q2
           if constexpr (sizeof(Real) == 8) {
             const Real r = rsqrt(p2 * q2), r2 = r * r;
@@ -964,18 +1064,19 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
           }
           const Real pqc = fabs(co) > MAXC ? (Real)copysign(apq * MAXC, co) : pq;
           const Real da = acos(co > (Real)1 ? (Real)1 : (co < (Real)-1 ? (Real)-1 : co)) - cf[r1 ? 2 : 1], ca = role < 2 ? cf[r1 ? 9 : 8] : (Real)0;
-          const Real pre = (r1 ? (Real)-2 : (Real)2) * ca * da * invsqrt(p2 * q2 - pqc * pqc);
+          const Real pre = (r1 ? (Real)-2 : (Real)2) * ca * da * invsqrt(det2(p2, q2, pqc, pqc));
           const bool live = role < 2;   // threads 2 and 3 add no angle term (their angle may be capped to 0 / 0)
           const R3<Real> zero{0, 0, 0};
-          const R3<Real> fi = live ? R3<Real>{pre * (q.x - cp * p.x), pre * (q.y - cp * p.y), pre * (q.z - cp * p.z)} : zero;
-          const R3<Real> fk = live ? R3<Real>{pre * (p.x - cq * q.x), pre * (p.y - cq * q.y), pre * (p.z - cq * q.z)} : zero;
+          const R3<Real> A{fma(-cp, p.x, q.x), fma(-cp, p.y, q.y), fma(-cp, p.z, q.z)};
+          const R3<Real> B{fma(-cq, q.x, p.x), fma(-cq, q.y, p.y), fma(-cq, q.z, p.z)};
+          const R3<Real> fi = live ? mul3(pre, A) : zero, fk = live ? mul3(pre, B) : zero;
+          const R3<Real> fik = live ? mul3(-pre, add3(A, B)) : zero;
           Real ex = -o.e;
-          if (role < 2) ex -= ca * da * da;
-          if (role == 2) ex -= cf[7] * d12 * d12;
+          if (role < 2) ex -= mulr(mulr(ca, da), da);
+          if (role == 2) ex -= mulr(mulr(cf[7], d12), d12);
           if (role == 3) { ex = 0; o.a = o.b = o.c = o.d = zero; }
           const Real gd = role == 2 ? (Real)2 * cf[7] * d12 * r12 : (Real)0;
           // the thread's share of the forces of beads 1..4 (5 is thread 1's alone, 6 thread 2's)
-          const R3<Real> fik{-fi.x - fk.x, -fi.y - fk.y, -fi.z - fk.z};
           R3<Real> b1 = add3(add3(r2 ? o.a : o.c, r1 ? fi : fik), mul3(gd, v12));
           R3<Real> b2 = add3(add3(r1 ? o.d : o.b, r1 ? fik : fk), mul3(-gd, v12));
           R3<Real> b3 = add3(role == 0 ? o.d : (r1 ? o.b : zero), r1 ? zero : fi);
@@ -1020,19 +1121,25 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
       } else {
         const int k = ((c - c_ts) << 5) + lid;
         if (k < nts) {
-          const SplitSmem<Real> s2 = s;
+          const SplitView<Real> s2 = split_view(s);   // copies: the values used elsewhere stay in registers
           const TopDesc T2 = T;
           const SplitDst<Real> d2 = dst;
-          term_tstack<Real>(a, T2, s2, d2, ts0 + k);
+          term_tstack<Real>(a, T2, s2, d2, tsk[k]);
         }
       }
       PHASE_KIND(c < c_ts ? 1 : c < c_st ? 0 : c < c_dh ? 2 : c < c_ex ? 3 : c < c_ba ? 4 : c < c_bd ? 5 : c < c_nz ? 6 : 7, t_c);
       c = __shfl_sync(0xffffffffu, cn, 0);
     }
     PHASE_ADD(1, t_s);
+#ifdef TIS_PHASE_TIMING
+    if (lid == 0) atomicMax(&misc[15], (int)(clock64() - t_s));
+    __syncthreads();
+    if (tid == 0) { atomicAdd(&g_phase[64 + blockIdx.x % 16], (unsigned long long)misc[15]); misc[15] = 0; }
+#endif
     PHASE_T0(t_b);
     cl.sync();
     PHASE_ADD(2, t_b);
+    PHASE_CTA(80, t_b);
     if (tid == 0) {
       misc[MISC_CHUNK] = NW;   // every warp has taken its last chunk
       misc[MISC_NEAR_BAD] = 0;
@@ -1070,7 +1177,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   for (int step = 0;; ++step) {
     const int par = (int)(istep & 1);
     PHASE_T0(t_l);
-    if (do_build) build(istep);
+    if (do_build) build(istep, step == 0);
     PHASE_ADD(5, t_l);
     if (do_x) {
       for (int l0 = 0; l0 < nown; l0 += NG) xmove(l0 + grp, l0 + grp < nown, par, fire);
@@ -1088,12 +1195,15 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     if (next && a.mode == KM_STEP) {
       if (!skin) fire = cadence(istep + 1);
       else {
-        int M = 0;
-        for (int r = 0; r < nr; ++r) M = max(M, dmax[par * SPLIT_MAX + r]);
+        const int M = __reduce_max_sync(0xffffffffu, lid < nr ? dmax[par * SPLIT_MAX + lid].x : 0);
         fire = 2.0f * sqrtf(__int_as_float(M)) >= (float)a.neigh_margin * 0.9999f && skin_exact(false);
       }
     }
-    sweep(istep, stepping ? a.noise_base + step : (a.mode == KM_PRE ? a.noise_base : -1), par);
+    // the near lists are recorded anew, by every CTA: after a build or a
+    // launch, or when a bead has moved too far since
+    const int far = __reduce_max_sync(0xffffffffu, lid < nr ? dmax[par * SPLIT_MAX + lid].y : 0);
+    const bool rec = misc[MISC_NEAR_BAD] != 0 || __int_as_float(far) > SP_SKIN_DISP * SP_SKIN_DISP;
+    sweep(istep, stepping ? a.noise_base + step : (a.mode == KM_PRE ? a.noise_base : -1), par, rec);
     const bool move = next && !fire;
     PHASE_T0(t_u);
     for (int l0 = 0; l0 < nown; l0 += NG) {
@@ -1105,23 +1215,25 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
           fx += (double)slots[3 * p]; fy += (double)slots[3 * p + 1]; fz += (double)slots[3 * p + 2];
         }
       group_reduce<Real>(fx, fy, fz, SG);
+      PHASE_ADD(10, t_u);
       if (valid && g < 3) {
         double f = (g == 0 ? fx : (g == 1 ? fy : fz)) + exF[3 * li + g] + dhF[3 * li + g];
-        if (a.f_ext)   // the reciprocal-space partial forces, in k-range order
-          for (int p = 0; p < EW_F_SPLIT; ++p) f += a.f_ext[3 * ((size_t)p * a.nbead_total + L.state0 + i) + g];
+        if (PER && a.f_ext) f += a.f_ext[3 * (size_t)(L.state0 + i) + g];   // the reciprocal-space force
         const int q = g * OS + li;
         if (a.mode == KM_FORCE) {
           a.out_force[3 * (size_t)(L.state0 + i) + g] = f;
         } else {
           // time_integral.F90:169-183 (KM_PRE: a(0)), each product rounded as the reference evaluates it
-          const double acc = mad2<Real>(f, RC[li], C1[li], NZ[q]);
-          if (stepping) Vv[q] = mad2<Real>(C2[li], Vv[q], C3[li], add_rn<Real>(Av[q], acc));
+          const double acc = smad<Real>(f, RC[li], C1[li], NZ[q]);
+          if (stepping) Vv[q] = smad<Real>(C2[li], Vv[q], C3[li], __dadd_rn(Av[q], acc));
           Av[q] = acc;
           if (stepping && !(f == f)) misc[MISC_NAN] = 1;
         }
       }
       __syncwarp();
+      PHASE_ADD(11, t_u);
       if (move) xmove(li, valid, par ^ 1, false);
+      PHASE_ADD(12, t_u);
     }
     if (move) send(par ^ 1);
     PHASE_ADD(4, t_u);

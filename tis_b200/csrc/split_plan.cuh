@@ -7,6 +7,13 @@ namespace tis {
 
 constexpr int SG = 8;            // threads per bead (update phase, exv lists)
 constexpr int SP_NEAR = 8;       // near-list entries per thread of a bead's group
+// near lists: partners within the screen radius + SP_SKIN, recorded by every
+// CTA of a lane together as soon as any bead has moved SP_SKIN_DISP since (two
+// beads then close in by less than SP_SKIN - 0.1 A).  A wider skin than the
+// one-CTA kernel's: a recording scans the exv rows (~8 k cycles for 1,199
+// beads on 16 CTAs), a list entry out of reach costs one screened pair
+constexpr float SP_SKIN = 2.0f;
+constexpr float SP_SKIN_DISP = 0.95f;
 constexpr int SP_IMG = 11;       // pair entries: bead in the low bits, periodic image above (periodic lanes: N < 2048)
 
 // threads of a warp that share one charged row: short rows take few
@@ -17,15 +24,15 @@ __host__ __device__ inline int split_row_lanes(int nq, bool ewald) {
 // own beads of a CTA for a lane of N beads
 __host__ __device__ inline int split_own(int N, int nr) { return ((N + nr - 1) / nr + 3) & ~3; }
 
-// T: the largest counts of the context's topologies
-inline SplitPlan split_plan(const TopDesc &T, int nq, int nr, bool periodic, bool skin, bool ewald, int real,
+// T: the largest counts of the context's topologies; bonded items: of a CTA
+// row: partners of a charged row to make room for (on average over a CTA's rows)
+inline SplitPlan split_plan(const TopDesc &T, int nq, int row, int nr, bool periodic, bool skin, bool ewald, int real,
                             unsigned limit) {
   SplitPlan p;
   const int N = T.nmp;
   p.own = split_own(N, nr);
   p.rows = (nq + nr - 1) / nr;
-  p.nst = (T.nst + nr - 1) / nr; p.nhb = (T.nhb + nr - 1) / nr;
-  p.nba = (T.nba + nr - 1) / nr; p.nbd = (T.nbd + nr - 1) / nr;
+  p.nst = T.nst; p.nhb = T.nhb; p.nba = T.nba; p.nbd = T.nbd; p.nts = T.ntst;
   p.np = (N + 3) & ~3;
   const unsigned n = p.np, o = p.own, W = (N + 31) / 32, R = real;
   unsigned b = 0;
@@ -39,6 +46,8 @@ inline SplitPlan split_plan(const TopDesc &T, int nq, int nr, bool periodic, boo
   p.C = take(32 * o);                     // rlan_const(2..4), 1 / m of the own beads
   p.scr = take(R * o);                    // exv screen radius
   p.iptr = take(4 * (o + 1));
+  p.cnt = take(4 * 5);                    // hydrogen bonds, stacks, tertiary stacks, angles, bonds of the CTA
+  p.stk = take(4 * p.nst); p.hbk = take(4 * p.nhb); p.tsk = take(4 * p.nts);   // their numbers in the topology
   p.bdi = take(4 * p.nbd); p.bdd = take(8 * p.nbd); p.bdc = take(2 * R * p.nbd);
   p.bai = take(8 * p.nba); p.bad = take(12 * p.nba); p.bac = take(2 * R * p.nba);
   p.sti = take(16 * p.nst); p.std_ = take(28 * p.nst); p.stc = take(6 * R * p.nst);
@@ -59,25 +68,17 @@ inline SplitPlan split_plan(const TopDesc &T, int nq, int nr, bool periodic, boo
   p.mexv = take(4 * W * o); p.mele = take(4 * W * p.rows);
   p.slots = take(3 * R * T.sp_ninc);
   p.exc = take(4 * T.nsite); p.hbf = take(p.nhb);
-  p.red = take(8 * (64 + 2 * SPLIT_MAX) + 8 * SPLIT_MAX);   // reductions; then the CTAs' displacement maxima, 2 parities
+  p.red = take(8 * (64 + 2 * SPLIT_MAX) + 16 * SPLIT_MAX);   // reductions; then the CTAs' displacement maxima, 2 parities
   p.img = periodic ? take(4 * R * 27) : 0;
   p.misc = take(4 * (SPLIT_MISC + T.nunit * T.nunit + 8));
-  // partner lists of the charged rows: room for the longest possible ones, or
-  // what is left of the shared memory (Debye-Hueckel rows fill theirs, the
-  // 20 A rows of an ion box need a fraction)
-  const unsigned eb = 2 * split_row_lanes(nq, ewald), most = p.rows * ((nq + eb - 1) / eb * eb);
+  // partner lists of the charged rows, or what is left of the shared memory
+  const unsigned eb = 2 * split_row_lanes(nq, ewald), most = p.rows * (((row < nq ? row : nq) + eb - 1) / eb * eb);
   p.eoff = take(4 * (p.rows + 1));
   const unsigned left = b < limit ? (limit - b) / 32 * 16 : 0;
   p.ecap = most < left ? most : left;
   p.elist = take(2 * p.ecap);
   p.total = b;
   return p;
-}
-
-// CTA r's share of n items divided by index
-__host__ __device__ inline int split_share(int n, int nr, int r) {
-  const int per = (n + nr - 1) / nr;
-  return per * r < n ? per * r : n;
 }
 
 } // namespace tis
