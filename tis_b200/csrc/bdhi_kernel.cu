@@ -7,7 +7,7 @@
 //   [every n_step_hydro steps] D = RPY tensor at x (simu_hydro_tensors.F90:
 //       139-182, HI_TENSOR%RPY), L = Cholesky factor of D (:304-324):
 //       rpy_kernel, chol_diag_kernel (L_00), then per 64-wide panel k:
-//       chol_panel_kernel (L_ik = A_ik L_kk^-T below the diagonal tile),
+//       chol_panel_kernel (L_ik = A_ik L_kk^-T below the diagonal tile) and
 //       chol_update_kernel or chol_update_tc_kernel (A_ij -= L_ik L_jk^T for
 //       the trailing tiles, FP64 or tensor cores; the CTA that finishes tile
 //       (k + 1, k + 1) factors it for the next panel)
@@ -30,7 +30,10 @@
 namespace tis {
 
 constexpr int CT = 64;          // Cholesky tile
-constexpr int CTP = CT + 1;     // padded shared-memory row
+// row of an operand tile in shared memory: 136 words, so the 4 x 4 doubles of
+// a half-warp's matrix fragment lie in different banks
+constexpr int CTP = CT + 4;
+constexpr int BD_SMS = 148;
 
 // ------------------------------------------------------------ RPY tensor
 // The 3x3 block pre1 I + pre2 r r^T of the bead pair (i < j, r = x_j - x_i)
@@ -156,242 +159,312 @@ __device__ __forceinline__ void tf32_split(double x, float &hi, float &lo) {
 // groups outermost: float offset of (r, c) = (r / 8) 512 + (c / 4) 32 +
 // (r % 8) 4 + c % 4, so consecutive row tiles form one operand of 128 rows.
 constexpr int PT = CT * CT;   // floats per plane tile
-// shared memory of the FP64 tile kernels: a padded tile and an unpadded one
-constexpr int U64_SMEM = (CT * CTP + CT * CT) * (int)sizeof(double);
+// shared memory of the FP64 tile kernels: two padded tiles
+constexpr int U64_SMEM = 2 * CT * CTP * (int)sizeof(double);
+
+// FP64 matrix instruction, c += a b for 8 x 8 x 4: lane l holds a(l / 4, l % 4),
+// b(l % 4, l / 4) and c(l / 4, 2 (l % 4) + {0, 1}).  Its rate is that of the
+// FP64 FMAs (64 per SM and cycle, measured), but one 64-bit load per operand
+// feeds 8 products: with FMAs on 4 x 4 register tiles the tile products were
+// bound by shared memory (96 cycles of loads per 64 of FMAs).
+__device__ __forceinline__ void mma8(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+// Load diagonal tile td of a lane for factor_diag_tile: the lower part of the
+// matrix, identity beyond it, zeros above the diagonal.
+__device__ __forceinline__ void load_diag_tile(const double *Lm, int n, int td, int tid, double (&acc)[8][2]) {
+  const int w = tid >> 5, r = (tid & 31) >> 2, k2 = 2 * (tid & 3), i = 8 * w + r, i0 = td * CT;
+#pragma unroll
+  for (int ct = 0; ct < 8; ++ct)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int c = 8 * ct + k2 + q;
+      acc[ct][q] = (c <= i && i0 + i < n) ? Lm[(size_t)(i0 + i) * n + i0 + c] : (i == c ? 1.0 : 0.0);
+    }
+}
 
 // Factor diagonal tile td of a lane and invert its factor with the 256
 // threads of the calling group (tid 0..255, 8 warps; sync() is the group's
-// barrier).  The tile A (identity beyond the matrix) sits in shared memory S
-// (row stride CTP).  Blocked right-looking Cholesky in the unscaled form
-// A_ic -= A_ij A_cj / p_j (p_j the pivot, L_ij = A_ij / sqrt(p_j)), 16
-// columns per block:
-//   warp 0 factors the block's columns for all rows below in registers (lane
-//     l holds rows 16 b + l and 16 b + l + 32), column values passed by warp
-//     shuffles, one pivot after the other;
-//   all warps apply the block's rank-16 update to the trailing lower part.
-// Then W = L^-1 by forward substitution L W = I, four threads per column of
-// W (rows t, t + 4, ...), the solved element passed by shuffles.
+// barrier).  Warp w holds rows 8 w .. + 7 of the tile in the accumulator
+// layout of mma8: acc[ct] = columns 8 ct .. + 7.
+//
+// This is the serial chain of a refresh: 64 pivots per panel, one after the
+// other, the rest of a small problem's chip idle meanwhile.  Right-looking
+// Cholesky in the unscaled form A_ic -= A_ij A_cj / p_j (p_j the pivot, L_ij =
+// A_ij / sqrt(p_j)), 8 columns per block:
+//   every lane of warps 0..2 factors the block's 8 x 8 diagonal block by
+//     itself in registers: a pivot costs its reciprocal, a product and an
+//     update, with no shuffle and no barrier between two pivots;
+//   thread t < 64 then solves row t of the block's columns against it;
+//   all warps apply the block's rank-8 update to the columns to the right, in
+//     their accumulators.
+// The inverse comes with it: the rows of the identity are appended below the
+// matrix and take the same steps, which leaves Lu^-T (Lu the unit lower
+// factor).  Row r of it is zero before column r, so it takes the places of the
+// tile's upper part, and at every block the 64 threads have one row each: a
+// row of the matrix below the block or a row of the identity above.
+// In one launch of its own, cold (ncu): 36.8 us when one warp factored 16
+// columns for all rows, pivots and columns passed by shuffles, and the inverse
+// followed in 64 more steps; FD_NOW us this way.
+//
+// The results are written at the end: with the idle warps writing a block's
+// while the next is factored, all phases of both took longer (17.1 against
+// FD_CYC thousand cycles a tile).
+//
 // A pivot <= 0 is replaced by 1 (no NaN spreads) and flags the lane.  Stores
 // L_tt (zero above the diagonal; FP32 copy for mixed precision) and, when a
 // panel follows, U_tt = L_tt^-T into the lane's inverse slot.  vec holds
-// 4 CT doubles.
+// FD_VEC doubles (16-byte aligned).
+constexpr int FB = 8;           // columns per block
+constexpr int FBP = FB + 4;     // row of a block's columns: fragments without bank conflicts
+constexpr int FD_X = (CT + FB) * FBP + 2 * FB + 4;   // a block: rows, the block's own lower rows, pivots, 1 / pivots
+constexpr int FD_VEC = CT / FB * FD_X + CT * FBP;
+static_assert(FD_VEC * (int)sizeof(double) <= U64_SMEM, "the factor's work space reuses the operand tiles");
+
+// 1 / p to within an ulp for a normal p: the hardware's approximation y with
+// e = 1 - p y, then Chebyshev's third-order step y (1 + e + e^2).  Without the
+// division's branch the updates of one pivot fill the wait of the next.
+__device__ __forceinline__ double pivot_rcp(double p) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(p));
+  const double e = fma(-p, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// Factor the 8 x 8 block at xin + c0 FBP and solve the thread's row v against
+// it; d = pivots, ip = their reciprocals.  Returns true if a pivot is not > 0:
+// the values are then of no use without guard, which replaces such a pivot by
+// 1 (its compare and selects are on the chain of every pivot: 742 against 574
+// cycles).
+template <bool guard>
+__device__ __forceinline__ bool diag_block(const double *xin, const double *row, int own, double (&v)[FB],
+                                           double (&d)[FB], double (&ip)[FB]) {
+  double b[FB][FB + 1];
+#pragma unroll
+  for (int i = 0; i < FB; ++i)
+#pragma unroll
+    for (int c = 0; c <= i; c += 2) {
+      const double2 x = *(const double2 *)&xin[i * FBP + c];
+      b[i][c] = x.x;
+      b[i][c + 1] = x.y;
+    }
+#pragma unroll
+  for (int q = 0; q < FB; q += 2) {
+    const double2 x = *(const double2 *)&row[q];
+    v[q] = own < 0 ? x.x : (q == own ? 1.0 : 0.0);
+    v[q + 1] = own < 0 ? x.y : (q + 1 == own ? 1.0 : 0.0);
+  }
+  bool bad = false;
+#pragma unroll
+  for (int j = 0; j < FB; ++j) {
+    double p = b[j][j], r = pivot_rcp(p);
+    const bool ok = p > 0.0;
+    bad |= !ok;
+    if (guard && !ok) p = r = 1.0;
+    d[j] = p;
+    ip[j] = r;
+    double m[FB];   // column j of the unit factor
+#pragma unroll
+    for (int i = j + 1; i < FB; ++i) m[i] = b[i][j] * r;
+#pragma unroll
+    for (int i = j + 1; i < FB; ++i)
+#pragma unroll
+      for (int c = j + 1; c <= i; ++c) b[i][c] -= m[i] * b[c][j];
+#pragma unroll
+    for (int i = j + 1; i < FB; ++i) v[i] -= v[j] * m[i];
+  }
+  return bad;
+}
+
+// Columns to the right of block s: acc -= (X / p) X^T.  acc[j] holds column
+// tile s + j on entry and s + 1 + j on return (the products move it one place
+// down), whose first goes to xin as block s + 1.  A row of the matrix stops at
+// its diagonal, a row of the identity goes to the end; beyond, the operands are
+// zero (a branch per column tile cost more than its products).  NJ >= 7 - s
+// column tiles.
+template <int NJ>
+__device__ __forceinline__ void diag_trailing(int s, double (&acc)[8][2], const double *X, double *xin, int tid) {
+  const int w = tid >> 5, r = (tid & 31) >> 2, k = tid & 3;
+  const double *xa = X + (8 * w + r) * FBP + k, *ip = X + (CT + FB) * FBP + FB;
+  const double a0 = -xa[0] * ip[k], a1 = -xa[4] * ip[4 + k];
+  const int last = w <= s ? 7 : w;
+  double b0[NJ], b1[NJ];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    const int ct = s + 1 + j;
+    const double *xb = X + (8 * min(ct, 7) + r) * FBP + k;
+    b0[j] = ct <= last ? xb[0] : 0.0;
+    b1[j] = ct <= last ? xb[4] : 0.0;
+  }
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    acc[j][0] = acc[j + 1][0];
+    acc[j][1] = acc[j + 1][1];
+    mma8(acc[j], a0, b0[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) mma8(acc[j], a1, b1[j]);
+  *(double2 *)&xin[(8 * w + r) * FBP + 2 * k] = make_double2(acc[0][0], acc[0][1]);
+}
+
 template <typename Sync>
-__device__ void factor_diag_tile(const KArgs &a, int lane, double *Lm, int n, int td, double *S, double *vec,
-                                 int tid, Sync sync) {
-  const long long L32 = a.lanes[lane].bd32;
-  const int r0 = td * CT, nb = min(CT, n - r0);
-  const int warp = tid >> 5, ln = tid & 31;
-  double *A = S, *piv = vec, *ipv = vec + CT, *rinv = vec + 2 * CT;
-  sync();   // the group's stores to the tile are visible; earlier users of S and vec are done
-  {
-    double v[CT * CT / 256];   // all loads in flight before the shared-memory stores
-#pragma unroll
-    for (int q = 0; q < CT * CT / 256; ++q) {
-      const int e = tid + 256 * q, i = e >> 6, c = e & 63;
-      v[q] = (i < nb && c < nb) ? Lm[(size_t)(r0 + i) * n + r0 + c] : (i == c ? 1.0 : 0.0);
-    }
-#pragma unroll
-    for (int q = 0; q < CT * CT / 256; ++q) {
-      const int e = tid + 256 * q;
-      A[(e >> 6) * CTP + (e & 63)] = v[q];
-    }
-  }
-  int bad = 0;   // warp 0
-  for (int b = 0; b < CT / 16; ++b) {
-    const int c0 = 16 * b;
-    sync();
-    if (warp == 0) {
-      const int ra = c0 + ln, rb = c0 + ln + 32;
-      double pa[16], pb[16];
-#pragma unroll
-      for (int cc = 0; cc < 16; ++cc) {
-        pa[cc] = (ra < CT) ? A[ra * CTP + c0 + cc] : 0.0;
-        pb[cc] = (rb < CT) ? A[rb * CTP + c0 + cc] : 0.0;
+__device__ void factor_diag_tile(const KArgs &a, int lane, double *Lm, int n, int td, double (&acc)[8][2],
+                                 double *vec, int tid, Sync sync) {
+  const int r0 = td * CT, nb = min(CT, n - r0), np = (n + 3) & ~3;
+  float *L32 = a.bd_tc ? a.bd_L32 + a.lanes[lane].bd32 : nullptr;
+  double *wout = r0 + CT < n ? a.bd_W + (size_t)lane * CT * CT : nullptr;   // a panel of rows below follows (then nb = CT)
+  double *xin = vec + CT / FB * FD_X;
+  bool bad = false;
+  sync();   // vec is free
+  *(double2 *)&xin[(tid >> 2) * FBP + 2 * (tid & 3)] = make_double2(acc[0][0], acc[0][1]);
+#pragma unroll 1
+  for (int s = 0; s < CT / FB; ++s) {
+    sync();   // xin: the block's columns with all earlier blocks applied
+    double *X = vec + s * FD_X;
+    if (tid < 96) {
+      // threads 0 .. 63: row tid below the block, or the identity's row tid
+      // (own: one that starts in this block); 64 .. 71: the block's own rows
+      const int o = tid - FB * s, own = tid < CT && (unsigned)o < (unsigned)FB ? o : -1;
+      const double *row = xin + (tid < CT ? tid : FB * s + (tid & 7)) * FBP;
+      double v[FB], d[FB], ip[FB];
+      if (diag_block<false>(xin + FB * s * FBP, row, own, v, d, ip)) {   // the same in every thread
+        bad = true;
+        diag_block<true>(xin + FB * s * FBP, row, own, v, d, ip);
       }
+      if (tid < CT + FB) {
 #pragma unroll
-      for (int jj = 0; jj < 16; ++jj) {
-        double p = __shfl_sync(0xffffffffu, pa[jj], jj);   // A_jj: row c0 + jj is lane jj's first row
-        if (!(p > 0.0)) {
-          p = 1.0;
-          bad = 1;
+        for (int q = 0; q < FB; q += 2) *(double2 *)&X[tid * FBP + q] = make_double2(v[q], v[q + 1]);
+      } else if (tid == CT + FB) {
+#pragma unroll
+        for (int q = 0; q < FB; q += 2) {
+          *(double2 *)&X[(CT + FB) * FBP + q] = make_double2(d[q], d[q + 1]);
+          *(double2 *)&X[(CT + FB) * FBP + FB + q] = make_double2(ip[q], ip[q + 1]);
         }
-        const double ip = 1.0 / p;
-        if (ln == 0) {
-          piv[c0 + jj] = p;
-          ipv[c0 + jj] = ip;
-        }
-        double cv[16];   // A_{c0 + cc, j}, cc > jj
-#pragma unroll
-        for (int cc = jj + 1; cc < 16; ++cc) cv[cc] = __shfl_sync(0xffffffffu, pa[jj], cc);
-        if (ln > jj && ra < CT) {
-          const double m = pa[jj] * ip;
-#pragma unroll
-          for (int cc = jj + 1; cc < 16; ++cc)
-            if (cc <= ln) pa[cc] -= m * cv[cc];
-        }
-        if (rb < CT) {
-          const double m = pb[jj] * ip;
-#pragma unroll
-          for (int cc = jj + 1; cc < 16; ++cc) pb[cc] -= m * cv[cc];
-        }
-      }
-#pragma unroll
-      for (int cc = 0; cc < 16; ++cc) {
-        if (ra < CT) A[ra * CTP + c0 + cc] = pa[cc];
-        if (rb < CT) A[rb * CTP + c0 + cc] = pb[cc];
       }
     }
     sync();
-    // rank-16 update of the trailing lower part: rows and columns >= c0 + 16;
-    // thread (ty, tx) owns rows t0 + ty + 16 u and columns t0 + tx + 16 v
-    // (u, v < 3), all of them accumulated side by side
-    const int t0 = c0 + 16;
-    if (t0 < CT) {
-      const int tx = tid & 15, ty = tid >> 4;
-      double acc[3][3];
-#pragma unroll
-      for (int u = 0; u < 3; ++u)
-#pragma unroll
-        for (int v = 0; v < 3; ++v) acc[u][v] = 0.0;
-#pragma unroll
-      for (int jj = 0; jj < 16; ++jj) {
-        double ai[3], ac[3];
-#pragma unroll
-        for (int u = 0; u < 3; ++u) {
-          const int i = min(t0 + ty + 16 * u, CT - 1), c = min(t0 + tx + 16 * u, CT - 1);
-          ai[u] = A[i * CTP + c0 + jj];
-          ac[u] = A[c * CTP + c0 + jj] * ipv[c0 + jj];
-        }
-#pragma unroll
-        for (int u = 0; u < 3; ++u)
-#pragma unroll
-          for (int v = 0; v < 3; ++v) acc[u][v] += ai[u] * ac[v];
-      }
-#pragma unroll
-      for (int u = 0; u < 3; ++u)
-#pragma unroll
-        for (int v = 0; v < 3; ++v) {
-          const int i = t0 + ty + 16 * u, c = t0 + tx + 16 * v;
-          if (i < CT && c <= i) A[i * CTP + c] -= acc[u][v];
-        }
-    }
+    if (s < 3) diag_trailing<7>(s, acc, X, xin, tid);
+    else if (s + 1 < CT / FB) diag_trailing<4>(s, acc, X, xin, tid);
   }
-  sync();
-  if (tid < CT) {
-    const double d = sqrt(piv[tid]);
-    piv[tid] = d;
-    rinv[tid] = 1.0 / d;
-  }
-  sync();
+  // L[i][c] and U[i][c] = (L^-1)[c][i]; thread: column c, rows i0 + 4 u.  A
+  // block's column is unscaled: L_ic = x / sqrt(p_c)
+  const int c = tid & 63, q = c & 7;
+  const double *X = vec + (c >> 3) * FD_X;
+  const double d = sqrt(X[(CT + FB) * FBP + q]), ri = pivot_rcp(d);
+  const int i0 = tid >> 6, c8 = c & ~7;
+  double u[CT / 4];
 #pragma unroll
-  for (int q = 0; q < CT * CT / 256; ++q) {
-    const int e = tid + 256 * q, i = e >> 6, c = e & 63;
-    const double l = (c < i) ? A[i * CTP + c] * rinv[c] : (c == i ? piv[c] : 0.0);
-    A[i * CTP + c] = l;
+  for (int t = 0; t < CT / 4; ++t) u[t] = X[(i0 + 4 * t) * FBP + q] * ri;   // L below the block, else U
+#pragma unroll
+  for (int t = 0; t < FB / 4; ++t) {   // the block's own rows of L
+    const int o = i0 + 4 * t, i = c8 + o;
+    const double l = q < o ? X[(CT + o) * FBP + q] * ri : (q == o ? d : 0.0);
     if (i < nb && c < nb) {
       Lm[(size_t)(r0 + i) * n + r0 + c] = l;
-      if (a.bd_tc) a.bd_L32[L32 + (size_t)(r0 + i) * ((n + 3) & ~3) + r0 + c] = (float)l;
+      if (L32) L32[(size_t)(r0 + i) * np + r0 + c] = (float)l;
     }
+  }
+#pragma unroll
+  for (int t = 0; t < CT / 4; ++t) {
+    const int i = i0 + 4 * t;
+    const double l = i > c ? u[t] : 0.0;
+    if ((i ^ c) >= FB && i < nb && c < nb) {
+      Lm[(size_t)(r0 + i) * n + r0 + c] = l;
+      if (L32) L32[(size_t)(r0 + i) * np + r0 + c] = (float)l;
+    }
+    if (wout) wout[i * CT + c] = c > i ? u[t] : (c == i ? ri : 0.0);
   }
   if (tid == 0 && bad) atomicOr(&a.not_spd[lane], 1);
-  if (r0 + CT < n) {   // a panel of rows below follows (then nb = CT)
-    sync();
-    // column c of W: thread t of the group of four owns rows t + 4 s
-    const int c = tid >> 2, t = tid & 3, lead = ln & ~3;
-    double w[16];
-#pragma unroll
-    for (int s2 = 0; s2 < 16; ++s2) w[s2] = (t + 4 * s2 == c) ? 1.0 : 0.0;
-#pragma unroll
-    for (int j = 0; j < CT; ++j) {
-      double lj[16];   // column j of L for the rows of this thread, loaded off the chain
-#pragma unroll
-      for (int s2 = (j >> 2); s2 < 16; ++s2) lj[s2] = A[(t + 4 * s2) * CTP + j];
-      double wj = 0.0;
-      if (t == (j & 3)) {
-        w[j >> 2] *= rinv[j];
-        wj = w[j >> 2];
-      }
-      wj = __shfl_sync(0xffffffffu, wj, lead | (j & 3));   // zero while j < c
-#pragma unroll
-      for (int s2 = (j >> 2); s2 < 16; ++s2)
-        if (t + 4 * s2 > j) w[s2] -= lj[s2] * wj;
-    }
-    double *wout = a.bd_W + (size_t)lane * CT * CT + (size_t)c * CT;   // U[c][i] = W[i][c]
-#pragma unroll
-    for (int s2 = 0; s2 < 16; ++s2) wout[t + 4 * s2] = w[s2];
-  }
 }
 
 struct BlockSync {
   __device__ void operator()() const { __syncthreads(); }
 };
 
-// grid nlane, 256 threads: the diagonal tile of panel k of every lane.  On
-// the tensor-core path the diagonal tile of a later panel is factored by the
-// update launch that finishes it (the CTA that owns it), so only panel 0
-// needs this launch; the FP64 path launches it for every panel.
+// grid nlane, 256 threads: the first diagonal tile of every lane.  A later one
+// is factored by the update launch that finishes it (the CTA that owns it).
 __global__ void __launch_bounds__(256) chol_diag_kernel(KArgs a) {
   const int lane = blockIdx.x;
   if (lane >= a.nlane) return;
   const LaneDesc L = a.lanes[lane];
-  int n;
-  lane_tiles(a, L, n);
-  __shared__ double S[CT * CTP], vec[5 * CT];
-  if (a.bd_kpanel < lane_tiles(a, L, n)) factor_diag_tile(a, lane, a.bd_L + L.bd0, n, a.bd_kpanel, S, vec, threadIdx.x, BlockSync{});
+  const int n = 3 * a.tops[L.top].nmp;
+  extern __shared__ __align__(16) double vec[];   // FD_VEC
+  double acc[8][2];
+  load_diag_tile(a.bd_L + L.bd0, n, 0, threadIdx.x, acc);
+  factor_diag_tile(a, lane, a.bd_L + L.bd0, n, 0, acc, vec, threadIdx.x, BlockSync{});
 }
 
-// grid (T - k - 1, nlane), 256 threads: row tile ti = k + 1 + blockIdx.x of
-// the panel below the factored diagonal tile: X = A_ik L_kk^-T as a 64 x 64
-// x 64 FP64 product with the stored transposed inverse U_kk (thread (ty, tx)
-// owns rows ty + 16 u, columns tx + 16 v; sums over m in increasing order),
-// stored in FP64 and, for the tensor-core update, split into TF32 hi / lo
-// in the panel planes.  Loads and stores are row-contiguous.
+// grid ((T - k - 1) 64 / RB, nlane), 256 threads: RB rows of row tile ti of
+// the panel below the factored diagonal tile: X = A_ik L_kk^-T as an RB x 64
+// x 64 FP64 product with the stored transposed inverse U_kk, upper triangular:
+// column tile ct (8 columns) sums over m < 8 ct + 8, in increasing order.
+// Stored in FP64 and, for the tensor-core update, split into TF32 hi / lo in
+// the panel planes.  Loads and stores are row-contiguous.
+// RB = 64: warp w has rows 8 w .. + 7; RB = 16: 8 rows and the column tiles q
+// and 7 - q, the same work for every warp.
+template <int RB>
 __global__ void __launch_bounds__(256) chol_panel_kernel(KArgs a) {
+  constexpr int SUB = CT / RB;
   const int lane = blockIdx.y;
   if (lane >= a.nlane) return;
   const LaneDesc L = a.lanes[lane];
   int n;
   const int T = lane_tiles(a, L, n), k = a.bd_kpanel;
-  const int ti = k + 1 + blockIdx.x;
+  const int ti = k + 1 + blockIdx.x / SUB, rb = (blockIdx.x % SUB) * RB;   // first row in the tile
   if (ti >= T) return;   // rows below the diagonal tile: the panel is full (64 columns)
-  const int r0 = k * CT, i0 = ti * CT, mi = min(CT, n - i0);
+  const int r0 = k * CT, i0 = ti * CT + rb, mi = min(RB, n - i0);
   double *Lm = a.bd_L + L.bd0;
-  extern __shared__ double dsm[];   // U64_SMEM
-  double *As = dsm, *Us = As + CT * CTP;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  extern __shared__ __align__(16) double dsm[];
+  double *As = dsm, *Us = As + RB * CTP;
+  const int tid = threadIdx.x, wp = tid >> 5, fr = (tid & 31) >> 2, fk = tid & 3;
   const double *w = a.bd_W + (size_t)lane * CT * CT;
-#pragma unroll 4
-  for (int e = tid; e < CT * CT; e += 256) {
-    const int r = e >> 6, c = e & 63;
+#pragma unroll
+  for (int q = 0; q < RB * CT / 256; ++q) {
+    const int e = tid + 256 * q, r = e >> 6, c = e & 63;
     As[r * CTP + c] = (r < mi) ? Lm[(size_t)(i0 + r) * n + r0 + c] : 0.0;
-    Us[e] = w[e];
+  }
+#pragma unroll
+  for (int q = 0; q < CT * CT / 256; ++q) {
+    const int e = tid + 256 * q;
+    Us[(e >> 6) * CTP + (e & 63)] = w[e];
   }
   __syncthreads();
-  double acc[4][4];
+  constexpr int NT = RB == CT ? 8 : 2;   // column tiles of a warp
+  double acc[NT][2];
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = 0.0;
+  const int row = RB == CT ? 8 * wp + fr : 8 * (wp & 1) + fr;
+  const int ct0 = RB == CT ? 0 : wp >> 1, ct1 = 7 - ct0;
+  if (RB == CT) {
 #pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
+    for (int mb = 0; mb < 8; ++mb)
+#pragma unroll
+      for (int h = 0; h < 8; h += 4) {
+        const int m = 8 * mb + h + fk;
+        const double av = As[row * CTP + m];
+#pragma unroll
+        for (int t = mb; t < NT; ++t) mma8(acc[t], av, Us[m * CTP + 8 * t + fr]);
+      }
+  } else {
 #pragma unroll 4
-  for (int m = 0; m < CT; ++m) {
-    double av[4], bv[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) av[u] = As[(ty + 16 * u) * CTP + m];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) bv[v] = Us[m * CT + tx + 16 * v];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) acc[u][v] += av[u] * bv[v];
+    for (int m = fk; m < 8 * ct1 + 8; m += 4) {
+      const double av = As[row * CTP + m];
+      if (m < 8 * ct0 + 8) mma8(acc[0], av, Us[m * CTP + 8 * ct0 + fr]);   // uniform: 4 divides the bound
+      mma8(acc[1], av, Us[m * CTP + 8 * ct1 + fr]);
+    }
   }
   __syncthreads();
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) As[(ty + 16 * u) * CTP + tx + 16 * v] = acc[u][v];
+  for (int t = 0; t < NT; ++t) {
+    const int ct = RB == CT ? t : (t ? ct1 : ct0);
+    *(double2 *)&As[row * CTP + 8 * ct + 2 * fk] = make_double2(acc[t][0], acc[t][1]);
+  }
   __syncthreads();
 #pragma unroll 4
-  for (int e = tid; e < CT * CT; e += 256) {
+  for (int e = tid; e < RB * CT; e += 256) {
     const int r = e >> 6, c = e & 63;
     if (r < mi) {
       Lm[(size_t)(i0 + r) * n + r0 + c] = As[r * CTP + c];
@@ -402,24 +475,29 @@ __global__ void __launch_bounds__(256) chol_panel_kernel(KArgs a) {
     float *ph = a.bd_P + L.bdp0 + (size_t)(k & 1) * 2 * (T + 1) * PT + (size_t)ti * PT;
     float *pl = ph + (size_t)(T + 1) * PT;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + 256 * q, r = e & 63, g = e >> 6;
-      const double *x = As + r * CTP + 4 * g;
+    for (int q = 0; q < RB / 16; ++q) {
+      const int e = tid + 256 * q, r = e % RB, g = e / RB, rt = rb + r;
+      const double2 x01 = *(const double2 *)(As + r * CTP + 4 * g), x23 = *(const double2 *)(As + r * CTP + 4 * g + 2);
       float4 h, l;
-      tf32_split(x[0], h.x, l.x);
-      tf32_split(x[1], h.y, l.y);
-      tf32_split(x[2], h.z, l.z);
-      tf32_split(x[3], h.w, l.w);
-      const int o = (r >> 3) * 512 + g * 32 + (r & 7) * 4;
+      tf32_split(x01.x, h.x, l.x);
+      tf32_split(x01.y, h.y, l.y);
+      tf32_split(x23.x, h.z, l.z);
+      tf32_split(x23.y, h.w, l.w);
+      const int o = (rt >> 3) * 512 + g * 32 + (rt & 7) * 4;
       *(float4 *)(ph + o) = h;
       *(float4 *)(pl + o) = l;
     }
   }
 }
 
-// grid (nlane, pairs), 256 threads: trailing tile (ti, tj), k < tj <= ti:
-// A_ij -= L_ik L_jk^T, a 64x64x64 FP64 product (4x4 outputs per thread)
+// grid (nlane, tile pairs, parts), 256 threads: trailing tile (ti, tj),
+// k < tj <= ti: A_ij -= L_ik L_jk^T in FP64.  B = 64: a CTA has the whole 64 x
+// 64 tile (1 part), a warp 8 rows of it; B = 32: a quarter (4 parts), a warp 8
+// rows of 16 columns.  The tile (k + 1, k + 1) belongs to one CTA either way,
+// which factors it for the next panel.
+template <int B>
 __global__ void __launch_bounds__(256) chol_update_kernel(KArgs a) {
+  constexpr int SUB = CT / B;
   const int lane = blockIdx.x;
   if (lane >= a.nlane) return;
   const LaneDesc L = a.lanes[lane];
@@ -432,46 +510,64 @@ __global__ void __launch_bounds__(256) chol_update_kernel(KArgs a) {
   while (ii * (ii + 1) / 2 > p) --ii;
   while ((ii + 1) * (ii + 2) / 2 <= p) ++ii;
   const int jj = p - ii * (ii + 1) / 2;
-  const int ti = k + 1 + ii, tj = k + 1 + jj;
-  const int r0 = k * CT, nb = min(CT, n - r0);
-  const int i0 = ti * CT, mi = min(CT, n - i0);
-  const int j0 = tj * CT, mj = min(CT, n - j0);
+  const int ti = k + 1 + ii, tj = k + 1 + jj, r0 = k * CT;
+  const int qi = blockIdx.z / SUB, qj = blockIdx.z % SUB;
   double *Lm = a.bd_L + L.bd0;
-  extern __shared__ double sh[];
-  double *As = sh, *Bs = sh + CT * CT;   // transposed: As[m][r], Bs[m][c]
-  const int tid = threadIdx.x;
-  for (int e = tid; e < CT * CT; e += blockDim.x) {
-    const int r = e / CT, mm = e - r * CT;
-    As[mm * CT + r] = (r < mi && mm < nb) ? Lm[(size_t)(i0 + r) * n + r0 + mm] : 0.0;
-    Bs[mm * CT + r] = (r < mj && mm < nb) ? Lm[(size_t)(j0 + r) * n + r0 + mm] : 0.0;
-  }
-  __syncthreads();
-  const int tx = tid & 15, ty = tid >> 4;
-  double acc[4][4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
-  for (int mm = 0; mm < nb; ++mm) {
-    const double2 a01 = *(const double2 *)&As[mm * CT + 4 * ty], a23 = *(const double2 *)&As[mm * CT + 4 * ty + 2];
-    const double2 b01 = *(const double2 *)&Bs[mm * CT + 4 * tx], b23 = *(const double2 *)&Bs[mm * CT + 4 * tx + 2];
-    const double av[4] = {a01.x, a01.y, a23.x, a23.y}, bv[4] = {b01.x, b01.y, b23.x, b23.y};
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) acc[u][v] += av[u] * bv[v];
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int r = 4 * ty + u;
-    if (r >= mi) continue;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int c = 4 * tx + v;
-      if (c >= mj) continue;
-      Lm[(size_t)(i0 + r) * n + j0 + c] -= acc[u][v];
+  extern __shared__ __align__(16) double sh[];
+  double *As = sh, *Bs = sh + CT * CTP;
+  const int tid = threadIdx.x, w = tid >> 5, fr = (tid & 31) >> 2, fk = tid & 3;
+  auto load = [&](double *dst, int i0, int rows) {   // rows i0 .. of the panel
+#pragma unroll 8
+    for (int e = tid; e < rows * CT; e += 256) {
+      const int r = e >> 6, c = e & 63;
+      dst[r * CTP + c] = (i0 + r < n) ? Lm[(size_t)(i0 + r) * n + r0 + c] : 0.0;
     }
+  };
+  if (p == 0) {
+    if (blockIdx.z) return;
+    load(As, ti * CT, CT);
+    double acc[8][2];
+    load_diag_tile(Lm, n, ti, tid, acc);
+    __syncthreads();
+    // rows beyond the matrix have zero panel rows: the identity stays
+#pragma unroll 2
+    for (int mm = fk; mm < CT; mm += 4) {
+      const double av = -As[(8 * w + fr) * CTP + mm];
+#pragma unroll
+      for (int ct = 0; ct < 8; ++ct)
+        if (ct <= w) mma8(acc[ct], av, As[(8 * ct + fr) * CTP + mm]);
+    }
+    factor_diag_tile(a, lane, Lm, n, ti, acc, sh, tid, BlockSync{});   // FD_VEC doubles fit the two tiles
+    return;
   }
+  if (ti == tj && qj > qi) return;
+  const int i0 = ti * CT + qi * B, j0 = tj * CT + qj * B;
+  load(As, i0, B);
+  load(Bs, j0, B);
+  constexpr int NT = B == CT ? 8 : 2;
+  const int row = B == CT ? 8 * w + fr : 8 * (w >> 1) + fr, ct0 = B == CT ? 0 : 2 * (w & 1);
+  double acc[NT][2];
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int i = i0 + row, c = j0 + 8 * (ct0 + t) + 2 * fk + q;
+      acc[t][q] = (i < n && c < n) ? Lm[(size_t)i * n + c] : 0.0;
+    }
+  __syncthreads();
+#pragma unroll 4
+  for (int mm = fk; mm < CT; mm += 4) {
+    const double av = -As[row * CTP + mm];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) mma8(acc[t], av, Bs[(8 * (ct0 + t) + fr) * CTP + mm]);
+  }
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int i = i0 + row, c = j0 + 8 * (ct0 + t) + 2 * fk + q;
+      if (i < n && c < n) Lm[(size_t)i * n + c] = acc[t][q];
+    }
 }
 
 // ------------------------------------------------------------ tensor cores
@@ -719,8 +815,9 @@ __global__ void __launch_bounds__(U_THREADS, 1) chol_update_tc_kernel(KArgs a, c
                    : "r"(eok)
                    : "memory");
       if (all_ok) {
-        double *fs = (double *)base, *fv = fs + CT * CTP;
-        factor_diag_tile(a, lane, Lm, n, cf, fs, fv, tid - 64, esync);
+        double acc[8][2];
+        load_diag_tile(Lm, n, cf, tid - 64, acc);
+        factor_diag_tile(a, lane, Lm, n, cf, acc, (double *)base, tid - 64, esync);
       }
     }
   }
@@ -1067,31 +1164,46 @@ void bd_update_items(const std::vector<int> &lane_T, std::vector<int> &items, st
   }
 }
 
+// Panel launch: 64 rows per CTA, or 16 while the 64-row CTAs would leave SMs
+// idle (a panel is FP64-bound, so splitting the rows divides its time, but
+// every CTA reads U again).
+cudaError_t panel_launch(cudaStream_t st, const KArgs &a, int m) {
+  if ((long long)m * a.nlane <= BD_SMS)
+    chol_panel_kernel<16><<<dim3(4 * m, a.nlane), 256, (16 + CT) * CTP * sizeof(double), st>>>(a);
+  else
+    chol_panel_kernel<CT><<<dim3(m, a.nlane), 256, U64_SMEM, st>>>(a);
+  return cudaGetLastError();
+}
+
 cudaError_t bd_refactor_launch(cudaStream_t st, KArgs a, int max_nmp, const int *items, const int *koff) {
-  cudaError_t e = cudaFuncSetAttribute(chol_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       U64_SMEM);
+  cudaError_t e = cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FD_VEC * sizeof(double));
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(chol_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, U64_SMEM);
+  e = cudaFuncSetAttribute(chol_update_kernel<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, U64_SMEM);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(chol_update_kernel<CT / 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, U64_SMEM);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(chol_panel_kernel<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, U64_SMEM);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(chol_update_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, U_SMEM + 1024);
   if (e != cudaSuccess) return e;
   if (a.bd_tc && (!a.bd_P || !items || !koff)) return cudaErrorInvalidValue;
   const long long nn = (long long)max_nmp * max_nmp;
   rpy_kernel<<<dim3((unsigned)((nn + 255) / 256), a.nlane), 256, 0, st>>>(a);
-  a.bd_kpanel = 0;
-  chol_diag_kernel<<<a.nlane, 256, 0, st>>>(a);
+  chol_diag_kernel<<<a.nlane, 256, FD_VEC * sizeof(double), st>>>(a);
   const int T = (3 * max_nmp + CT - 1) / CT;
   if (a.bd_tc) {
     // panel pairs: panel k, narrow update (column k + 1), panel k + 1, wide update
     for (int k = 0; k + 1 < T; k += 2) {
       a.bd_kpanel = k;
-      chol_panel_kernel<<<dim3(T - k - 1, a.nlane), 256, U64_SMEM, st>>>(a);
+      e = panel_launch(st, a, T - k - 1);
+      if (e != cudaSuccess) return e;
       int nit = koff[k + 1] - koff[k];
       if (nit > 0) chol_update_tc_kernel<<<nit, U_THREADS, U_SMEM + 1024, st>>>(a, items + koff[k], 1);
       if (k + 2 < T) {
         KArgs b = a;
         b.bd_kpanel = k + 1;
-        chol_panel_kernel<<<dim3(T - k - 2, a.nlane), 256, U64_SMEM, st>>>(b);
+        e = panel_launch(st, b, T - k - 2);
+        if (e != cudaSuccess) return e;
         nit = koff[k + 2] - koff[k + 1];
         if (nit > 0) chol_update_tc_kernel<<<nit, U_THREADS, U_SMEM + 1024, st>>>(a, items + koff[k + 1], 2);
       }
@@ -1099,14 +1211,13 @@ cudaError_t bd_refactor_launch(cudaStream_t st, KArgs a, int max_nmp, const int 
   } else {
     for (int k = 0; k + 1 < T; ++k) {
       a.bd_kpanel = k;
-      const int m = T - k - 1;
-      if (k > 0) chol_diag_kernel<<<a.nlane, 256, 0, st>>>(a);
-      chol_panel_kernel<<<dim3(m, a.nlane), 256, U64_SMEM, st>>>(a);
-      chol_update_kernel<<<dim3(a.nlane, m * (m + 1) / 2), 256, U64_SMEM, st>>>(a);
+      const int m = T - k - 1, np = m * (m + 1) / 2;
+      e = panel_launch(st, a, m);
+      if (e != cudaSuccess) return e;
+      // quarter tiles while the whole ones would leave SMs idle
+      if ((long long)np * a.nlane <= BD_SMS) chol_update_kernel<CT / 2><<<dim3(a.nlane, np, 4), 256, U64_SMEM, st>>>(a);
+      else chol_update_kernel<CT><<<dim3(a.nlane, np), 256, U64_SMEM, st>>>(a);
     }
-    // the last diagonal tile
-    a.bd_kpanel = T - 1;
-    if (T > 1) chol_diag_kernel<<<a.nlane, 256, 0, st>>>(a);
   }
   if (a.bd_refine) {
     e = cudaFuncSetAttribute(refine_residual_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM);
@@ -1122,7 +1233,7 @@ cudaError_t bd_refactor_launch(cudaStream_t st, KArgs a, int max_nmp, const int 
 
 int bd_refactor_launches(int max_nmp, bool tc) {
   const int T = (3 * max_nmp + CT - 1) / CT;
-  if (!tc) return 2 + 3 * (T - 1);
+  if (!tc) return 2 + 2 * (T - 1);
   int nl = 2;
   for (int k = 0; k + 1 < T; k += 2) nl += (k + 2 < T) ? 4 : 2;
   return nl;
