@@ -54,9 +54,11 @@ cudaError_t rex_exchange_launch(cudaStream_t st, const KArgs &a, RexState *rex, 
                                 double *velo);
 cudaError_t ewald_recip_launch(cudaStream_t st, const KArgs &a, int nq_max, bool forces);
 cudaError_t ewald_energy_launch(cudaStream_t st, const KArgs &a);
-cudaError_t bd_refactor_launch(cudaStream_t st, KArgs a, int max_nmp, const int *items, const int *koff);
+cudaError_t bd_refactor_launch(cudaStream_t st, KArgs a, int max_nmp, const int *items, const int *koff,
+                               const int *kug);
 int bd_refactor_launches(int max_nmp, bool tc);
-void bd_update_items(const std::vector<int> &lane_T, std::vector<int> &items, std::vector<int> &koff);
+void bd_update_items(const std::vector<int> &lane_T, std::vector<int> &items, std::vector<int> &koff,
+                     std::vector<int> &kug);
 long long bd_plane_floats(int nmp);
 cudaError_t bd_step_launch(cudaStream_t st, const KArgs &a, int max_nmp);
 cudaError_t bd_force_launch(cudaStream_t st, const KArgs &a, int max_nmp);
@@ -200,7 +202,7 @@ struct tis_ctx {
   DBuf<double> fene_nat, fene_coef, fene_d2, wca_nat, wca_coef, bd_D, bd_L, bd_F, bd_xi;
   DBuf<float> bd_P, bd_D32, bd_L32;
   DBuf<int> bd_items;               // tensor-core update work items, per launch
-  std::vector<int> bd_koff;
+  std::vector<int> bd_koff, bd_kug;   // per launch: first item, column tiles per item
   DBuf<double> bd_W;
   bool refine = false;               // Brownian-HI: refined noise (tis_params.hi_refine)
   DBuf<double> bd_D64, bd_z;
@@ -1257,7 +1259,7 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
         tis_destroy(c);
         return TIS_E_UNSUPPORTED;   // work items pack the row block in 8 bits, the lane in 15
       }
-      bd_update_items(lane_T, items, c->bd_koff);
+      bd_update_items(lane_T, items, c->bd_koff, c->bd_kug);
       if (items.empty()) items.push_back(0);
       CK(c->bd_items.upload(items));
       CK(c->bd_D32.alloc((size_t)bd32_off)); CK(c->bd_L32.alloc((size_t)bd32_off));
@@ -1877,7 +1879,8 @@ int enqueue_steps(tis_ctx *c, int nsteps, const int *lane_n_dev) {
       b.noise_base = c->noise_base + (int)k;
       if ((istep - 1) % every == 0) {
         c->launches += bd_refactor_launches(c->max_nmp, b.bd_tc != 0) + (c->refine ? 2 : 0);
-        CK(bd_refactor_launch(c->stream, b, c->max_nmp, c->bd_items.p, c->bd_koff.data()));
+        CK(bd_refactor_launch(c->stream, b, c->max_nmp, c->bd_items.p, c->bd_koff.data(),
+                              c->bd_kug.data()));
       }
       c->launches += 3 + (c->refine ? 1 : 0);
       CK(bd_step_launch(c->stream, b, c->max_nmp));

@@ -654,7 +654,7 @@ __device__ __forceinline__ const float *plane_hi(const KArgs &a, const LaneDesc 
 // One CTA per work item (lane << 16 | R << 8 | g) of the launch (bd_update_items):
 // narrow (nph = 1): column tile k + 1 only, panel k; wide (nph = 2): column
 // tiles >= k + 2, panels k and k + 1.  U_THREADS threads, one CTA per SM.
-__global__ void __launch_bounds__(U_THREADS, 1) chol_update_tc_kernel(KArgs a, const int *items, int nph) {
+__global__ void __launch_bounds__(U_THREADS, 1) chol_update_tc_kernel(KArgs a, const int *items, int nph, int ug) {
   const int item = items[blockIdx.x];
   const int lane = item >> 16, R = (item >> 8) & 255, g = item & 255;
   const LaneDesc L = a.lanes[lane];
@@ -663,9 +663,9 @@ __global__ void __launch_bounds__(U_THREADS, 1) chol_update_tc_kernel(KArgs a, c
   const int cf = k + nph;   // first updated row and column tile
   const int m = T - cf;
   if (m <= 0 || 2 * R >= m) return;   // not produced by the item tables; uniform over the CTA
-  const int ncol = nph == 1 ? 1 : min(2 * R + 2, m), c0 = g * UG;
+  const int ncol = nph == 1 ? 1 : min(2 * R + 2, m), c0 = g * ug;   // ug <= UG
   if (c0 >= ncol) return;
-  const int nt = min(UG, ncol - c0);
+  const int nt = min(ug, ncol - c0);
   const int ti0 = cf + 2 * R, tj0 = cf + c0;
   double *Lm = a.bd_L + L.bd0;
 
@@ -767,6 +767,25 @@ __global__ void __launch_bounds__(U_THREADS, 1) chol_update_tc_kernel(KArgs a, c
     float *stg = (float *)(base + U_A + 2 * U_B + e * U_STG);
     uint32_t eok = 1;
     for (int t = 0; t < nt; ++t) {
+      const int tj = tj0 + t, col = tj * CT + h * 32 + lid;
+      // the tile's FP64 elements while its products are on their way, and the
+      // next tile's lines towards L2: a tile's time was that of its loads,
+      // issued after the wait (4.2 us a tile; now EP_NOW)
+      double old[32];
+#pragma unroll
+      for (int rr = 0; rr < 32; ++rr) {
+        const int rw = q * 32 + rr, trow = ti0 + (rw >> 6), grow = trow * CT + (rw & 63);
+        old[rr] = (grow < n && col < n && trow >= tj) ? Lm[(size_t)grow * n + col] : 0.0;
+      }
+      if (t + 1 < nt) {
+        const int rw = q * 32 + lid, trow = ti0 + (rw >> 6), grow = trow * CT + (rw & 63), c0 = (tj + 1) * CT + h * 32;
+        if (grow < n && c0 + 31 < n && trow > tj) {
+          const double *next = Lm + (size_t)grow * n + c0;
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(next));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(next + 16));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(next + 31));
+        }
+      }
       const bool ok = __all_sync(0xffffffffu, mbar_wait(b_tfull + 8 * t, 0));
       if (!ok) {
         if (lid == 0) gaveup = 1;
@@ -789,13 +808,6 @@ __global__ void __launch_bounds__(U_THREADS, 1) chol_update_tc_kernel(KArgs a, c
 #pragma unroll
       for (int c = 0; c < 32; ++c) stg[lid * 33 + c] = __uint_as_float(v[c]);
       __syncwarp();
-      const int tj = tj0 + t, col = tj * CT + h * 32 + lid;
-      double old[32];
-#pragma unroll
-      for (int rr = 0; rr < 32; ++rr) {
-        const int rw = q * 32 + rr, trow = ti0 + (rw >> 6), grow = trow * CT + (rw & 63);
-        old[rr] = (grow < n && col < n && trow >= tj) ? Lm[(size_t)grow * n + col] : 0.0;
-      }
 #pragma unroll
       for (int rr = 0; rr < 32; ++rr) {
         const int rw = q * 32 + rr, trow = ti0 + (rw >> 6), grow = trow * CT + (rw & 63);
@@ -845,92 +857,160 @@ __global__ void __launch_bounds__(128) bd_noise_kernel(KArgs a) {
   xi[0] = n0; xi[1] = n1; xi[2] = n2;
 }
 
-// grid (ceil(maxN * 3 / 8), nlane), 256 threads: one warp per row k of the
-// lane: dx_k = rlan1 sum_c D_kc F_c + rlan2 sum_{c <= k} L_kc xi_c, x += dx.
+// grid (ceil(maxN * 3 / (8 R)), nlane), 256 threads: one warp per R rows k of
+// the lane: dx_k = rlan1 sum_c D_kc F_c + rlan2 sum_{c <= k} L_kc xi_c, x += dx.
 // HBM-bound: the mixed-precision path streams FP32 copies of D and L
-// (products and sums in FP64), the FP64 path the FP64 matrices.
-__device__ __forceinline__ void row_dots64(const double *Drow, const double *Lrow, const double *F,
-                                           const double *xi, int n, int k, int lid, double &df, double &dr) {
-  df = 0.0;
-  dr = 0.0;
+// (products and sums in FP64), the FP64 path the FP64 matrices.  A group of
+// four columns costs 4 cycles of L1 for a row's elements but 32 for its F (four
+// doubles per lane, 32 bytes apart), so with one row per warp L1 was the bound
+// (640 MB in 187 us, 3.4 TB/s; 32 lanes of 100 to 1000 beads).  R = 4 rows share
+// the loads of F and xi: BDU_NOW.  Every row's sum has the same order for
+// either R (columns by lane, then a butterfly).
+struct Rows64 {
+  const double *D, *L;
+  size_t stride;
+};
+struct Rows32 {   // rows padded to a multiple of 4 (16-byte aligned)
+  const float *D, *L;
+  size_t stride;
+};
+
+template <int R>
+__device__ __forceinline__ void row_dots(const Rows64 &m, const double *F, const double *xi, int n, int k0, int lid,
+                                         double (&df)[R], double (&dr)[R]) {
+  const double *D[R], *L[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const size_t o = (size_t)min(k0 + r, n - 1) * m.stride;
+    D[r] = m.D + o;
+    L[r] = m.L + o;
+  }
   int c = lid;
-  for (; c + 96 < n; c += 128)
-    df += Drow[c] * F[c] + Drow[c + 32] * F[c + 32] + Drow[c + 64] * F[c + 64] + Drow[c + 96] * F[c + 96];
-  for (; c < n; c += 32) df += Drow[c] * F[c];
-  c = lid;
-  for (; c + 96 <= k; c += 128)
-    dr += Lrow[c] * xi[c] + Lrow[c + 32] * xi[c + 32] + Lrow[c + 64] * xi[c + 64] + Lrow[c + 96] * xi[c + 96];
-  for (; c <= k; c += 32) dr += Lrow[c] * xi[c];
+#pragma unroll 4
+  for (; c <= k0; c += 32) {   // L: columns up to k0 for all rows
+    const double f = F[c], x = xi[c];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      df[r] = fma(D[r][c], f, df[r]);
+      dr[r] = fma(L[r][c], x, dr[r]);
+    }
+  }
+#pragma unroll 4
+  for (; c < n; c += 32) {
+    const double f = F[c];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      df[r] = fma(D[r][c], f, df[r]);
+      if (r > 0 && c <= k0 + r) dr[r] = fma(L[r][c], xi[c], dr[r]);
+    }
+  }
 }
 
-// FP32 rows padded to a multiple of 4 (16-byte aligned): float4 loads for
-// the whole 4-column groups inside the matrix, then the < 4 last columns
-__device__ __forceinline__ void row_dots32(const float *Drow, const float *Lrow, const double *F, const double *xi,
-                                           int n, int k, int lid, double &df, double &dr) {
-  df = 0.0;
-  dr = 0.0;
-  const float4 *D4 = (const float4 *)Drow, *L4 = (const float4 *)Lrow;
+// float4 loads for the whole 4-column groups inside the matrix, then the < 4
+// last columns; k0 is a multiple of R
+template <int R>
+__device__ __forceinline__ void row_dots(const Rows32 &m, const double *F, const double *xi, int n, int k0, int lid,
+                                         double (&df)[R], double (&dr)[R]) {
+  const float4 *D4[R], *L4[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const size_t o = (size_t)min(k0 + r, n - 1) * m.stride;
+    D4[r] = (const float4 *)(m.D + o);
+    L4[r] = (const float4 *)(m.L + o);
+  }
   const int n4 = n >> 2;
-  // L is zero above the diagonal: whole groups up to column k
-  const int k4 = min((k >> 2) + 1, n4);
-  auto dot4 = [](const float4 &m, const double *v) {
-    return (double)m.x * v[0] + (double)m.y * v[1] + (double)m.z * v[2] + (double)m.w * v[3];
+  // L is zero above the diagonal: whole groups up to the rows' own columns
+  const int k4 = min((k0 >> 2) + 1, n4);
+  auto dot4 = [](const float4 &e, const double *v, double s) {
+    return fma((double)e.w, v[3], fma((double)e.z, v[2], fma((double)e.y, v[1], fma((double)e.x, v[0], s))));
   };
   int g = lid;
-  for (; g + 96 < n4; g += 128) {   // four loads in flight per lane
-    const float4 d0 = D4[g], d1 = D4[g + 32], d2 = D4[g + 64], d3 = D4[g + 96];
-    df += dot4(d0, F + 4 * g) + dot4(d1, F + 4 * g + 128) + dot4(d2, F + 4 * g + 256) + dot4(d3, F + 4 * g + 384);
+#pragma unroll 2
+  for (; g < k4; g += 32) {
+    float4 d[R], l[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) d[r] = D4[r][g];
+#pragma unroll
+    for (int r = 0; r < R; ++r) l[r] = L4[r][g];
+    const double f[4] = {F[4 * g], F[4 * g + 1], F[4 * g + 2], F[4 * g + 3]};
+    const double x[4] = {xi[4 * g], xi[4 * g + 1], xi[4 * g + 2], xi[4 * g + 3]};
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      df[r] = dot4(d[r], f, df[r]);
+      dr[r] = dot4(l[r], x, dr[r]);
+    }
   }
-  for (; g < n4; g += 32) df += dot4(D4[g], F + 4 * g);
-  if (lid < n - 4 * n4) df += (double)Drow[4 * n4 + lid] * F[4 * n4 + lid];
-  g = lid;
-  for (; g + 96 < k4; g += 128) {
-    const float4 l0 = L4[g], l1 = L4[g + 32], l2 = L4[g + 64], l3 = L4[g + 96];
-    dr += dot4(l0, xi + 4 * g) + dot4(l1, xi + 4 * g + 128) + dot4(l2, xi + 4 * g + 256) + dot4(l3, xi + 4 * g + 384);
+#pragma unroll 4
+  for (; g < n4; g += 32) {
+    const double f[4] = {F[4 * g], F[4 * g + 1], F[4 * g + 2], F[4 * g + 3]};
+#pragma unroll
+    for (int r = 0; r < R; ++r) df[r] = dot4(D4[r][g], f, df[r]);
   }
-  for (; g < k4; g += 32) dr += dot4(L4[g], xi + 4 * g);
-  if (4 * k4 + lid <= k) dr += (double)Lrow[4 * k4 + lid] * xi[4 * k4 + lid];
+  const int c = 4 * n4 + lid;
+  if (c < n) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      df[r] = fma((double)((const float *)D4[r])[c], F[c], df[r]);
+      if (c <= k0 + r) dr[r] = fma((double)((const float *)L4[r])[c], xi[c], dr[r]);
+    }
+  }
 }
 
+template <int R>
 __global__ void __launch_bounds__(256) bd_update_kernel(KArgs a) {
   const int lane = blockIdx.y;
   if (lane >= a.nlane) return;
   const LaneDesc L = a.lanes[lane];
   const int n = 3 * a.tops[L.top].nmp;
   const int warp = threadIdx.x >> 5, lid = threadIdx.x & 31;
-  const int k = blockIdx.x * 8 + warp;
+  const int k0 = (blockIdx.x * 8 + warp) * R;
   if (blockIdx.x == 0 && threadIdx.x == 0) a.lstate[lane].istep = a.bd_istep;
-  if (k >= n) return;
+  if (k0 >= n) return;
   const double *F = a.bd_F + 3 * (size_t)L.state0, *xi = a.bd_xi + 3 * (size_t)L.state0;
-  double df, dr;
+  double df[R], dr[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) df[r] = dr[r] = 0.0;
   if (a.bd_tc) {
-    const size_t row = L.bd32 + (size_t)k * ((n + 3) & ~3);
-    row_dots32(a.bd_D32 + row, a.bd_L32 + row, F, xi, n, k, lid, df, dr);
+    const int np = (n + 3) & ~3;
+    row_dots<R>(Rows32{a.bd_D32 + L.bd32, a.bd_L32 + L.bd32, (size_t)np}, F, xi, n, k0, lid, df, dr);
     if (a.bd_refine) {   // - (E z)_k / 2
-      const float4 *E4 = (const float4 *)(a.bd_E32 + row);
       const double *z = a.bd_z + 3 * (size_t)L.state0;
       const int n4 = n >> 2;
-      double ez = 0.0;
-      for (int g = lid; g < n4; g += 32) {
-        const float4 e = E4[g];
-        ez += (double)e.x * z[4 * g] + (double)e.y * z[4 * g + 1] + (double)e.z * z[4 * g + 2] + (double)e.w * z[4 * g + 3];
+#pragma unroll 1
+      for (int r = 0; r < R; ++r) {
+        const size_t row = L.bd32 + (size_t)min(k0 + r, n - 1) * np;
+        const float4 *E4 = (const float4 *)(a.bd_E32 + row);
+        double ez = 0.0;
+        for (int g = lid; g < n4; g += 32) {
+          const float4 e = E4[g];
+          ez += (double)e.x * z[4 * g] + (double)e.y * z[4 * g + 1] + (double)e.z * z[4 * g + 2] + (double)e.w * z[4 * g + 3];
+        }
+        if (lid < n - 4 * n4) ez += (double)a.bd_E32[row + 4 * n4 + lid] * z[4 * n4 + lid];
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+          if (q == r) dr[q] -= 0.5 * ez;
       }
-      if (lid < n - 4 * n4) ez += (double)a.bd_E32[row + 4 * n4 + lid] * z[4 * n4 + lid];
-      dr -= 0.5 * ez;
     }
   } else {
-    const size_t row = L.bd0 + (size_t)k * n;
-    row_dots64(a.bd_D + row, a.bd_L + row, F, xi, n, k, lid, df, dr);
+    row_dots<R>(Rows64{a.bd_D + L.bd0, a.bd_L + L.bd0, (size_t)n}, F, xi, n, k0, lid, df, dr);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    df += __shfl_xor_sync(0xffffffffu, df, o);
-    dr += __shfl_xor_sync(0xffffffffu, dr, o);
+  double mf = 0.0, mr = 0.0;   // lane r: row k0 + r
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    for (int o = 16; o > 0; o >>= 1) {
+      df[r] += __shfl_xor_sync(0xffffffffu, df[r], o);
+      dr[r] += __shfl_xor_sync(0xffffffffu, dr[r], o);
+    }
+    if (lid == r) {
+      mf = df[r];
+      mr = dr[r];
+    }
   }
-  if (lid == 0) {
+  if (lid < R && k0 + lid < n) {
     const double T = a.lab_T[a.lstate[lane].label];
     const double rl1 = a.tstep / (a.boltz * T), rl2 = sqrt(2.0 * a.tstep);
-    const double dx = rl1 * df + rl2 * dr;
-    const size_t o = 3 * (size_t)L.state0 + k;
+    const double dx = rl1 * mf + rl2 * mr;
+    const size_t o = 3 * (size_t)L.state0 + k0 + lid;
     a.xyz[o] += dx;
     a.pxyz[o] += dx;
     a.dxyz[o] += dx;
@@ -1092,6 +1172,7 @@ __global__ void __launch_bounds__(256) bd_force_kernel(KArgs a) {
   const double xi0 = x[3 * i], xi1 = x[3 * i + 1], xi2 = x[3 * i + 2];
   double fx = 0.0, fy = 0.0, fz = 0.0;
   int nclamp = 0;
+  const double far = a.wca_rcut2 * (1.0 - 1e-12);   // nat2 / dist2 is below the cutoff ratio whatever the rounding
   // entry (j, class * 2 + kind): the record's force on i is f (x_i - x_j),
   // the same numbers as -/+ f (x_i2 - x_i1) in the record's own orientation
   for (int p = p0 + lid; p < p1; p += 32) {
@@ -1108,6 +1189,7 @@ __global__ void __launch_bounds__(256) bd_force_kernel(KArgs a) {
       const double *pc = a.wca_cls + 3 * (size_t)cl;    // nat, coef rep, coef att
       const double dist2 = v0 * v0 + v1 * v1 + v2 * v2;
       const double nat2 = pc[0] * pc[0];
+      if (nat2 < far * dist2) continue;   // most pairs: no division
       const double ro2 = nat2 / dist2;
       if (ro2 < a.wca_rcut2) continue;
       const double ro4 = ro2 * ro2, ro8 = ro4 * ro4, ro14 = ro8 * ro4 * ro2;
@@ -1136,31 +1218,57 @@ __global__ void __launch_bounds__(256) bd_force_kernel(KArgs a) {
 // items[koff[k] .. koff[k + 1]) and the wide launch's items[koff[k + 1] ..
 // koff[k + 2]).  Items that factor the next diagonal tile come first, the
 // rest by decreasing tile count.  lane_T = tiles per lane.
-void bd_update_items(const std::vector<int> &lane_T, std::vector<int> &items, std::vector<int> &koff) {
+// kug[i]: column tiles per item of launch i.  UG of them share one load of the
+// 128 rows' operands, but the chip has 148 CTAs and a launch lasts as long as
+// its last item: the size with the shortest time at U_ITEM us per item, U_TILE
+// per column tile and U_DIAG for the diagonal tile (measured with 8 tiles per
+// item: UG_NOW).
+void bd_update_items(const std::vector<int> &lane_T, std::vector<int> &items, std::vector<int> &koff,
+                     std::vector<int> &kug) {
+  constexpr double U_ITEM = 5.0, U_TILE = 3.5, U_DIAG = 10.0;
   int tmax = 0;
   for (int t : lane_T) tmax = std::max(tmax, t);
   items.clear();
   koff.assign(1, 0);
+  kug.clear();
   for (int k = 0; k < tmax + 1; ++k) {
     const int nph = (k & 1) ? 2 : 1;   // odd entries: the wide launch of the pair starting at k - 1
     const int kp = k & ~1;
-    std::vector<std::pair<int, int>> ks;   // (order key, item)
-    for (size_t l = 0; l < lane_T.size(); ++l) {
-      const int m = lane_T[l] - kp - nph;
-      for (int R = 0; 2 * R < m; ++R) {
-        const int ncol = nph == 1 ? 1 : std::min(2 * R + 2, m);
-        for (int g = 0; g * UG < ncol; ++g) {
-          const int nt = std::min(UG, ncol - g * UG);
-          const int first = (R == 0 && g == 0) ? 1 << 20 : 0;   // factors the next diagonal tile
-          ks.push_back({first + nt, (int)(l << 16) | (R << 8) | g});
+    std::vector<std::pair<int, int>> best;   // (order key, item)
+    double best_time = 0.0;
+    int best_ug = UG;
+    for (int ug = UG; ug >= (nph == 1 ? UG : 1); ug >>= 1) {
+      if (ug < UG && tmax > 255 * ug) break;   // g has 8 bits
+      std::vector<std::pair<int, int>> ks;
+      double sum = 0.0, longest = 0.0;
+      for (size_t l = 0; l < lane_T.size(); ++l) {
+        const int m = lane_T[l] - kp - nph;
+        for (int R = 0; 2 * R < m; ++R) {
+          const int ncol = nph == 1 ? 1 : std::min(2 * R + 2, m);
+          for (int g = 0; g * ug < ncol; ++g) {
+            const int nt = std::min(ug, ncol - g * ug);
+            const bool first = R == 0 && g == 0;   // factors the next diagonal tile
+            ks.push_back({(first ? 1 << 20 : 0) + nt, (int)(l << 16) | (R << 8) | g});
+            const double t = U_ITEM + nt * U_TILE + (first ? U_DIAG : 0.0);
+            sum += t;
+            longest = std::max(longest, t);
+          }
         }
       }
+      // the longest come first, so the rest fills up behind them
+      const double time = std::max(longest, sum / BD_SMS + 0.5 * (U_ITEM + ug * U_TILE));
+      if (best.empty() || time < best_time) {
+        best.swap(ks);
+        best_time = time;
+        best_ug = ug;
+      }
     }
-    std::stable_sort(ks.begin(), ks.end(), [](const std::pair<int, int> &x, const std::pair<int, int> &y) {
+    std::stable_sort(best.begin(), best.end(), [](const std::pair<int, int> &x, const std::pair<int, int> &y) {
       return x.first > y.first;
     });
-    for (auto &e : ks) items.push_back(e.second);
+    for (auto &e : best) items.push_back(e.second);
     koff.push_back((int)items.size());
+    kug.push_back(best_ug);
   }
 }
 
@@ -1175,7 +1283,8 @@ cudaError_t panel_launch(cudaStream_t st, const KArgs &a, int m) {
   return cudaGetLastError();
 }
 
-cudaError_t bd_refactor_launch(cudaStream_t st, KArgs a, int max_nmp, const int *items, const int *koff) {
+cudaError_t bd_refactor_launch(cudaStream_t st, KArgs a, int max_nmp, const int *items, const int *koff,
+                               const int *kug) {
   cudaError_t e = cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FD_VEC * sizeof(double));
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(chol_update_kernel<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, U64_SMEM);
@@ -1186,7 +1295,7 @@ cudaError_t bd_refactor_launch(cudaStream_t st, KArgs a, int max_nmp, const int 
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(chol_update_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, U_SMEM + 1024);
   if (e != cudaSuccess) return e;
-  if (a.bd_tc && (!a.bd_P || !items || !koff)) return cudaErrorInvalidValue;
+  if (a.bd_tc && (!a.bd_P || !items || !koff || !kug)) return cudaErrorInvalidValue;
   const long long nn = (long long)max_nmp * max_nmp;
   rpy_kernel<<<dim3((unsigned)((nn + 255) / 256), a.nlane), 256, 0, st>>>(a);
   chol_diag_kernel<<<a.nlane, 256, FD_VEC * sizeof(double), st>>>(a);
@@ -1198,14 +1307,14 @@ cudaError_t bd_refactor_launch(cudaStream_t st, KArgs a, int max_nmp, const int 
       e = panel_launch(st, a, T - k - 1);
       if (e != cudaSuccess) return e;
       int nit = koff[k + 1] - koff[k];
-      if (nit > 0) chol_update_tc_kernel<<<nit, U_THREADS, U_SMEM + 1024, st>>>(a, items + koff[k], 1);
+      if (nit > 0) chol_update_tc_kernel<<<nit, U_THREADS, U_SMEM + 1024, st>>>(a, items + koff[k], 1, kug[k]);
       if (k + 2 < T) {
         KArgs b = a;
         b.bd_kpanel = k + 1;
         e = panel_launch(st, b, T - k - 2);
         if (e != cudaSuccess) return e;
         nit = koff[k + 2] - koff[k + 1];
-        if (nit > 0) chol_update_tc_kernel<<<nit, U_THREADS, U_SMEM + 1024, st>>>(a, items + koff[k + 1], 2);
+        if (nit > 0) chol_update_tc_kernel<<<nit, U_THREADS, U_SMEM + 1024, st>>>(a, items + koff[k + 1], 2, kug[k + 1]);
       }
     }
   } else {
@@ -1253,7 +1362,11 @@ cudaError_t bd_step_launch(cudaStream_t st, const KArgs &a, int max_nmp) {
     if (e != cudaSuccess) return e;
     refine_trsv_kernel<<<a.nlane, TRSV_THREADS, sm, st>>>(a);
   }
-  bd_update_kernel<<<dim3((3 * max_nmp + 7) / 8, a.nlane), 256, 0, st>>>(a);
+  // four rows per warp once that still gives every SM two CTAs (64 rows)
+  if ((long long)3 * max_nmp * a.nlane >= 64LL * BD_SMS)
+    bd_update_kernel<4><<<dim3((3 * max_nmp + 31) / 32, a.nlane), 256, 0, st>>>(a);
+  else
+    bd_update_kernel<1><<<dim3((3 * max_nmp + 7) / 8, a.nlane), 256, 0, st>>>(a);
   bd_force_kernel<<<dim3((max_nmp + 7) / 8, a.nlane), 256, 0, st>>>(a);
   return cudaGetLastError();
 }
