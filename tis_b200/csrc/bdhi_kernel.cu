@@ -864,8 +864,10 @@ __global__ void __launch_bounds__(128) bd_noise_kernel(KArgs a) {
 // four columns costs 4 cycles of L1 for a row's elements but 32 for its F (four
 // doubles per lane, 32 bytes apart), so with one row per warp L1 was the bound
 // (640 MB in 187 us, 3.4 TB/s; 32 lanes of 100 to 1000 beads).  R = 4 rows share
-// the loads of F and xi: BDU_NOW.  Every row's sum has the same order for
-// either R (columns by lane, then a butterfly).
+// the loads of F and xi, and the matrices stream past L1 with 16 float4 in flight
+// per lane: 116 us (5.6 TB/s; more rows, warps or bytes in flight, or rows
+// staged by bulk copies, were no faster).  Every row's sum has the same order
+// for either R (columns by lane, then a butterfly).
 struct Rows64 {
   const double *D, *L;
   size_t stride;
@@ -929,9 +931,9 @@ __device__ __forceinline__ void row_dots(const Rows32 &m, const double *F, const
   for (; g < k4; g += 32) {
     float4 d[R], l[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) d[r] = D4[r][g];
+    for (int r = 0; r < R; ++r) d[r] = __ldcs(&D4[r][g]);
 #pragma unroll
-    for (int r = 0; r < R; ++r) l[r] = L4[r][g];
+    for (int r = 0; r < R; ++r) l[r] = __ldcs(&L4[r][g]);
     const double f[4] = {F[4 * g], F[4 * g + 1], F[4 * g + 2], F[4 * g + 3]};
     const double x[4] = {xi[4 * g], xi[4 * g + 1], xi[4 * g + 2], xi[4 * g + 3]};
 #pragma unroll
@@ -944,7 +946,7 @@ __device__ __forceinline__ void row_dots(const Rows32 &m, const double *F, const
   for (; g < n4; g += 32) {
     const double f[4] = {F[4 * g], F[4 * g + 1], F[4 * g + 2], F[4 * g + 3]};
 #pragma unroll
-    for (int r = 0; r < R; ++r) df[r] = dot4(D4[r][g], f, df[r]);
+    for (int r = 0; r < R; ++r) df[r] = dot4(__ldcs(&D4[r][g]), f, df[r]);
   }
   const int c = 4 * n4 + lid;
   if (c < n) {
@@ -957,7 +959,7 @@ __device__ __forceinline__ void row_dots(const Rows32 &m, const double *F, const
 }
 
 template <int R>
-__global__ void __launch_bounds__(256) bd_update_kernel(KArgs a) {
+__global__ void __launch_bounds__(256, 2) bd_update_kernel(KArgs a) {
   const int lane = blockIdx.y;
   if (lane >= a.nlane) return;
   const LaneDesc L = a.lanes[lane];
@@ -1174,30 +1176,48 @@ __global__ void __launch_bounds__(256) bd_force_kernel(KArgs a) {
   int nclamp = 0;
   const double far = a.wca_rcut2 * (1.0 - 1e-12);   // nat2 / dist2 is below the cutoff ratio whatever the rounding
   // entry (j, class * 2 + kind): the record's force on i is f (x_i - x_j),
-  // the same numbers as -/+ f (x_i2 - x_i1) in the record's own orientation
-  for (int p = p0 + lid; p < p1; p += 32) {
-    const int2 ent = a.bd_ent[T.be0 + p];
-    const int j = ent.x, cl = ent.y >> 1;
-    const double v0 = xi0 - x[3 * j], v1 = xi1 - x[3 * j + 1], v2 = xi2 - x[3 * j + 2];
-    double f;
-    if (!(ent.y & 1)) {
-      const double *pc = a.fene_cls + 3 * (size_t)cl;   // nat, coef, dist2
-      const double dist = sqrt(v0 * v0 + v1 * v1 + v2 * v2);
-      const double dd = dist - pc[0];
-      f = -pc[1] * dd / (1.0 - dd * dd / pc[2]) / dist;
-    } else {
-      const double *pc = a.wca_cls + 3 * (size_t)cl;    // nat, coef rep, coef att
-      const double dist2 = v0 * v0 + v1 * v1 + v2 * v2;
-      const double nat2 = pc[0] * pc[0];
-      if (nat2 < far * dist2) continue;   // most pairs: no division
-      const double ro2 = nat2 / dist2;
-      if (ro2 < a.wca_rcut2) continue;
-      const double ro4 = ro2 * ro2, ro8 = ro4 * ro4, ro14 = ro8 * ro4 * ro2;
-      const double coef = (ro2 > 1.0) ? pc[1] : pc[2];
-      f = 12.0 * coef / nat2 * (ro14 - ro8);
-      if (f > 50.0) { f = 50.0; nclamp += j > i; }   // DE_MAX; the record is counted once, from its lower bead
+  // the same numbers as -/+ f (x_i2 - x_i1) in the record's own orientation.
+  // A lane's entries, four at a time: entries, then positions and classes,
+  // are in flight together (one at a time each waited for its own two loads)
+  constexpr int U = 4;
+  for (int pb = p0 + lid; pb < p1; pb += 32 * U) {
+    int2 e[U];
+    double v[U][3], dist2[U], nat[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) e[u] = pb + 32 * u < p1 ? a.bd_ent[T.be0 + pb + 32 * u] : make_int2(-1, 0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int j = max(e[u].x, 0);
+      v[u][0] = xi0 - x[3 * j];
+      v[u][1] = xi1 - x[3 * j + 1];
+      v[u][2] = xi2 - x[3 * j + 2];
+      nat[u] = ((e[u].y & 1) ? a.wca_cls : a.fene_cls)[3 * (size_t)(e[u].y >> 1)];
     }
-    fx += f * v0; fy += f * v1; fz += f * v2;
+#pragma unroll
+    for (int u = 0; u < U; ++u) dist2[u] = v[u][0] * v[u][0] + v[u][1] * v[u][1] + v[u][2] * v[u][2];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int cl = e[u].y >> 1;
+      if (e[u].x < 0) continue;
+      double f;
+      if (!(e[u].y & 1)) {
+        const double *pc = a.fene_cls + 3 * (size_t)cl;   // nat, coef, dist2
+        const double dist = sqrt(dist2[u]);
+        const double dd = dist - nat[u];
+        f = -pc[1] * dd / (1.0 - dd * dd / pc[2]) / dist;
+      } else {
+        const double *pc = a.wca_cls + 3 * (size_t)cl;    // nat, coef rep, coef att
+        const double nat2 = nat[u] * nat[u];
+        if (nat2 < far * dist2[u]) continue;   // most pairs: no division
+        const double ro2 = nat2 / dist2[u];
+        if (ro2 < a.wca_rcut2) continue;
+        const double ro4 = ro2 * ro2, ro8 = ro4 * ro4, ro14 = ro8 * ro4 * ro2;
+        const double coef = (ro2 > 1.0) ? pc[1] : pc[2];
+        f = 12.0 * coef / nat2 * (ro14 - ro8);
+        if (f > 50.0) { f = 50.0; nclamp += e[u].x > i; }   // DE_MAX; the record is counted once, from its lower bead
+      }
+      fx += f * v[u][0]; fy += f * v[u][1]; fz += f * v[u][2];
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
     fx += __shfl_xor_sync(0xffffffffu, fx, o);
