@@ -1180,11 +1180,18 @@ __global__ void __launch_bounds__(256) bd_force_kernel(KArgs a) {
   // A lane's entries, four at a time: entries, then positions and classes,
   // are in flight together (one at a time each waited for its own two loads)
   constexpr int U = 4;
+  int2 nx[U];   // the next four
+  auto fetch = [&](int pb) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) nx[u] = pb + 32 * u < p1 ? __ldcs(&a.bd_ent[T.be0 + pb + 32 * u]) : make_int2(-1, 0);
+  };
+  fetch(p0 + lid);
   for (int pb = p0 + lid; pb < p1; pb += 32 * U) {
     int2 e[U];
     double v[U][3], dist2[U], nat[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) e[u] = pb + 32 * u < p1 ? a.bd_ent[T.be0 + pb + 32 * u] : make_int2(-1, 0);
+    for (int u = 0; u < U; ++u) e[u] = nx[u];
+    fetch(pb + 32 * U);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int j = max(e[u].x, 0);
