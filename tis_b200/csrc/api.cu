@@ -192,6 +192,9 @@ struct tis_ctx {
   int ew_ncol = 0, hmax = 0, nq_max = 0;
   DBuf<char4> ew_col;
   DBuf<double> ew_w, ew_S, f_ext;
+  int ew_work = 0;                  // worker CTAs of the reciprocal sum in the split lanes' launch (0: its own kernels)
+  DBuf<unsigned> ew_sync;
+  DBuf<double2> ew_E;
   // Brownian dynamics with hydrodynamic interactions
   bool bdhi = false;
   int max_nmp = 0;
@@ -1296,6 +1299,17 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     CK(c->ew_col.upload(col));
     CK(c->ew_w.upload(w));
     CK(c->ew_S.alloc((size_t)nlane * EW_H * c->ew_ncol * 4));
+    // every lane split and SMs left over: the reciprocal sum runs beside the
+    // lanes in one launch per call.  It takes the chip's rest, so a batch
+    // that leaves less than about a third of it keeps the separate kernels
+    if (c->nsplit && c->n_split == nlane && c->nq_max > 0) {
+      const int left = split_clusters(c->nsplit, p.precision == TIS_PREC_MIXED, true) - nlane;
+      if (left * c->nsplit >= 48) {
+        c->ew_work = left * c->nsplit;
+        CK(c->ew_sync.alloc(EWS_WORDS));
+        CK(c->ew_E.alloc((size_t)nlane * 3 * c->nq_max));
+      }
+    }
     CK(c->f_ext.alloc(n3));
     CK(cudaMemset(c->f_ext.p, 0, n3 * 8));
   }
@@ -1347,7 +1361,7 @@ extern "C" void tis_destroy(tis_ctx *c) {
   c->out_force.free(); c->out_energy.free(); c->scale.free();
   c->mask.free(); c->site_exc.free(); c->mirror.free(); c->hb_flag.free();
   c->hb_ene.free(); c->hb_flag2.free(); c->hb_ene2.free(); c->site_exc2.free(); c->slots.free(); c->noise.free(); c->unif.free(); c->lane_n.free(); c->d_order.free();
-  c->ew_col.free(); c->ew_w.free(); c->ew_S.free(); c->f_ext.free();
+  c->ew_col.free(); c->ew_w.free(); c->ew_S.free(); c->f_ext.free(); c->ew_sync.free(); c->ew_E.free();
   c->fene_idx.free(); c->wca_idx.free(); c->bd_ptr.free(); c->bd_ent.free(); c->fene_cls.free(); c->wca_cls.free(); c->b_hrad.free(); c->d_not_spd.free();
   c->fene_nat.free(); c->fene_coef.free(); c->fene_d2.free(); c->wca_nat.free(); c->wca_coef.free();
   c->bd_D64.free(); c->bd_z.free(); c->bd_E32.free(); c->bd_W32.free();
@@ -1497,8 +1511,10 @@ KArgs make_args(tis_ctx *c, int mode, int nsteps, int only_lane) {
     a.hmax = c->hmax; a.ew_ncol = c->ew_ncol;
     a.two_pi_L = 2.0 * F_PI / p.psize[0];
     a.ew_col = c->ew_col.p; a.ew_w = c->ew_w.p; a.ew_S = c->ew_S.p;
+    a.ew_sync = c->ew_sync.p; a.ew_E = c->ew_E.p; a.ew_nqmax = c->nq_max;
   }
   a.f_ext = nullptr;
+  a.ew_nwork = 0;
   a.fene_idx = c->fene_idx.p; a.fene_nat = c->fene_nat.p; a.fene_coef = c->fene_coef.p; a.fene_d2 = c->fene_d2.p;
   a.wca_idx = c->wca_idx.p; a.wca_nat = c->wca_nat.p; a.wca_coef = c->wca_coef.p;
   a.wca_rcut2 = 1.0 / (p.wca_coef_cutoff * p.wca_coef_cutoff);
@@ -1627,6 +1643,10 @@ int check_lanes(tis_ctx *c) {
     if (ls[i].flags & LF_PMF)
       code = fail(c, TIS_E_PMF_RANGE, "Mg-P pair below the PMF table in lane " + std::to_string(i + 1));
     if (ls[i].flags & LF_OVERFLOW) code = fail(c, TIS_E_LIST_OVERFLOW, "hbond site list overflow");
+    if (ls[i].flags & LF_WAIT) {
+      c->wait_timeout = 1;
+      code = fail(c, TIS_E_TIMEOUT, "a wait for the reciprocal Ewald sum gave up in lane " + std::to_string(i + 1));
+    }
     if (ls[i].flags & LF_SMEM)
       code = fail(c, TIS_E_UNSUPPORTED, "the shared-memory layout of lane " + std::to_string(i + 1) + " does not fit");
     if (ls[i].flags & (LF_UNIF_EXHAUSTED | LF_NOISE_EXHAUSTED))
@@ -1887,6 +1907,13 @@ int enqueue_steps(tis_ctx *c, int nsteps, const int *lane_n_dev) {
       c->bd_istep = istep;
     }
   } else if (c->par.i_ele != TIS_ELE_EWALD) {
+    int rc = launch_lane(c, a);
+    if (rc < 0) return rc;
+  } else if (c->ew_work && !lane_n_dev) {
+    // one launch: the lanes' clusters and the workers of the reciprocal sum
+    CK(cudaMemsetAsync(c->ew_sync.p, 0, EWS_WORDS * sizeof(unsigned), c->stream));
+    a.f_ext = c->f_ext.p;
+    a.ew_nwork = c->ew_work;
     int rc = launch_lane(c, a);
     if (rc < 0) return rc;
   } else {

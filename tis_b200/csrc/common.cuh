@@ -20,6 +20,7 @@ constexpr int MAX_THREADS = 1024;
 constexpr int N_ETYPE = 25;   // E_TYPE%MAX
 constexpr int CHMAX = 1024;   // electrostatic row chunks per lane (at least one per charged bead)
 constexpr int EW_H = 12;      // Ewald: hz = 0 .. 11 of a column (hx, hy) of reciprocal vectors
+enum { EWS_READY = 0, EWS_BARRIER = 32, EWS_DONE = 64, EWS_ABORT = 96, EWS_WORDS = 128 };   // words of ew_sync
 constexpr int EW_COLS = 192;  // columns of the half space at most (189 for |h| <= 11)
 // HI_TENSOR (const_index.F90:39-45)
 constexpr int TIS_HI_RPY_DEV = 1, TIS_HI_RPY_OVER_DEV = 2, TIS_HI_ERMAK_OVER_DEV = 3, TIS_HI_ZUK_RPY_DEV = 4;
@@ -84,7 +85,8 @@ struct LaneState {
 };
 
 enum LaneFlags { LF_OVERFLOW = 1, LF_NAN = 2, LF_UNIF_EXHAUSTED = 4, LF_NOISE_EXHAUSTED = 8, LF_PMF = 16,
-                 LF_SMEM = 32 /* the lane's base layout did not fit the launch's shared memory: nothing ran */ };
+                 LF_SMEM = 32 /* the lane's base layout did not fit the launch's shared memory: nothing ran */,
+                 LF_WAIT = 64 /* a wait for the reciprocal sum gave up */ };
 
 enum KMode {
   KM_NEIGHBOR = 1,     // rebuild lists (wrap pxyz if periodic)
@@ -147,6 +149,10 @@ struct KArgs {
   const double *ew_w;             // (EW_H, ncol) weight of +-hz: 2 C(k) (hz = 0: C(k)), C(k) = 2 pi / L^3
                                   // exp(-k^2 / 4 alpha^2) / k^2; half for the column (0, 0)
   double *ew_S;                   // (lane, EW_H, ncol, 4) structure-factor sums of +-hz
+  // reciprocal sum inside the launch of the split lanes (split_ewald.cuh); ew_nwork 0: separate kernels
+  int ew_nwork, ew_nqmax;         // worker CTAs behind the lanes'; largest charge count of a lane
+  unsigned *ew_sync;              // counters
+  double2 *ew_E;                  // (lane, 3, ew_nqmax) e^{i 2 pi x_d / L} of the charges
   double *f_ext;                  // (3, nbead_total) force added to each bead's sum, or null
   // Brownian dynamics with hydrodynamic interactions (time_integral.F90:429-457)
   const int *fene_idx; const double *fene_nat, *fene_coef, *fene_d2;   // force_fene.F90

@@ -44,6 +44,7 @@
 #include <type_traits>
 
 #include "lane_common.cuh"
+#include "split_ewald.cuh"
 #include "split_plan.cuh"
 
 namespace tis {
@@ -259,6 +260,12 @@ __device__ __forceinline__ void acopy4(void *dst, const void *src) { __pipeline_
 template <typename Real, int NT, bool PER>
 __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs a) {
   typedef typename V4<Real>::T V;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if constexpr (PER)
+    if (a.ew_nwork && blockIdx.x >= gridDim.x - (unsigned)a.ew_nwork) {
+      ewald_worker<NT>(a, smem_raw);
+      return;
+    }
   const cg::cluster_group cl = cg::this_cluster();
   const int nr = a.nsplit, rank = (int)cl.block_rank();
   const int lane = (a.only_lane >= 0) ? a.only_lane
@@ -277,7 +284,6 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   constexpr int NW = NT / 32;
   const bool skin = a.n_step_neighbor <= 0;
   LaneState &st = a.lstate[lane];
-  extern __shared__ __align__(16) unsigned char smem_raw[];
   const SplitPlan &pl = a.sp;
   SplitSmem<Real> s;
   unsigned char *sm = smem_raw;
@@ -752,6 +758,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     }
   };
 
+  unsigned ew_done = 0;   // count of the workers' forces of this step
   // ---- one evaluation of the forces, up to and including the second barrier
   const double cdist = a.lab_cdist[label], coefT = a.lab_coef[label];
   const Real rcd = (Real)(1.0 / cdist);
@@ -1137,6 +1144,8 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     if (tid == 0) { atomicAdd(&g_phase[64 + blockIdx.x % 16], (unsigned long long)misc[15]); misc[15] = 0; }
 #endif
     PHASE_T0(t_b);
+    if constexpr (PER)
+      if (a.ew_nwork && tid == 0) ew_wait(a, EWS_DONE, ew_done);   // this step's reciprocal forces
     cl.sync();
     PHASE_ADD(2, t_b);
     PHASE_CTA(80, t_b);
@@ -1189,6 +1198,25 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     PHASE_T0(t_a);
     cl.sync();   // the positions of this step are complete
     PHASE_ADD(3, t_a);
+    if constexpr (PER)
+      if (a.ew_nwork) {
+        ew_done = (unsigned)(step + 1) * (unsigned)a.ew_nwork;
+        if (warp == NW - 1) {   // the workers' input: the own charges' exponentials
+          double2 *E = a.ew_E + (size_t)lane * 3 * a.ew_nqmax;
+          for (int k = lid; k < NQ; k += 32) {
+            const int i = qb[k];
+            if (i < lo || i >= hi) continue;
+            const double P[3] = {s.PX[i], s.PY[i], s.PZ[i]};
+            for (int d = 0; d < 3; ++d) {
+              double sn, cs;
+              sincos(a.two_pi_L * P[d], &sn, &cs);
+              __stcg(E + d * a.ew_nqmax + k, make_double2(cs, sn));
+            }
+          }
+          __syncwarp();
+          if (lid == 0) ew_signal(a, EWS_READY);
+        }
+      }
     const bool next = a.mode == KM_STEP ? step + 1 < nloop
                                         : (a.mode == KM_VXSTEP && (!a.lane_nsteps || a.step_k + 1 < a.lane_nsteps[lane]));
     // trigger of the next step's x update
@@ -1218,7 +1246,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
       PHASE_ADD(10, t_u);
       if (valid && g < 3) {
         double f = (g == 0 ? fx : (g == 1 ? fy : fz)) + exF[3 * li + g] + dhF[3 * li + g];
-        if (PER && a.f_ext) f += a.f_ext[3 * (size_t)(L.state0 + i) + g];   // the reciprocal-space force
+        if (PER && a.f_ext) f += __ldcg(a.f_ext + 3 * (size_t)(L.state0 + i) + g);   // the reciprocal-space force
         const int q = g * OS + li;
         if (a.mode == KM_FORCE) {
           a.out_force[3 * (size_t)(L.state0 + i) + g] = f;
@@ -1266,6 +1294,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     if (misc[MISC_CLAMP]) atomicAdd((unsigned long long *)&st.nclamp, (unsigned long long)misc[MISC_CLAMP]);
     if (misc[MISC_NAN]) atomicOr(&st.flags, LF_NAN);
     if (misc[MISC_PMF]) atomicOr(&st.flags, LF_PMF);
+    if (PER && a.ew_nwork && rank == 0 && __ldcg(a.ew_sync + EWS_ABORT)) atomicOr(&st.flags, LF_WAIT);
     if (rank == 0) st.istep = istep_end;
   }
 }

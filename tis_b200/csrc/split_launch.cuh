@@ -20,8 +20,14 @@ inline void split_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int n
 template <typename Real, int NT, bool PER>
 cudaError_t split_run(int nlane, size_t smem, cudaStream_t st, const KArgs &a) {
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   split_config(cfg, at, nlane, a.nsplit, NT, smem, st);
+  if (a.ew_nwork) {   // lanes and workers wait for one another: all resident, or an error
+    cfg.gridDim.x += a.ew_nwork;
+    at[1].id = cudaLaunchAttributeCooperative;
+    at[1].val.cooperative = 1;
+    cfg.numAttrs = 2;
+  }
   return cudaLaunchKernelEx(&cfg, split_kernel<Real, NT, PER>, a);
 }
 
