@@ -192,6 +192,7 @@ struct tis_ctx {
   int ew_ncol = 0, hmax = 0, nq_max = 0;
   DBuf<char4> ew_col;
   DBuf<double> ew_w, ew_S, f_ext;
+  int ew_nb = 0;
   int ew_work = 0;                  // worker CTAs of the reciprocal sum in the split lanes' launch (0: its own kernels)
   DBuf<unsigned> ew_sync;
   DBuf<double2> ew_E;
@@ -1304,10 +1305,11 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     // that leaves less than about a third of it keeps the separate kernels
     if (c->nsplit && c->n_split == nlane && c->nq_max > 0) {
       const int left = split_clusters(c->nsplit, p.precision == TIS_PREC_MIXED, true) - nlane;
-      if (left * c->nsplit >= 48) {
+      if (left * c->nsplit >= 48 && ew_smem(nlane, c->nq_max, c->ew_ncol).total <= 227 * 1024) {
         c->ew_work = left * c->nsplit;
+        c->ew_nb = (int)(n3 / 3);
         CK(c->ew_sync.alloc(EWS_WORDS));
-        CK(c->ew_E.alloc((size_t)nlane * 3 * c->nq_max));
+        CK(c->ew_E.alloc((size_t)EW_H * n3));
       }
     }
     CK(c->f_ext.alloc(n3));
@@ -1512,6 +1514,7 @@ KArgs make_args(tis_ctx *c, int mode, int nsteps, int only_lane) {
     a.two_pi_L = 2.0 * F_PI / p.psize[0];
     a.ew_col = c->ew_col.p; a.ew_w = c->ew_w.p; a.ew_S = c->ew_S.p;
     a.ew_sync = c->ew_sync.p; a.ew_E = c->ew_E.p; a.ew_nqmax = c->nq_max;
+    a.ew_nb = c->ew_nb;
   }
   a.f_ext = nullptr;
   a.ew_nwork = 0;

@@ -152,7 +152,8 @@ struct KArgs {
   // reciprocal sum inside the launch of the split lanes (split_ewald.cuh); ew_nwork 0: separate kernels
   int ew_nwork, ew_nqmax;         // worker CTAs behind the lanes'; largest charge count of a lane
   unsigned *ew_sync;              // counters
-  double2 *ew_E;                  // (lane, 3, ew_nqmax) e^{i 2 pi x_d / L} of the charges
+  int ew_nb;                      // beads of the context
+  double2 *ew_E;                  // (EW_H, 3, ew_nb) powers e^{i 2 pi h x_d / L}
   double *f_ext;                  // (3, nbead_total) force added to each bead's sum, or null
   // Brownian dynamics with hydrodynamic interactions (time_integral.F90:429-457)
   const int *fene_idx; const double *fene_nat, *fene_coef, *fene_d2;   // force_fene.F90

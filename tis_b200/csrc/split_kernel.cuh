@@ -1195,28 +1195,16 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     if (step >= nloop) break;
     // dxyz_mp = 0 (time_integral_pre.F90:79)
     if (a.mode == KM_PRE && skin) for (int q = tid; q < 3 * OS; q += NT) Dv[q] = 0.0;
+    if constexpr (PER)
+      if (a.ew_nwork) {   // (behind send's barrier)
+        ew_done = (unsigned)(step + 1) * (unsigned)a.ew_nwork;
+        ew_publish(a, s.PX, np, lo, nown, L.state0, tid, NT);
+      }
     PHASE_T0(t_a);
     cl.sync();   // the positions of this step are complete
     PHASE_ADD(3, t_a);
     if constexpr (PER)
-      if (a.ew_nwork) {
-        ew_done = (unsigned)(step + 1) * (unsigned)a.ew_nwork;
-        if (warp == NW - 1) {   // the workers' input: the own charges' exponentials
-          double2 *E = a.ew_E + (size_t)lane * 3 * a.ew_nqmax;
-          for (int k = lid; k < NQ; k += 32) {
-            const int i = qb[k];
-            if (i < lo || i >= hi) continue;
-            const double P[3] = {s.PX[i], s.PY[i], s.PZ[i]};
-            for (int d = 0; d < 3; ++d) {
-              double sn, cs;
-              sincos(a.two_pi_L * P[d], &sn, &cs);
-              __stcg(E + d * a.ew_nqmax + k, make_double2(cs, sn));
-            }
-          }
-          __syncwarp();
-          if (lid == 0) ew_signal(a, EWS_READY);
-        }
-      }
+      if (a.ew_nwork && tid == 0) ew_signal(a, EWS_READY);
     const bool next = a.mode == KM_STEP ? step + 1 < nloop
                                         : (a.mode == KM_VXSTEP && (!a.lane_nsteps || a.step_k + 1 < a.lane_nsteps[lane]));
     // trigger of the next step's x update
@@ -1238,6 +1226,8 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
       const int li = l0 + grp, i = lo + li;
       const bool valid = li < nown;
       double fx = 0, fy = 0, fz = 0;
+      // the reciprocal-space force (from L2: other SMs wrote it)
+      const double fe = (PER && a.f_ext && valid && g < 3) ? __ldcg(a.f_ext + 3 * (size_t)(L.state0 + i) + g) : 0.0;
       if (valid)
         for (int p = iptr[li] + g; p < iptr[li + 1]; p += SG) {
           fx += (double)slots[3 * p]; fy += (double)slots[3 * p + 1]; fz += (double)slots[3 * p + 2];
@@ -1246,7 +1236,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
       PHASE_ADD(10, t_u);
       if (valid && g < 3) {
         double f = (g == 0 ? fx : (g == 1 ? fy : fz)) + exF[3 * li + g] + dhF[3 * li + g];
-        if (PER && a.f_ext) f += __ldcg(a.f_ext + 3 * (size_t)(L.state0 + i) + g);   // the reciprocal-space force
+        if (PER) f += fe;
         const int q = g * OS + li;
         if (a.mode == KM_FORCE) {
           a.out_force[3 * (size_t)(L.state0 + i) + g] = f;

@@ -1,5 +1,7 @@
 // split_launch.cuh -- launches of split_kernel.
 #pragma once
+#include <algorithm>
+
 #include "split_kernel.cuh"
 
 namespace tis {
@@ -24,6 +26,7 @@ cudaError_t split_run(int nlane, size_t smem, cudaStream_t st, const KArgs &a) {
   split_config(cfg, at, nlane, a.nsplit, NT, smem, st);
   if (a.ew_nwork) {   // lanes and workers wait for one another: all resident, or an error
     cfg.gridDim.x += a.ew_nwork;
+    cfg.dynamicSmemBytes = std::max<size_t>(smem, ew_smem(a.nlane, a.ew_nqmax, a.ew_ncol).total);
     at[1].id = cudaLaunchAttributeCooperative;
     at[1].val.cooperative = 1;
     cfg.numAttrs = 2;

@@ -81,4 +81,28 @@ inline SplitPlan split_plan(const TopDesc &T, int nq, int row, int nr, bool peri
   return p;
 }
 
+// Workers of the reciprocal Ewald sum (split_ewald.cuh).
+constexpr int EW_WQ = 8;   // charges of a force block at most
+// Their shared memory: reductions, the force block's exponentials, and
+// what never changes during a launch (the waits drop L1, so it would come from
+// L2 step after step, through four dependent loads)
+struct EwSmem {
+  unsigned red, ex, rf, wt, bq, bi, lane, col, total;
+};
+__host__ __device__ inline EwSmem ew_smem(int nlane, int nqm, int ncol) {
+  EwSmem m;
+  unsigned b = 0;
+  auto take = [&](unsigned bytes) { const unsigned at = b; b = (b + bytes + 15u) & ~15u; return at; };
+  m.red = take(8 * 4 * 16 * 6);                // sums of the warps: 512 threads 4 groups x 24, 256 threads 2 x 48
+  m.ex = take(16 * EW_WQ * 3 * EW_H);
+  m.rf = take(8 * 16 * 32);
+  m.wt = take(8 * EW_H * ncol);
+  m.bq = take(8 * nlane * nqm);                // charges, in the order of
+  m.bi = take(4 * nlane * nqm);                // their rows in ew_E
+  m.lane = take(16 * nlane);                   // force factor, charges
+  m.col = take(4 * ncol);
+  m.total = b;
+  return m;
+}
+
 } // namespace tis
