@@ -30,6 +30,8 @@ namespace tis {
 
 constexpr int EW_WAIT_POLLS = 4000000;   // about 2 s
 
+// By a whole warp: after a loop that one thread takes alone the warp stayed in
+// two parts, up to the next shuffle (4 k cycles of a lane's update).
 __device__ __forceinline__ void ew_wait(const KArgs &a, int word, unsigned target) {
   const unsigned *p = a.ew_sync + word;
   for (int i = 0;; ++i) {
@@ -45,6 +47,7 @@ __device__ __forceinline__ void ew_wait(const KArgs &a, int word, unsigned targe
   }
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  __syncwarp();
 }
 
 // called by one thread after a barrier behind the writes it announces
@@ -126,7 +129,7 @@ __device__ __forceinline__ void ewald_worker(const KArgs &a, unsigned char *smem
   __syncthreads();
   const int per = min(EW_WQ, (nqm * a.nlane + nw - 1) / nw), blocks = (nqm + per - 1) / per;
   for (int step = 0; step < a.nsteps; ++step) {
-    if (tid == 0) ew_wait(a, EWS_READY, (unsigned)(step + 1) * (unsigned)(a.nlane * a.nsplit));
+    if (warp == 0) ew_wait(a, EWS_READY, (unsigned)(step + 1) * (unsigned)(a.nlane * a.nsplit));
     __syncthreads();
     // ---- structure factors, see ewald_kernel.cu: 128 threads a column (or half of one)
     {
@@ -188,10 +191,8 @@ __device__ __forceinline__ void ewald_worker(const KArgs &a, unsigned char *smem
       }
     }
     __syncthreads();
-    if (tid == 0) {
-      ew_signal(a, EWS_BARRIER);
-      ew_wait(a, EWS_BARRIER, (unsigned)(step + 1) * (unsigned)nw);
-    }
+    if (tid == 0) ew_signal(a, EWS_BARRIER);
+    if (warp == 0) ew_wait(a, EWS_BARRIER, (unsigned)(step + 1) * (unsigned)nw);
     __syncthreads();
     // ---- forces of `per` charges: a thread per column (or half of one)
     for (int u = w; u < a.nlane * blocks; u += nw) {

@@ -1145,7 +1145,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
 #endif
     PHASE_T0(t_b);
     if constexpr (PER)
-      if (a.ew_nwork && tid == 0) ew_wait(a, EWS_DONE, ew_done);   // this step's reciprocal forces
+      if (a.ew_nwork && warp == 0) ew_wait(a, EWS_DONE, ew_done);   // this step's reciprocal forces
     cl.sync();
     PHASE_ADD(2, t_b);
     PHASE_CTA(80, t_b);
