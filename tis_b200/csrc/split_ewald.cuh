@@ -209,14 +209,14 @@ __device__ __forceinline__ void ewald_worker(const KArgs &a, unsigned char *smem
       const int mz = col.z, mw = __reduce_max_sync(0xffffffffu, mz);   // CP is a multiple of 32: h0 is the warp's
       double p[HN], r[HN], s[HN], t[HN];
 #pragma unroll
-      for (int h = 0; h < HN; ++h) {
-        p[h] = r[h] = s[h] = t[h] = 0.0;
-        if (h0 + h <= mz) {
-          const double2 *S = (const double2 *)(a.ew_S + (((size_t)lane * EW_H + h0 + h) * ncol + c) * 4);
-          const double2 S0 = __ldcg(S), S1 = __ldcg(S + 1);
-          const double f = wt[(h0 + h) * ncol + c];
-          p[h] = f * S0.x; s[h] = -(f * S0.y); t[h] = f * S1.x; r[h] = f * S1.y;
-        }
+      for (int h = 0; h < HN; ++h) {   // all loads in flight: a column without this h reads its first one
+        const bool ok = h0 + h <= mz;
+        const int at = (ok ? h0 + h : 0) * ncol + (on ? c : 0);
+        const double2 *S = (const double2 *)(a.ew_S + ((size_t)lane * EW_H * ncol + at) * 4);
+        const double2 S0 = __ldcg(S), S1 = __ldcg(S + 1);
+        const double f = wt[at];
+        p[h] = ok ? f * S0.x : 0.0; s[h] = ok ? -(f * S0.y) : 0.0;
+        t[h] = ok ? f * S1.x : 0.0; r[h] = ok ? f * S1.y : 0.0;
       }
       __syncthreads();
       if (h0 <= mw)
