@@ -2,8 +2,10 @@
 
     python -m tis_b200.build          (or __graft_entry__.build())
 
-nvcc compiles every .cu under tis_b200/csrc into one shared object; the
-library is loaded from the package directory by tis_b200.abi.load_library.
+nvcc compiles the .cu files under tis_b200/csrc side by side (the variants of
+the split kernel take over a minute each) and links them into one shared
+object; the library is loaded from the package directory by
+tis_b200.abi.load_library.
 """
 from __future__ import annotations
 
@@ -11,13 +13,15 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libtis_b200.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
-         "-Xcompiler", "-fPIC,-ffp-contract=off", "-shared"]
+         "-Xcompiler", "-fPIC,-ffp-contract=off"]
 
 
 def sources():
@@ -43,10 +47,18 @@ def needs_build() -> bool:
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
         return OUT
-    cmd = [nvcc()] + ARCH + FLAGS + ["-o", OUT + ".tmp"] + sources()
-    if verbose:
-        print(" ".join(cmd), file=sys.stderr)
-    subprocess.run(cmd, check=True)
+    exe = nvcc()
+
+    def run(cmd):
+        if verbose:
+            print(" ".join(cmd), file=sys.stderr)
+        subprocess.run(cmd, check=True)
+
+    with tempfile.TemporaryDirectory() as tmp:
+        objs = [os.path.join(tmp, os.path.basename(f) + ".o") for f in sources()]
+        with ThreadPoolExecutor(max(1, os.cpu_count() or 1)) as pool:
+            list(pool.map(lambda fo: run([exe] + ARCH + FLAGS + ["-c", "-o", fo[1], fo[0]]), zip(sources(), objs)))
+        run([exe] + ARCH + ["-shared", "-o", OUT + ".tmp"] + objs)
     os.replace(OUT + ".tmp", OUT)
     return OUT
 

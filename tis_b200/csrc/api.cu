@@ -200,6 +200,12 @@ struct tis_ctx {
   bool bdhi = false;
   int max_nmp = 0;
   long long bd_istep = 0;
+  // pinned staging of the state's and the replicas' copies; null: the caller's
+  // memory is copied directly
+  unsigned char *stage = nullptr;
+  size_t stage_state = 0;             // bytes for three state arrays; the replicas' states and flags follow
+  cudaEvent_t stage_ev = nullptr;     // the last copy out of it
+  bool stage_busy = false;
   DBuf<int> fene_idx, wca_idx, bd_ptr, d_not_spd;
   DBuf<int2> bd_ent;
   DBuf<double> fene_cls, wca_cls, b_hrad;
@@ -1316,6 +1322,17 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     CK(cudaMemset(c->f_ext.p, 0, n3 * 8));
   }
   c->clamp_seen.assign(nlane, 0);
+  {
+    // up to 64 MB of the host's memory stay pinned while the context lives
+    const size_t state = 3 * n3 * sizeof(double), all = state + nlane * (sizeof(LaneState) + sizeof(int));
+    if (all <= ((size_t)64 << 20) && cudaHostAlloc((void **)&c->stage, all, cudaHostAllocDefault) == cudaSuccess) {
+      c->stage_state = state;
+      CK(cudaEventCreateWithFlags(&c->stage_ev, cudaEventDisableTiming));
+    } else {
+      c->stage = nullptr;
+      cudaGetLastError();
+    }
+  }
   *out = c;
   return TIS_OK;
 }
@@ -1345,6 +1362,8 @@ extern "C" int tis_init(const tis_topology *top, const tis_params *par, int32_t 
 extern "C" void tis_destroy(tis_ctx *c) {
   if (!c) return;
   if (c->stream) cudaStreamSynchronize(c->stream);
+  if (c->stage) cudaFreeHost(c->stage);
+  if (c->stage_ev) cudaEventDestroy(c->stage_ev);
   c->d_tops.free(); c->d_lanes.free(); c->d_lstate.free();
   c->b_type.free(); c->b_class.free(); c->b_unit.free();
   c->b_rcmass.free(); c->b_cmass.free(); c->b_fric.free(); c->b_radius.free(); c->b_eps.free(); c->b_charge.free();
@@ -1389,27 +1408,65 @@ extern "C" int tis_nmp(const tis_ctx *c, int32_t irep) {
 }
 
 // ------------------------------------------------------------------- state
+namespace {
+// A blocking copy behind everything queued on the context's stream (set_state
+// and set_step return before their work is done).
+cudaError_t copy_now(tis_ctx *c, void *dst, const void *src, size_t n, cudaMemcpyKind kind) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, n, kind, c->stream);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(c->stream);
+}
+
+__global__ void set_istep_kernel(LaneState *ls, int n, long long istep) {
+  for (int l = threadIdx.x; l < n; l += blockDim.x) ls[l].istep = istep;
+}
+
+// Waits until the staging memory may be overwritten.
+cudaError_t stage_free(tis_ctx *c) {
+  if (!c->stage_busy) return cudaSuccess;
+  c->stage_busy = false;
+  return cudaEventSynchronize(c->stage_ev);
+}
+}  // namespace
+
+// The caller's arrays are copied to pinned memory and queued from there, so
+// that the call does not wait for the device (one copy of the positions; the
+// wrapped ones start as a device copy).
 extern "C" int tis_set_state(tis_ctx *c, const double *xyz, const double *velo, const double *accel) {
   if (!c || !xyz) return TIS_E_ARG;
   size_t n = 3 * (size_t)c->nbead_total * sizeof(double);
-  CK(cudaMemcpyAsync(c->xyz.p, xyz, n, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(c->pxyz.p, xyz, n, cudaMemcpyHostToDevice, c->stream));
-  if (velo) CK(cudaMemcpyAsync(c->velo.p, velo, n, cudaMemcpyHostToDevice, c->stream));
-  else CK(cudaMemsetAsync(c->velo.p, 0, n, c->stream));
-  if (accel) CK(cudaMemcpyAsync(c->accel.p, accel, n, cudaMemcpyHostToDevice, c->stream));
-  else CK(cudaMemsetAsync(c->accel.p, 0, n, c->stream));
+  CK(stage_free(c));
+  auto put = [&](double *dst, const double *src, int part) {
+    if (!src) return cudaMemsetAsync(dst, 0, n, c->stream);
+    if (!c->stage) return cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, c->stream);
+    std::memcpy(c->stage + part * n, src, n);
+    return cudaMemcpyAsync(dst, c->stage + part * n, n, cudaMemcpyHostToDevice, c->stream);
+  };
+  CK(put(c->xyz.p, xyz, 0));
+  CK(put(c->velo.p, velo, 1));
+  CK(put(c->accel.p, accel, 2));
+  if (c->stage) {
+    CK(cudaEventRecord(c->stage_ev, c->stream));
+    c->stage_busy = true;
+  }
+  CK(cudaMemcpyAsync(c->pxyz.p, c->xyz.p, n, cudaMemcpyDeviceToDevice, c->stream));
   CK(cudaMemsetAsync(c->dxyz.p, 0, n, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  if (!c->stage) CK(cudaStreamSynchronize(c->stream));
   return TIS_OK;
 }
 
 extern "C" int tis_get_state(tis_ctx *c, double *xyz, double *velo, double *accel) {
   if (!c) return TIS_E_ARG;
   size_t n = 3 * (size_t)c->nbead_total * sizeof(double);
-  if (xyz) CK(cudaMemcpyAsync(xyz, c->xyz.p, n, cudaMemcpyDeviceToHost, c->stream));
-  if (velo) CK(cudaMemcpyAsync(velo, c->velo.p, n, cudaMemcpyDeviceToHost, c->stream));
-  if (accel) CK(cudaMemcpyAsync(accel, c->accel.p, n, cudaMemcpyDeviceToHost, c->stream));
+  CK(stage_free(c));
+  double *const out[3] = {xyz, velo, accel};
+  const double *const dev[3] = {c->xyz.p, c->velo.p, c->accel.p};
+  for (int k = 0; k < 3; ++k)
+    if (out[k])
+      CK(cudaMemcpyAsync(c->stage ? (void *)(c->stage + k * n) : out[k], dev[k], n, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  if (c->stage)
+    for (int k = 0; k < 3; ++k)
+      if (out[k]) std::memcpy(out[k], c->stage + k * n, n);
   return TIS_OK;
 }
 
@@ -1419,12 +1476,8 @@ KArgs make_args(tis_ctx *c, int mode, int nsteps, int only_lane);
 
 extern "C" int tis_set_step(tis_ctx *c, int64_t istep) {
   if (!c || istep < 0) return TIS_E_ARG;
-  std::vector<LaneState> ls(c->nlane);
-  CK(cudaMemcpyAsync(ls.data(), c->d_lstate.p, ls.size() * sizeof(LaneState), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  for (auto &l : ls) l.istep = istep;
-  CK(cudaMemcpyAsync(c->d_lstate.p, ls.data(), ls.size() * sizeof(LaneState), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  set_istep_kernel<<<1, 256, 0, c->stream>>>(c->d_lstate.p, c->nlane, istep);
+  CK(cudaGetLastError());
   c->bd_istep = istep;
   return TIS_OK;
 }
@@ -1454,7 +1507,7 @@ extern "C" int tis_get_dtrna_status(tis_ctx *c, int32_t irep, int32_t *hb_status
 
 extern "C" int tis_get_pxyz(tis_ctx *c, double *pxyz) {
   if (!c || !pxyz) return TIS_E_ARG;
-  CK(cudaMemcpy(pxyz, c->pxyz.p, 3 * (size_t)c->nbead_total * sizeof(double), cudaMemcpyDeviceToHost));
+  CK(copy_now(c, pxyz, c->pxyz.p, 3 * (size_t)c->nbead_total * sizeof(double), cudaMemcpyDeviceToHost));
   return TIS_OK;
 }
 
@@ -1479,12 +1532,12 @@ extern "C" int tis_set_noise(tis_ctx *c, const double *noise, int32_t nsteps, co
     c->n_unif = 0;
     for (int i = 0; i < c->nlane; ++i) c->lanes[i].unif0 = 0;
   }
-  CK(cudaMemcpy(c->d_lanes.p, c->lanes.data(), c->lanes.size() * sizeof(LaneDesc), cudaMemcpyHostToDevice));
+  CK(copy_now(c, c->d_lanes.p, c->lanes.data(), c->lanes.size() * sizeof(LaneDesc), cudaMemcpyHostToDevice));
   // reset the per-lane uniform positions
   std::vector<LaneState> ls(c->nlane);
-  CK(cudaMemcpy(ls.data(), c->d_lstate.p, ls.size() * sizeof(LaneState), cudaMemcpyDeviceToHost));
+  CK(copy_now(c, ls.data(), c->d_lstate.p, ls.size() * sizeof(LaneState), cudaMemcpyDeviceToHost));
   for (auto &s : ls) { s.unif_pos = 0; s.flags &= ~(LF_UNIF_EXHAUSTED | LF_NOISE_EXHAUSTED); }
-  CK(cudaMemcpy(c->d_lstate.p, ls.data(), ls.size() * sizeof(LaneState), cudaMemcpyHostToDevice));
+  CK(copy_now(c, c->d_lstate.p, ls.data(), ls.size() * sizeof(LaneState), cudaMemcpyHostToDevice));
   return TIS_OK;
 }
 
@@ -1636,8 +1689,19 @@ int launch_lane(tis_ctx *c, const KArgs &a) {
 }
 
 int check_lanes(tis_ctx *c) {
-  std::vector<LaneState> ls(c->nlane);
-  CK(cudaMemcpyAsync(ls.data(), c->d_lstate.p, ls.size() * sizeof(LaneState), cudaMemcpyDeviceToHost, c->stream));
+  const size_t nb = c->nlane * sizeof(LaneState);
+  std::vector<LaneState> own;
+  std::vector<int> own_spd;
+  LaneState *ls = (LaneState *)(c->stage + c->stage_state);
+  int *ns = (int *)(c->stage + c->stage_state + nb);
+  if (!c->stage) {
+    own.resize(c->nlane);
+    own_spd.resize(c->nlane);
+    ls = own.data();
+    ns = own_spd.data();
+  }
+  CK(cudaMemcpyAsync(ls, c->d_lstate.p, nb, cudaMemcpyDeviceToHost, c->stream));
+  if (c->bdhi) CK(cudaMemcpyAsync(ns, c->d_not_spd.p, c->nlane * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   long long clamps = 0;
   int code = TIS_OK;
@@ -1658,8 +1722,6 @@ int check_lanes(tis_ctx *c) {
     c->clamp_seen[i] = ls[i].nclamp;
   }
   if (c->bdhi) {
-    std::vector<int> ns(c->nlane);
-    CK(cudaMemcpy(ns.data(), c->d_not_spd.p, ns.size() * sizeof(int), cudaMemcpyDeviceToHost));
     for (int i = 0; i < c->nlane; ++i) {
       if (ns[i] & 1) {
         c->not_spd = 1;
@@ -1693,10 +1755,10 @@ int fetch_masks(tis_ctx *c, int lane, std::vector<uint32_t> &m, std::vector<uint
   const LaneDesc &L = c->lanes[lane];
   const int N = c->lane_nmp[lane], W = (N + 31) / 32;
   m.resize(2 * (size_t)N * W);
-  CK(cudaMemcpy(m.data(), c->mask.p + L.mask0, m.size() * 4, cudaMemcpyDeviceToHost));
+  CK(copy_now(c, m.data(), c->mask.p + L.mask0, m.size() * 4, cudaMemcpyDeviceToHost));
   if (c->par.i_periodic == 1) {
     mir.resize((size_t)N * N);
-    CK(cudaMemcpy(mir.data(), c->mirror.p + L.mirror0, mir.size(), cudaMemcpyDeviceToHost));
+    CK(copy_now(c, mir.data(), c->mirror.p + L.mirror0, mir.size(), cudaMemcpyDeviceToHost));
   }
   return TIS_OK;
 }
@@ -1738,17 +1800,17 @@ extern "C" int tis_get_ele_list(tis_ctx *c, int32_t irep, int32_t *iele2mp, doub
   const uint32_t *mele = m.data() + (size_t)N * W;
   std::vector<double> q(N);
   std::vector<int8_t> typ(N);
-  CK(cudaMemcpy(q.data(), c->b_charge.p + T.bead0, N * sizeof(double), cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(typ.data(), c->b_type.p + T.bead0, N, cudaMemcpyDeviceToHost));
+  CK(copy_now(c, q.data(), c->b_charge.p + T.bead0, N * sizeof(double), cudaMemcpyDeviceToHost));
+  CK(copy_now(c, typ.data(), c->b_type.p + T.bead0, N, cudaMemcpyDeviceToHost));
   std::vector<LaneState> ls(1);
-  CK(cudaMemcpy(ls.data(), c->d_lstate.p + lane, sizeof(LaneState), cudaMemcpyDeviceToHost));
+  CK(copy_now(c, ls.data(), c->d_lstate.p + lane, sizeof(LaneState), cudaMemcpyDeviceToHost));
   double coefT = 0.0;
-  CK(cudaMemcpy(&coefT, c->lab_coef.p + ls[0].label, sizeof(double), cudaMemcpyDeviceToHost));
+  CK(copy_now(c, &coefT, c->lab_coef.p + ls[0].label, sizeof(double), cudaMemcpyDeviceToHost));
   if (c->b_qkind.p) {   // i_charge = 1: the label's phosphate charge
     std::vector<uint8_t> qk(N);
     double zp = 0.0;
-    CK(cudaMemcpy(qk.data(), c->b_qkind.p + T.bead0, N, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(&zp, c->lab_zp.p + ls[0].label, sizeof(double), cudaMemcpyDeviceToHost));
+    CK(copy_now(c, qk.data(), c->b_qkind.p + T.bead0, N, cudaMemcpyDeviceToHost));
+    CK(copy_now(c, &zp, c->lab_zp.p + ls[0].label, sizeof(double), cudaMemcpyDeviceToHost));
     for (int i = 0; i < N; ++i)
       if (qk[i]) q[i] = -zp;
   }
@@ -1779,7 +1841,7 @@ extern "C" int tis_get_hb_list(tis_ctx *c, int32_t irep, int32_t *ineigh2hb, int
   const LaneDesc &L = c->lanes[irep - 1];
   const TopDesc &T = c->tops[L.top];
   std::vector<uint8_t> f(std::max(T.nhb, 1));
-  if (T.nhb) CK(cudaMemcpy(f.data(), c->hb_flag.p + L.hb0, T.nhb, cudaMemcpyDeviceToHost));
+  if (T.nhb) CK(copy_now(c, f.data(), c->hb_flag.p + L.hb0, T.nhb, cudaMemcpyDeviceToHost));
   int k = 0;
   for (int h = 0; h < T.nhb; ++h)
     if (f[h] & 1) {
@@ -2320,7 +2382,7 @@ extern "C" int tis_rex_exchange_all(tis_ctx *c, const double *replica_energy_all
 extern "C" int tis_status(tis_ctx *c, tis_status_t *st) {
   if (!c || !st) return TIS_E_ARG;
   std::vector<LaneState> ls(c->nlane);
-  CK(cudaMemcpy(ls.data(), c->d_lstate.p, ls.size() * sizeof(LaneState), cudaMemcpyDeviceToHost));
+  CK(copy_now(c, ls.data(), c->d_lstate.p, ls.size() * sizeof(LaneState), cudaMemcpyDeviceToHost));
   std::memset(st, 0, sizeof(*st));
   st->step = ls[0].istep;
   for (int i = 0; i < c->nlane; ++i) {
@@ -2380,11 +2442,11 @@ extern "C" int tis_get_hydro_tensors(tis_ctx *c, int32_t irep, double *diffuse, 
     if (which == 0 && c->bd_D32.p) {
       const size_t ld = (n + 3) / 4 * 4;
       fbuf.resize(n * ld);
-      CK(cudaMemcpy(fbuf.data(), c->bd_D32.p + L.bd32, n * ld * sizeof(float), cudaMemcpyDeviceToHost));
+      CK(copy_now(c, fbuf.data(), c->bd_D32.p + L.bd32, n * ld * sizeof(float), cudaMemcpyDeviceToHost));
       for (size_t r = 0; r < n; ++r)
         for (size_t col = 0; col < n; ++col) buf[r * n + col] = fbuf[r * ld + col];
     } else {
-      CK(cudaMemcpy(buf.data(), (which == 0 ? c->bd_D.p : c->bd_L.p) + L.bd0, n * n * sizeof(double),
+      CK(copy_now(c, buf.data(), (which == 0 ? c->bd_D.p : c->bd_L.p) + L.bd0, n * n * sizeof(double),
                     cudaMemcpyDeviceToHost));
     }
     for (size_t r = 0; r < n; ++r)

@@ -208,11 +208,11 @@ __device__ __forceinline__ void load_diag_tile(const double *Lm, int n, int td, 
 // row of the matrix below the block or a row of the identity above.
 // In one launch of its own, cold (ncu): 36.8 us when one warp factored 16
 // columns for all rows, pivots and columns passed by shuffles, and the inverse
-// followed in 64 more steps; FD_NOW us this way.
+// followed in 64 more steps; 11.6 us this way.
 //
 // The results are written at the end: with the idle warps writing a block's
-// while the next is factored, all phases of both took longer (17.1 against
-// FD_CYC thousand cycles a tile).
+// while the next is factored, a block took 900 + 1050 cycles (factor, update)
+// instead of 800 + 690.
 //
 // A pivot <= 0 is replaced by 1 (no NaN spreads) and flags the lane.  Stores
 // L_tt (zero above the diagonal; FP32 copy for mixed precision) and, when a
@@ -770,7 +770,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) chol_update_tc_kernel(KArgs a, c
       const int tj = tj0 + t, col = tj * CT + h * 32 + lid;
       // the tile's FP64 elements while its products are on their way, and the
       // next tile's lines towards L2: a tile's time was that of its loads,
-      // issued after the wait (4.2 us a tile; now EP_NOW)
+      // issued after the wait (4.2 us a tile of the widest launch; now 3.6)
       double old[32];
 #pragma unroll
       for (int rr = 0; rr < 32; ++rr) {
@@ -1248,8 +1248,10 @@ __global__ void __launch_bounds__(256) bd_force_kernel(KArgs a) {
 // kug[i]: column tiles per item of launch i.  UG of them share one load of the
 // 128 rows' operands, but the chip has 148 CTAs and a launch lasts as long as
 // its last item: the size with the shortest time at U_ITEM us per item, U_TILE
-// per column tile and U_DIAG for the diagonal tile (measured with 8 tiles per
-// item: UG_NOW).
+// per column tile and U_DIAG for the diagonal tile.  With 8 tiles per item
+// always, the last ten wide launches of 32 chains of 100 to 1,000 beads took
+// 40 us each, with 1 to 4 they take 22 (a launch of the diagonal tile alone:
+// 20).
 void bd_update_items(const std::vector<int> &lane_T, std::vector<int> &items, std::vector<int> &koff,
                      std::vector<int> &kug) {
   constexpr double U_ITEM = 5.0, U_TILE = 3.5, U_DIAG = 10.0;
@@ -1301,7 +1303,10 @@ void bd_update_items(const std::vector<int> &lane_T, std::vector<int> &items, st
 
 // Panel launch: 64 rows per CTA, or 16 while the 64-row CTAs would leave SMs
 // idle (a panel is FP64-bound, so splitting the rows divides its time, but
-// every CTA reads U again).
+// every CTA reads U again); the FP64 update's quarter tiles follow the same
+// line.  A step with refresh, small against large blocks: 150 beads 167 / 177
+// us, 8 x 150 186 / 193, 16 x 150 226 / 227, 32 x 150 301 / 302, 400 beads 405 /
+// 418; mixed 400 beads 500 / 531, 16 x 400 794 / 805.
 cudaError_t panel_launch(cudaStream_t st, const KArgs &a, int m) {
   if ((long long)m * a.nlane <= BD_SMS)
     chol_panel_kernel<16><<<dim3(4 * m, a.nlane), 256, (16 + CT) * CTP * sizeof(double), st>>>(a);
@@ -1389,7 +1394,9 @@ cudaError_t bd_step_launch(cudaStream_t st, const KArgs &a, int max_nmp) {
     if (e != cudaSuccess) return e;
     refine_trsv_kernel<<<a.nlane, TRSV_THREADS, sm, st>>>(a);
   }
-  // four rows per warp once that still gives every SM two CTAs (64 rows)
+  // four rows per warp once that still gives every SM two CTAs (64 rows): 32
+  // chains of 100 to 1,000 beads 110 us against 187 with one row; below, the
+  // rows of one warp would queue up behind one another on idle SMs
   if ((long long)3 * max_nmp * a.nlane >= 64LL * BD_SMS)
     bd_update_kernel<4><<<dim3((3 * max_nmp + 31) / 32, a.nlane), 256, 0, st>>>(a);
   else
