@@ -20,7 +20,7 @@ constexpr int MAX_THREADS = 1024;
 constexpr int N_ETYPE = 25;   // E_TYPE%MAX
 constexpr int CHMAX = 1024;   // electrostatic row chunks per lane (at least one per charged bead)
 constexpr int EW_H = 12;      // Ewald: hz = 0 .. 11 of a column (hx, hy) of reciprocal vectors
-enum { EWS_READY = 0, EWS_BARRIER = 32, EWS_DONE = 64, EWS_ABORT = 96, EWS_WORDS = 128 };   // words of ew_sync
+enum { EWS_READY = 0, EWS_BARRIER = 32, EWS_DONE = 64, EWS_ABORT = 96, EWS_ARRIVED = 128, EWS_WORDS = 160 };   // words of ew_sync
 constexpr int EW_COLS = 192;  // columns of the half space at most (189 for |h| <= 11)
 // HI_TENSOR (const_index.F90:39-45)
 constexpr int TIS_HI_RPY_DEV = 1, TIS_HI_RPY_OVER_DEV = 2, TIS_HI_ERMAK_OVER_DEV = 3, TIS_HI_ZUK_RPY_DEV = 4;

@@ -262,6 +262,8 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   typedef typename V4<Real>::T V;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if constexpr (PER)
+    if (a.ew_nwork && threadIdx.x == 0) ew_signal(a, EWS_ARRIVED);
+  if constexpr (PER)
     if (a.ew_nwork && blockIdx.x >= gridDim.x - (unsigned)a.ew_nwork) {
       ewald_worker<NT>(a, smem_raw);
       return;
