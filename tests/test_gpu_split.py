@@ -155,3 +155,22 @@ def test_near_lists_follow_beads_of_other_ctas(tis_lib, ctas, precision):
         out.append(eng.get_state()[0])
         eng.close()
     assert np.abs(out[0] - out[1]).max() < {0: 1e-6, 1: 1e-2}[precision]
+
+
+@pytest.mark.parametrize("every,pair", [(0, False), (10, True), (43, True), (44, False)])
+def test_short_rebuild_cadence_keeps_the_two_cta_kernel(tis_lib, every, pair):
+    """64 replicas on two CTAs each: the split, or, with lists rebuilt often,
+    the kernel whose rebuild is cheaper; both against one CTA per replica."""
+    s = synth.set_friction(synth.dt15_chain(76, 5), 0.5)
+    par = synth.dt15_params(ionic_strength=0.15, n_step_neighbor=every, precision=1)
+    out = []
+    for extra in ({}, {"launch_ctas": 1}):
+        eng = Engine([s], dict(par, **extra), list(np.geomspace(280.0, 400.0, 64)))
+        if not extra:
+            assert eng.status()["ctas_per_lane"] == (2 if pair else 1)
+        eng.set_state(np.tile(s["xyz"], (64, 1)))
+        eng.time_integral_pre()
+        eng.step(12)
+        out.append(eng.get_state()[0])
+        eng.close()
+    assert np.abs(out[0] - out[1]).max() < POS_TOL[1]

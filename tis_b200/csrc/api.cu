@@ -1061,6 +1061,10 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
           const double x = total(o.nr, o.least, clusters);
           if (x < least_time) { least_time = x; best = o.nr; best_least = o.least; }
         }
+        // Lists rebuilt every few steps: the two-CTA kernel rebuilds in 14 us
+        // (64 chains of 227 beads; each pair tested once), the split in 36,
+        // and a step takes 10.75 against 10.25 us: even at one in 44
+        if (best == 2 && !best_least && c->pair && p.n_step_neighbor > 0 && p.n_step_neighbor < 44) best = 0;
       }
       c->nsplit = 0;
       if (best) {
