@@ -13,7 +13,7 @@ whole job (all ranks).  Inputs are synthetic (seeded random-walk chains).
 Other fields: e2e (same metric through the C-ABI with host buffers, state
 copied in from pinned host memory and out every step), the plain FP64
 single-system path (65-bead chain, one replica) as the denominator of the
-batched/plain ratio, the roofline of the dominant kernel (lane_kernel<float>)
+batched/plain ratio, the roofline of the dominant kernel (split_kernel<float>)
 and the CPU restatement timed on the host cores.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
@@ -318,10 +318,10 @@ def aggregate_rate(units_per_rank, world, total_ms):
 
 
 def profiled_traffic():
-    """DRAM bytes per lane_kernel launch at the bench size, from the committed
+    """DRAM bytes per split_kernel launch at the bench size, from the committed
     ncu summary (dram__bytes_read.sum + dram__bytes_write.sum), or None."""
     import re
-    path = os.path.join(ROOT, "profiles", "lane_kernel_c3_launches.md")
+    path = os.path.join(ROOT, "profiles", "split_kernel_c3_launches.md")
     try:
         m = re.search(r"traffic per launch \| ([\d,]+) B", open(path).read())
         return int(m.group(1).replace(",", "")) if m else None
@@ -579,11 +579,11 @@ def run_ours(args, rank, world, local_rank):
                          "frac": achieved / peak,
                          "traffic": profiled_traffic() if (args.workload == "c3" and period_len == PERIOD) else None,
                          "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch "
-                                            "(profiles/lane_kernel_c3_launches.md)") if args.workload == "c3"
+                                            "(profiles/split_kernel_c3_launches.md)") if args.workload == "c3"
                                            else "not captured for this workload",
                          "kernel": ("Brownian-HI step: bd_update_kernel matrix-vector products + Cholesky refresh "
                                     "(chol_update_tc_kernel dominant)" if args.workload == "c5"
-                                    else "lane_kernel<float>"), "peak_source": src,
+                                    else "split_kernel<float>"), "peak_source": src,
                          "bytes_per_replica_step": bytes_per_rs,
                          "note": ("time-averaged over whole refresh periods; achieved counts the algorithmic "
                                   "HBM bytes of the step and of the amortised refresh" if args.workload == "c5" else
