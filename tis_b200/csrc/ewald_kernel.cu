@@ -25,6 +25,11 @@
 // (four launches; 8.8 + 9.8 + 3.2 + 12.7 us for 165 charges): ten times the
 // FP64 work of the column form and four dependent launches.
 //
+// Steps of lanes split over clusters take these sums inside their own launch
+// where enough CTAs are left (split_ewald.cuh: 62 -> 20 us a step for 51
+// nucleotides with 590 ions); these kernels serve single-point calls, one-CTA
+// lanes, batches that fill the chip and replicas with their own step counts.
+//
 // All sums run in a fixed order, so the results do not depend on scheduling.
 #include <algorithm>
 

@@ -3,8 +3,8 @@
 // A step of a lane is a short chain of dependent work: on one CTA a 1,199-bead
 // lane keeps one of 148 SMs busy for 121 us a step, and what bounds it is that
 // SM's issue rate and the latency of its longest items, not memory.  Split
-// over 16 CTAs the same step takes 18.6 us; 599 beads in FP64 82 -> 12.1 us,
-// 227 beads mixed 10.3 -> 6.3 us (8 CTAs), 65 beads FP64 11.2 -> 6.5 us (B200,
+// over 16 CTAs the same step takes 12.2 us; 599 beads in FP64 82 -> 9.5 us,
+// 227 beads mixed 10.3 -> 5.8 us (8 CTAs), 65 beads FP64 11.2 -> 6.2 us (B200,
 // event time of the step kernel).  Every mode of the lane kernel (KM_*) runs
 // here, for both precisions, with or without a periodic box.
 //
