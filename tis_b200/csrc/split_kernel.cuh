@@ -96,6 +96,7 @@ struct SplitSmem {
   float *L3;               // mixed: pxyz - A4, so that A4 + L3 carries pxyz to ~2^-48
   Real *RE;                // exv radius, sqrt(eps)
   uint32_t *tcu;           // type | class << 8 | unit << 16
+  int *box;                // periodic: the cell of a bead, (X - P) / L, 10 bits a dimension; changed by list builds only
 };
 
 // pxyz of any bead from the copies that every step refreshes
@@ -124,6 +125,14 @@ __device__ __forceinline__ void split_pos(const SplitSmem<Real> &s, int i, doubl
     s.L3[3 * i] = (float)(x - (double)hx); s.L3[3 * i + 1] = (float)(y - (double)hy);
     s.L3[3 * i + 2] = (float)(z - (double)hz);
   }
+}
+
+// cells packed modulo 1024; component d of the difference of two of them, -512 .. 511
+__device__ __forceinline__ int cell_pack(double x, double y, double z) {
+  return ((int)x & 1023) | ((int)y & 1023) << 10 | ((int)z & 1023) << 20;
+}
+__device__ __forceinline__ int cell_diff(int p, int q, int d) {
+  return (int)((unsigned)((q >> 10 * d) - (p >> 10 * d)) << 22) >> 22;
 }
 
 // image of the pair (i, j) fixed at the last rebuild, as x_j - x_i sees it
@@ -298,6 +307,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   s.L3 = (float *)(sm + pl.L3);
   s.RE = (Real *)(sm + pl.RE);
   s.tcu = (uint32_t *)(sm + pl.tcu);
+  s.box = (int *)(sm + pl.box);
   auto typ = [&](int i) SPLIT_INL { return (int)(s.tcu[i] & 0xff); };
   auto cls = [&](int i) SPLIT_INL { return (int)(s.tcu[i] >> 8 & 0xff); };
   auto unit = [&](int i) SPLIT_INL { return (int)(s.tcu[i] >> 16); };
@@ -381,7 +391,11 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     if (tid == 0) { V far; far.x = far.y = far.z = (Real)1.0e6; far.w = 0; s.A4[np] = far; }
     __pipeline_wait_prior(0);
     __syncthreads();
-    for (int i = tid; i < N; i += NT) split_pos<Real>(s, i, s.PX[i], s.PY[i], s.PZ[i]);
+    for (int i = tid; i < N; i += NT) {
+      split_pos<Real>(s, i, s.PX[i], s.PY[i], s.PZ[i]);
+      if (PER) s.box[i] = cell_pack(rint((s.X[i] - s.PX[i]) / a.psize[0]), rint((s.Y[i] - s.PY[i]) / a.psize[1]),
+                                    rint((s.Z[i] - s.PZ[i]) / a.psize[2]));
+    }
   }
   cl.sync();   // loaded; and every CTA runs before any distributed access
 
@@ -400,32 +414,49 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
 
   const bool ewald = a.i_ele == 2, coul = a.i_ele == 3;
   const int LQ = split_row_lanes(NQ, ewald), RW = 32 / LQ;
-  // x_j - x_i of the bonded terms in W (nearest image when periodic: the
-  // chain's own, as its beads are close); in FP32 from the hi and lo parts,
-  // rounded once
-  auto rvec = [&](auto w, int i, int j) SPLIT_INL {
+  // x_j - x_i of the bonded terms in W, in FP32 from the hi and lo parts,
+  // rounded once.  Periodic: of the unwrapped positions (bonds, angles,
+  // stacks), i.e. of the wrapped ones and the beads' cells, or the nearest
+  // image (hydrogen bonds).  Across the box the two coordinates are ~L apart,
+  // so the rounding error of their difference is kept (TwoSum)
+  auto bvec = [&](auto nearest, auto w, int i, int j) SPLIT_INL {
     typedef decltype(w) Wt;
+    constexpr bool NEAREST = decltype(nearest)::value;
     const V p = s.A4[i], q = s.A4[j];
+    int ci = 0, cj = 0;
+    if (PER && !NEAREST) { ci = s.box[i]; cj = s.box[j]; }
     if constexpr (sizeof(Wt) == 4) {
       const float *l = s.L3 + 3 * i, *m = s.L3 + 3 * j;
       auto d1 = [&](float x, float y, float lx, float ly, int d) SPLIT_INL {
         const float t = y - x, bb = t - y, e = (y - (t - bb)) + (-x - bb) + (ly - lx);
         if (!PER) return t + e;
-        const float h = (float)a.psizeh[d], k = t > h ? -1.0f : (t < -h ? 1.0f : 0.0f);
+        float k;
+        if (NEAREST) { const float h = (float)a.psizeh[d]; k = t > h ? -1.0f : (t < -h ? 1.0f : 0.0f); }
+        else k = (float)cell_diff(ci, cj, d);
         const float Lh = (float)a.psize[d], Ll = (float)(a.psize[d] - (double)Lh);
         return fmaf(k, Lh, t) + fmaf(k, Ll, e);
       };
       return R3<Wt>{d1(p.x, q.x, l[0], m[0], 0), d1(p.y, q.y, l[1], m[1], 1), d1(p.z, q.z, l[2], m[2], 2)};
     } else {
-      double x = (double)q.x - (double)p.x, y = (double)q.y - (double)p.y, z = (double)q.z - (double)p.z;
+      double px = (double)p.x, py = (double)p.y, pz = (double)p.z, qx = (double)q.x, qy = (double)q.y, qz = (double)q.z;
       if constexpr (sizeof(Real) == 4) {
         const float *l = s.L3 + 3 * i, *m = s.L3 + 3 * j;
-        x += (double)m[0] - (double)l[0]; y += (double)m[1] - (double)l[1]; z += (double)m[2] - (double)l[2];
+        px += (double)l[0]; py += (double)l[1]; pz += (double)l[2];
+        qx += (double)m[0]; qy += (double)m[1]; qz += (double)m[2];
       }
+      if (PER && !NEAREST) {
+        auto d1 = [&](double x, double y, int d) SPLIT_INL {
+          const double t = y - x, bb = t - y, e = (y - (t - bb)) + (-x - bb);
+          return fma((double)cell_diff(ci, cj, d), a.psize[d], t) + e;
+        };
+        return R3<Wt>{d1(px, qx, 0), d1(py, qy, 1), d1(pz, qz, 2)};
+      }
+      double x = qx - px, y = qy - py, z = qz - pz;
       if (PER) { pb1(x, a.psize[0], a.psizeh[0]); pb1(y, a.psize[1], a.psizeh[1]); pb1(z, a.psize[2], a.psizeh[2]); }
       return R3<Wt>{x, y, z};
     }
   };
+  auto rvec = [&](auto w, int i, int j) SPLIT_INL { return bvec(std::false_type(), w, i, j); };
   // partner lists of the charged rows from their bit rows (with the image of
   // each pair when periodic): lane l expands words l, l + 32, ...
   // (called by the whole CTA; misc[MISC_ELIST]: they fit)
@@ -503,6 +534,13 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     if (PER) {
       for (int i = tid; i < N; i += NT) {
         const double x = wrap1(s.PX[i], a.psize[0]), y = wrap1(s.PY[i], a.psize[1]), z = wrap1(s.PZ[i], a.psize[2]);
+        const int moved = cell_pack(rint((s.PX[i] - x) / a.psize[0]), rint((s.PY[i] - y) / a.psize[1]),
+                                    rint((s.PZ[i] - z) / a.psize[2]));
+        if (moved) {
+          const int c = s.box[i];
+          s.box[i] = ((c & 1023) + (moved & 1023) & 1023) | ((c >> 10 & 1023) + (moved >> 10 & 1023) & 1023) << 10 |
+                     ((c >> 20 & 1023) + (moved >> 20 & 1023) & 1023) << 20;
+        }
         s.PX[i] = x; s.PY[i] = y; s.PZ[i] = z;
         s.QX[i] = x; s.QY[i] = y; s.QZ[i] = z;
         split_pos<Real>(s, i, x, y, z);
@@ -1045,14 +1083,14 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
         const int m[6] = {(int)(ix[0] & 0xffff), (int)(ix[0] >> 16), (int)(ix[1] & 0xffff), (int)(ix[1] >> 16),
                           (int)(ix[2] & 0xffff), (int)(ix[2] >> 16)};
         const uint8_t f = k0 < nh ? hbf[k] : (uint8_t)0;
-        const R3<Real> v12 = rvec(Real(), m[1], m[0]);
+        const R3<Real> v12 = bvec(std::true_type(), Real(), m[1], m[0]);
         Real a12, r12;
         length(sdot(v12, v12), a12, r12);
         const Real d12 = a12 - cf[0];
         const bool act = (f & 1) && !(fabs((double)d12) > a.hb_cutoff_dist);
         Real e = 0;
         if (__any_sync(0xffffffffu, act)) {
-          auto dv = [&](int p, int q) SPLIT_INL { return rvec(Real(), q, p); };   // x_p - x_q
+          auto dv = [&](int p, int q) SPLIT_INL { return bvec(std::true_type(), Real(), q, p); };   // x_p - x_q
           const Real MAXC = (Real)a.max_abscos;
           const R3<Real> v13 = dv(m[0], m[2]), v42 = dv(m[3], m[1]);
           const R3<Real> ve = dv(role == 1 ? m[4] : m[3], role == 1 ? m[2] : m[5]);   // v53 or v46

@@ -56,6 +56,7 @@ inline SplitPlan split_plan(const TopDesc &T, int nq, int row, int nr, bool peri
   p.X = take(24 * n);
   p.P = periodic ? take(24 * n) : p.X;
   p.Q = periodic ? take(24 * n) : p.X;
+  p.box = periodic ? take(4 * n) : 0;     // periodic cell of each bead
   p.A4 = take(4 * R * (n + 4));           // and a bead far away without charge (entry np)
   p.L3 = real == 4 ? take(12 * n) : 0;
   p.V = take((skin ? 72 : 48) * o);       // v, a, [dxyz]
