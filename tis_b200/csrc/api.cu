@@ -1026,7 +1026,8 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
           const double w = mixed ? 0.010 * n + 1.1e-4 * n * n : 0.02 * n + 1.6e-4 * n * n;
           return (nr == 16 ? 7.0 : 6.0) + n / 300.0 + w / nr;
         };
-        const double scale = lad ? (double)lad->nall / nlane : 1.0, sms = std::max(nsm, 1);
+        const int nall = lad ? lad->nall : nlane, sms = std::max(nsm, 1);
+        const double scale = (double)nall / nlane;
         auto total = [&](int nr, int least, int places) {   // nr 0: every lane on one CTA
           double work = 0.0, longest = 0.0;
           int n_split = 0;
@@ -1038,7 +1039,8 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
             longest = std::max(longest, t);
             n_split += sp;
           }
-          if (c->ntop == 1) return longest * std::ceil(nlane * scale / (nr ? places : sms));   // equal lanes: whole rounds
+          const int room = nr ? places : sms;
+          if (c->ntop == 1) return longest * ((nall + room - 1) / room);   // equal lanes: whole rounds
           const double turns = n_split > places || nlane > sms ? 0.25 * longest : 0.0;
           return std::max(longest, std::max(work * scale / sms, n_split ? work * n_split / nlane / (places * nr) : 0.0) + turns);
         };
@@ -1312,11 +1314,14 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     CK(c->ew_S.alloc((size_t)nlane * EW_H * c->ew_ncol * 4));
     // every lane split and SMs left over: the reciprocal sum runs beside the
     // lanes in one launch per call.  It takes the chip's rest, so a batch
-    // that leaves less than about a third of it keeps the separate kernels
+    // that leaves less than about a third of it keeps the separate kernels.
+    // The two add in different orders, so a ladder context decides for the
+    // whole ladder
     if (c->nsplit && c->n_split == nlane && c->nq_max > 0) {
-      const int left = split_clusters(c->nsplit, p.precision == TIS_PREC_MIXED, true) - nlane;
-      if (left * c->nsplit >= 48 && ew_smem(nlane, c->nq_max, c->ew_ncol).total <= 227 * 1024) {
-        c->ew_work = left * c->nsplit;
+      const int nall = lad ? lad->nall : nlane;
+      const int clusters = split_clusters(c->nsplit, p.precision == TIS_PREC_MIXED, true);
+      if ((clusters - nall) * c->nsplit >= 48 && ew_smem(nall, c->nq_max, c->ew_ncol).total <= 227 * 1024) {
+        c->ew_work = (clusters - nlane) * c->nsplit;
         c->ew_nb = (int)(n3 / 3);
         CK(c->ew_sync.alloc(EWS_WORDS));
         CK(c->ew_E.alloc((size_t)EW_H * n3));
