@@ -195,7 +195,9 @@ typedef struct tis_params {
                                       the library also chooses by itself (2 to 16) where that is faster */
   int32_t launch_noise_sweep;      /* two CTAs: 1 draws the noise in the bonded sweep, 2 in the update */
   int32_t launch_order;            /* 1: replicas launched in context order, 2: largest first */
-  const char *launch_table;        /* NULL: tuned_launch.tsv next to the library */
+  const char *launch_table;        /* NULL: tuned_launch.tsv next to the library, whose rows set the launch of
+                                      replicas that are not split; the rows of a table named here are
+                                      followed as they are (0 CTAs in a row: the library's choice) */
   int32_t launch_sweep;            /* bonded sweep of one CTA per replica: 1 item chunks dealt to the warps
                                       in turn, 2 warps take chunks from a shared counter, longest kinds
                                       first, 3 a longest-first deal made once per launch (two CTAs: 1) */

@@ -3,8 +3,10 @@
 For a workload (topologies, tis_params, temperatures) it times tis_step on
 the GPU for every valid configuration of
 
+* the library's own choice (a row of zeros);
 * CTAs per replica: 1, or 2 (a thread-block cluster; mixed precision, no
-  periodic box, no Ewald, >= 64 beads);
+  periodic box, no Ewald, >= 64 beads), or 4, 8 or 16 that split the replica
+  (at least 4 beads each);
 * threads per CTA: 128, 256, 512, and 1024 for one mixed-precision CTA
   (the cluster kernel runs 512);
 * threads per bead in the force gather: the per-replica rule, 1, 2, 4, 8;
@@ -56,7 +58,8 @@ def candidates(systems, par, nrep):
     pair_ok = (mixed and not par.get("i_periodic", 0) and par.get("i_ele", 0) != 2
                and min(int(s["nmp"]) for s in systems) >= 64)
     uneven = len({int(s["nmp"]) for s in systems}) > 1
-    out = []
+    zero = dict(launch_ctas=0, launch_threads=0, launch_group=0, launch_noise_sweep=0, launch_order=0, launch_sweep=0)
+    out = [zero] + [dict(zero, launch_ctas=c) for c in (4, 8, 16) if min(int(s["nmp"]) for s in systems) >= 4 * c]
     for ctas in ([1, 2] if pair_ok else [1]):
         threads = [512] if ctas == 2 else ([128, 256, 512] + ([1024] if mixed else []))
         sweeps = [1, 2] if ctas == 2 else [1]
@@ -71,7 +74,8 @@ def time_config(systems, par, temps, nrep, cfg, steps, reps):
     """Median replica-steps/s of `reps` launches of `steps` MD steps."""
     from .engine import Engine, TisError
     try:
-        eng = Engine(systems, dict(par, **cfg), temps, nrep=nrep)
+        # an empty table name: the row that is being measured, not one already there, sets the launch
+        eng = Engine(systems, dict(par, launch_table="", **cfg), temps, nrep=nrep)
     except TisError:
         return None
     try:

@@ -929,6 +929,7 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     if (p.launch_noise_sweep) { cfg.noise_sweep = p.launch_noise_sweep; source = 2; }
     if (p.launch_order) { cfg.order = p.launch_order; source = 2; }
     if (p.launch_sweep) { cfg.sweep = p.launch_sweep; source = 2; }
+    const int asked = cfg.ctas;
     if (cfg.ctas == 0) cfg.ctas = (pair_ok && nsm > 0 && 2 * nlane <= nsm) ? 2 : 1;
     if (cfg.ctas == 2 && !pair_ok) cfg.ctas = 1;
     if (cfg.ctas == 2) cfg.threads = 512;   // the cluster kernel runs 512 threads per CTA
@@ -957,9 +958,11 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     c->sweep = cfg.sweep;
     c->launch_source = source;
     c->smem2 = c->pair ? smem2 : 0;
-    // Lanes split over clusters of nr CTAs (split_kernel), unless the caller
-    // or the environment chose a configuration; launch_ctas 4, 8 or 16 asks
-    // for it.  least: the fewest beads of a lane that is split.
+    // Lanes split over clusters of nr CTAs (split_kernel), unless the caller,
+    // the environment or a row (with its number of CTAs) of a table that the
+    // caller names chose a configuration; 4, 8 or 16 CTAs ask for it.  Rows of
+    // the library's own table set the launch of the lanes that are not split.
+    // least: the fewest beads of a lane that is split.
     auto try_split = [&](int nr, int least, bool lists, int &clusters) {
       TopDesc mx{};   // the largest counts
       int mq = 0;
@@ -1007,10 +1010,10 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     };
     if (!c->bdhi && maxN < (periodic ? 2044 : 65532)) {
       int clusters = 0, best = 0, best_least = 0;
-      if (p.launch_ctas >= 4) {
-        for (int nr = std::min(p.launch_ctas, SPLIT_MAX); nr >= 2 && !best; nr /= 2)
+      if (asked >= 4) {
+        for (int nr = std::min(asked, SPLIT_MAX); nr >= 2 && !best; nr /= 2)
           if (try_split(nr, 0, false, clusters)) best = nr;
-      } else if (source != 2) {
+      } else if (!source || (source == 1 && !(p.launch_table && asked))) {
         // The split with the least estimated time of a step of the whole
         // context: nr CTAs for every lane, or for the lanes of a batch that
         // have at least `least` beads, the others on one CTA beside them.
