@@ -216,8 +216,9 @@ typedef struct tis_status_t {
   int32_t exv_pairs_max;           /* largest exv half list among replicas */
   int32_t ele_pairs_max;           /* largest ele half list among replicas */
   int32_t ctas_per_lane;           /* 2: pairs of CTAs that each hold the whole replica (launch_ctas 2);
-                                      1: one CTA, or replicas split over larger clusters */
-  int32_t threads_per_cta;         /* the launch configuration in use (see tis_params.launch_*) */
+                                      1: one CTA, or replicas split over clusters (see tis_get_launch) */
+  int32_t threads_per_cta;         /* the launch configuration in use (see tis_params.launch_*): of the
+                                      split replicas where every replica is split, else of the others */
   int32_t group;                   /* threads per bead in the force gather, 0: per-replica rule */
   int32_t noise_sweep;
   int32_t lane_order;
@@ -377,6 +378,14 @@ int tis_get_random_number(tis_ctx *ctx, int64_t istep, int32_t nstep, double *r_
  * one (-1: none): the information of the reference's neighbour-list record
  * (outfile%neigh, src/time_integral.F90:76-84).  Either pointer may be NULL. */
 int tis_get_rebuild_info(tis_ctx *ctx, int32_t irep, int64_t *n_rebuild, int64_t *last_step);
+
+/* What the steps of replica irep run on: layout 1 one CTA, 2 two CTAs that each
+ * hold the whole replica, 3 split over a cluster, 0 the Brownian-HI kernels;
+ * its CTAs and their threads (0 for Brownian-HI); row_lists 1 while the partner
+ * lists of a split replica's charged rows have always fit its shared memory (0:
+ * rows of bits were read instead at least once; 0 in the other layouts).  No
+ * reference counterpart.  Each pointer may be NULL. */
+int tis_get_launch(tis_ctx *ctx, int32_t irep, int32_t *layout, int32_t *ctas, int32_t *threads, int32_t *row_lists);
 
 /* Replica exchange over temperature labels (src/energy_allrep.F90:123-260 and
  * src/simu_replica_exchange.F90:18-300): energies at the own and the partner

@@ -206,7 +206,7 @@ EXPORTED = [
     "tis_last_error", "tis_timer", "tis_force_sumup_static", "tis_launch_count",
     "tis_get_hydro_tensors", "tis_set_step", "tis_get_dtrna_status",
     "tis_time_integral", "tis_get_steps", "tis_get_rebuild_info", "tis_get_random_number",
-    "tis_init_ladder", "tis_rex_energies", "tis_rex_exchange_all", "tis_rex_decide",
+    "tis_init_ladder", "tis_rex_energies", "tis_rex_exchange_all", "tis_rex_decide", "tis_get_launch",
 ]
 
 
@@ -252,5 +252,6 @@ def _declare(lib):
     lib.tis_get_random_number.argtypes = [vp, C.c_int64, C.c_int32, _f64p]
     lib.tis_get_steps.argtypes = [vp, C.POINTER(C.c_int64)]
     lib.tis_get_rebuild_info.argtypes = [vp, C.c_int32, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
+    lib.tis_get_launch.argtypes = [vp, C.c_int32, _i32p, _i32p, _i32p, _i32p]
     lib.tis_launch_count.argtypes = [vp]
     lib.tis_launch_count.restype = C.c_int64

@@ -1076,6 +1076,7 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
         try_split(best, best_least, false, clusters);
         c->split_least = best_least;
         c->pair = false;
+        if (source == 1 && minN >= best_least) c->launch_source = 0;   // the table's row is not in use
       }
     }
     // replicas largest first: a CTA that frees its SM takes the next one
@@ -2093,6 +2094,23 @@ extern "C" int tis_get_random_number(tis_ctx *c, int64_t istep, int32_t nstep, d
   return TIS_OK;
 }
 
+extern "C" int tis_get_launch(tis_ctx *c, int32_t irep, int32_t *layout, int32_t *ctas, int32_t *threads,
+                              int32_t *row_lists) {
+  if (!c || irep < 1 || irep > c->nlane) return TIS_E_ARG;
+  const bool split = c->nsplit && c->lane_nmp[irep - 1] >= c->split_least;
+  int lists = 0;
+  if (split) {
+    LaneState l{};
+    CK(copy_now(c, &l, c->d_lstate.p + (irep - 1), sizeof(LaneState), cudaMemcpyDeviceToHost));
+    lists = (l.flags & LF_ROW_BITS) ? 0 : 1;
+  }
+  if (layout) *layout = c->bdhi ? 0 : (split ? 3 : (c->pair ? 2 : 1));
+  if (ctas) *ctas = c->bdhi ? 0 : (split ? c->nsplit : (c->pair ? 2 : 1));
+  if (threads) *threads = c->bdhi ? 0 : (split ? c->split_nt : (c->pair ? 512 : c->threads));
+  if (row_lists) *row_lists = lists;
+  return TIS_OK;
+}
+
 extern "C" int tis_get_rebuild_info(tis_ctx *c, int32_t irep, int64_t *n_rebuild, int64_t *last_step) {
   if (!c || irep < 1 || irep > c->nlane) return TIS_E_ARG;
   LaneState l{};
@@ -2405,12 +2423,13 @@ extern "C" int tis_status(tis_ctx *c, tis_status_t *st) {
     st->exv_pairs_max = std::max(st->exv_pairs_max, ls[i].nexv);
     st->ele_pairs_max = std::max(st->ele_pairs_max, ls[i].nele);
   }
+  const bool split = c->nsplit && c->n_split == c->nlane;
   st->ctas_per_lane = c->pair ? 2 : 1;
-  st->threads_per_cta = c->pair ? 512 : c->threads;
-  st->group = c->group;
-  st->noise_sweep = c->noise_sweep;
+  st->threads_per_cta = split ? c->split_nt : (c->pair ? 512 : c->threads);
+  st->group = split ? SG : c->group;
+  st->noise_sweep = split ? 1 : c->noise_sweep;   // drawn in the sweep
   st->lane_order = c->order;
-  st->sweep = c->sweep;
+  st->sweep = split ? 2 : c->sweep;               // chunks from a shared counter
   st->launch_source = c->launch_source;
   st->wait_timeout = c->wait_timeout;
   st->not_spd = c->not_spd;

@@ -86,7 +86,8 @@ struct LaneState {
 
 enum LaneFlags { LF_OVERFLOW = 1, LF_NAN = 2, LF_UNIF_EXHAUSTED = 4, LF_NOISE_EXHAUSTED = 8, LF_PMF = 16,
                  LF_SMEM = 32 /* the lane's base layout did not fit the launch's shared memory: nothing ran */,
-                 LF_WAIT = 64 /* a wait for the reciprocal sum gave up */ };
+                 LF_WAIT = 64 /* a wait for the reciprocal sum gave up */,
+                 LF_ROW_BITS = 128 /* a split lane's partner lists did not fit its shared memory */ };
 
 enum KMode {
   KM_NEIGHBOR = 1,     // rebuild lists (wrap pxyz if periodic)

@@ -1324,6 +1324,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     if (misc[MISC_CLAMP]) atomicAdd((unsigned long long *)&st.nclamp, (unsigned long long)misc[MISC_CLAMP]);
     if (misc[MISC_NAN]) atomicOr(&st.flags, LF_NAN);
     if (misc[MISC_PMF]) atomicOr(&st.flags, LF_PMF);
+    if (!misc[MISC_ELIST]) atomicOr(&st.flags, LF_ROW_BITS);
     if (PER && a.ew_nwork && rank == 0 && __ldcg(a.ew_sync + EWS_ABORT)) atomicOr(&st.flags, LF_WAIT);
     if (rank == 0) st.istep = istep_end;
   }

@@ -200,6 +200,12 @@ class Engine:
         self._check(self.L.tis_get_rebuild_info(self.h, irep, C.byref(n), C.byref(last)), "rebuild_info")
         return n.value, last.value
 
+    def launch(self, irep=1):
+        """What the steps of replica irep run on (tis_get_launch)."""
+        v = [C.c_int32() for _ in range(4)]
+        self._check(self.L.tis_get_launch(self.h, irep, *[C.byref(q) for q in v]), "launch")
+        return dict(zip(("layout", "ctas", "threads", "row_lists"), (q.value for q in v)))
+
     def last_step_ms(self):
         return self.L.tis_last_step_ms(self.h)
 
