@@ -145,6 +145,17 @@ __device__ __forceinline__ int split_image(const KArgs &a, const S &s, int i, in
   for (int d = 2; d >= 0; --d) c = 3 * c + (v[d] > a.psizeh[d] ? 1 : (v[d] < -a.psizeh[d] ? 2 : 0));
   return c;
 }
+// place of set bit q of m (q < popc(m))
+__device__ __forceinline__ int nth_bit(uint32_t m, int q) {
+  int p = 0;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const int c = __popc(m & ((1u << o) - 1u));
+    if (q >= c) { q -= c; m >>= o; p += o; }
+  }
+  return p;
+}
+
 // b - a + k L (k in {-1, 0, 1}): across the box the two coordinates are ~L
 // apart, so the rounding error of their difference is kept (TwoSum) and the
 // box length taken in two parts; only the short result is rounded
@@ -907,13 +918,23 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
           ele_pair(kind, i, (int)(p & 0xffffu), pi, qci, pmf_row, ax, ay, az);
           ele_pair(kind, i, (int)(p >> 16), pi, qci, pmf_row, bx, by, bz);
         }
-      } else {   // lists too long for the shared memory: the bits of the row
-        const uint32_t pat = (LQ == 32 ? 1u : (LQ == 16 ? 0x00010001u : 0x01010101u)) << gq;
-        for (int w = 0; w < W; ++w)
-          for (uint32_t m = mele[k * W + w] & pat; m; m &= m - 1) {
-            const int j = (w << 5) + __ffs(m) - 1;
-            ele_pair(kind, i, PER ? (j | split_image(a, s, i, j) << SP_IMG) : j, pi, qci, pmf_row, ax, ay, az);
+      } else {
+        // lists too long for the shared memory: the bits of the row, the same
+        // entries in the same order as above (2 (gq + LQ r) and the one after)
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          Real x = 0, y = 0, z = 0;
+          for (int w = 0, n = 0; w < W; ++w) {
+            const uint32_t m = mele[k * W + w];
+            const int c = __popc(m);
+            for (int q = (2 * gq + h - n) & (2 * LQ - 1); q < c; q += 2 * LQ) {
+              const int j = (w << 5) + nth_bit(m, q);
+              ele_pair(kind, i, PER ? (j | split_image(a, s, i, j) << SP_IMG) : j, pi, qci, pmf_row, x, y, z);
+            }
+            n += c;
           }
+          if (h) { bx = x; by = y; bz = z; } else { ax = x; ay = y; az = z; }
+        }
       }
       fx = (double)ax + (double)bx; fy = (double)ay + (double)by; fz = (double)az + (double)bz;
     }
