@@ -968,6 +968,9 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
       int mq = 0;
       for (auto &d : c->tops) {
         if (d.nmp < least) continue;
+        if (d.nunit > 256) return false;
+        for (int b = d.bead0; b < d.bead0 + d.nmp; ++b)
+          if (b_type[b] < 0 || b_type[b] > 15 || b_class[b] < 0 || b_class[b] > 15) return false;   // packed, see SplitSmem
         const int own = split_own(d.nmp, nr);
         d.sp_ninc = 0;
         for (int r = 0; r < nr; ++r) {
@@ -1114,7 +1117,7 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
         Real *re = (Real *)(B0 + pl.RE);
         for (int i = 0; i < N; ++i) {
           const int b = d.bead0 + i;
-          tcu[i] = (uint32_t)(uint8_t)b_type[b] | (uint32_t)(uint8_t)b_class[b] << 8 | (uint32_t)(uint16_t)b_unit[b] << 16;
+          tcu[i] = (uint32_t)b_type[b] | (uint32_t)b_class[b] << 4 | (uint32_t)b_unit[b] << 8;
           re[2 * i] = (Real)b_radius[b]; re[2 * i + 1] = (Real)b_eps[b];
         }
         if (p.i_ele != TIS_ELE_NONE)

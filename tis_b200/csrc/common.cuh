@@ -118,7 +118,7 @@ struct SplitPlan {
   unsigned tcu, RE, qb, base, rn2, comm, C, scr, iptr, cnt, stk, hbk, tsk, bdi, bdd, bdc, bai, bad, bac, sti, std_, stc, hbi, hbd, hbc, hbs;
   unsigned stat;
   // state and scratch
-  unsigned X, P, Q, box, A4, L3, V, DD, C1, u0, NZ, exF, dhF, NR4, near, ncnt, mexv, mele, slots, exc, hbf, red, img, misc;
+  unsigned X, P, Q, A4, L3, V, DD, C1, u0, NZ, exF, dhF, NR4, near, ncnt, mexv, mele, slots, exc, hbf, red, img, misc;
   unsigned eoff, elist;
   unsigned total;
 };

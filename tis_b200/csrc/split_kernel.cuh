@@ -95,8 +95,8 @@ struct SplitSmem {
   typename V4<Real>::T *A4;
   float *L3;               // mixed: pxyz - A4, so that A4 + L3 carries pxyz to ~2^-48
   Real *RE;                // exv radius, sqrt(eps)
-  uint32_t *tcu;           // type | class << 8 | unit << 16
-  int *box;                // periodic: the cell of a bead, (X - P) / L, 10 bits a dimension; changed by list builds only
+  uint32_t *tcu;           // type | class << 4 | unit << 8 | cell << 16; cell: (X - P) / L of a periodic
+                           // lane's bead, 5 bits a dimension, changed by list builds only
 };
 
 // pxyz of any bead from the copies that every step refreshes
@@ -127,12 +127,14 @@ __device__ __forceinline__ void split_pos(const SplitSmem<Real> &s, int i, doubl
   }
 }
 
-// cells packed modulo 1024; component d of the difference of two of them, -512 .. 511
-__device__ __forceinline__ int cell_pack(double x, double y, double z) {
-  return ((int)x & 1023) | ((int)y & 1023) << 10 | ((int)z & 1023) << 20;
+// cells packed modulo 32; component d of the difference of two of them, -16
+// .. 15 (beads of one bonded term that are further apart are not told apart
+// from nearer ones)
+__device__ __forceinline__ uint32_t cell_pack(double x, double y, double z) {
+  return ((uint32_t)(int)x & 31u) | ((uint32_t)(int)y & 31u) << 5 | ((uint32_t)(int)z & 31u) << 10;
 }
-__device__ __forceinline__ int cell_diff(int p, int q, int d) {
-  return (int)((unsigned)((q >> 10 * d) - (p >> 10 * d)) << 22) >> 22;
+__device__ __forceinline__ int cell_diff(uint32_t p, uint32_t q, int d) {   // of two tcu words
+  return (int)(((q >> (16 + 5 * d)) - (p >> (16 + 5 * d))) << 27) >> 27;
 }
 
 // image of the pair (i, j) fixed at the last rebuild, as x_j - x_i sees it
@@ -318,10 +320,9 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   s.L3 = (float *)(sm + pl.L3);
   s.RE = (Real *)(sm + pl.RE);
   s.tcu = (uint32_t *)(sm + pl.tcu);
-  s.box = (int *)(sm + pl.box);
-  auto typ = [&](int i) SPLIT_INL { return (int)(s.tcu[i] & 0xff); };
-  auto cls = [&](int i) SPLIT_INL { return (int)(s.tcu[i] >> 8 & 0xff); };
-  auto unit = [&](int i) SPLIT_INL { return (int)(s.tcu[i] >> 16); };
+  auto typ = [&](int i) SPLIT_INL { return (int)(s.tcu[i] & 15u); };
+  auto cls = [&](int i) SPLIT_INL { return (int)(s.tcu[i] >> 4 & 15u); };
+  auto unit = [&](int i) SPLIT_INL { return (int)(s.tcu[i] >> 8 & 255u); };
   const int lo = min(N, rank * own), hi = min(N, lo + own), nown = hi - lo;
   double *Vv = (double *)(sm + pl.V), *Av = Vv + 3 * OS, *Dv = Av + 3 * OS;   // component d of own bead li at d OS + li
   double *DD = (double *)(sm + pl.DD), *C1 = (double *)(sm + pl.C1);
@@ -404,8 +405,8 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     __syncthreads();
     for (int i = tid; i < N; i += NT) {
       split_pos<Real>(s, i, s.PX[i], s.PY[i], s.PZ[i]);
-      if (PER) s.box[i] = cell_pack(rint((s.X[i] - s.PX[i]) / a.psize[0]), rint((s.Y[i] - s.PY[i]) / a.psize[1]),
-                                    rint((s.Z[i] - s.PZ[i]) / a.psize[2]));
+      if (PER) s.tcu[i] |= cell_pack(rint((s.X[i] - s.PX[i]) / a.psize[0]), rint((s.Y[i] - s.PY[i]) / a.psize[1]),
+                                     rint((s.Z[i] - s.PZ[i]) / a.psize[2])) << 16;
     }
   }
   cl.sync();   // loaded; and every CTA runs before any distributed access
@@ -434,8 +435,8 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     typedef decltype(w) Wt;
     constexpr bool NEAREST = decltype(nearest)::value;
     const V p = s.A4[i], q = s.A4[j];
-    int ci = 0, cj = 0;
-    if (PER && !NEAREST) { ci = s.box[i]; cj = s.box[j]; }
+    uint32_t ci = 0, cj = 0;
+    if (PER && !NEAREST) { ci = s.tcu[i]; cj = s.tcu[j]; }
     if constexpr (sizeof(Wt) == 4) {
       const float *l = s.L3 + 3 * i, *m = s.L3 + 3 * j;
       auto d1 = [&](float x, float y, float lx, float ly, int d) SPLIT_INL {
@@ -545,12 +546,12 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     if (PER) {
       for (int i = tid; i < N; i += NT) {
         const double x = wrap1(s.PX[i], a.psize[0]), y = wrap1(s.PY[i], a.psize[1]), z = wrap1(s.PZ[i], a.psize[2]);
-        const int moved = cell_pack(rint((s.PX[i] - x) / a.psize[0]), rint((s.PY[i] - y) / a.psize[1]),
-                                    rint((s.PZ[i] - z) / a.psize[2]));
+        const uint32_t moved = cell_pack(rint((s.PX[i] - x) / a.psize[0]), rint((s.PY[i] - y) / a.psize[1]),
+                                         rint((s.PZ[i] - z) / a.psize[2]));
         if (moved) {
-          const int c = s.box[i];
-          s.box[i] = ((c & 1023) + (moved & 1023) & 1023) | ((c >> 10 & 1023) + (moved >> 10 & 1023) & 1023) << 10 |
-                     ((c >> 20 & 1023) + (moved >> 20 & 1023) & 1023) << 20;
+          const uint32_t t = s.tcu[i], c = t >> 16;
+          s.tcu[i] = (t & 0xffffu) | ((c + (moved & 31u)) & 31u) << 16 | (((c >> 5) + (moved >> 5)) & 31u) << 21 |
+                     (((c >> 10) + (moved >> 10)) & 31u) << 26;
         }
         s.PX[i] = x; s.PY[i] = y; s.PZ[i] = z;
         s.QX[i] = x; s.QY[i] = y; s.QZ[i] = z;
@@ -921,19 +922,26 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
       } else {
         // lists too long for the shared memory: the bits of the row, the same
         // entries in the same order as above (2 (gq + LQ r) and the one after)
-#pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          Real x = 0, y = 0, z = 0;
-          for (int w = 0, n = 0; w < W; ++w) {
-            const uint32_t m = mele[k * W + w];
-            const int c = __popc(m);
-            for (int q = (2 * gq + h - n) & (2 * LQ - 1); q < c; q += 2 * LQ) {
-              const int j = (w << 5) + nth_bit(m, q);
-              ele_pair(kind, i, PER ? (j | split_image(a, s, i, j) << SP_IMG) : j, pi, qci, pmf_row, x, y, z);
-            }
+        int w = 0, n = 0;   // word, bits of the words before
+        uint32_t m = mele[k * W];
+        auto entry = [&](int e) SPLIT_INL {   // bead (and image) of entry e >= n, -1 beyond the last
+          int c;
+          while (n + (c = __popc(m)) <= e) {
+            if (++w >= W) return -1;
             n += c;
+            m = mele[k * W + w];
           }
-          if (h) { bx = x; by = y; bz = z; } else { ax = x; ay = y; az = z; }
+          const int j = (w << 5) + nth_bit(m, e - n);
+          return PER ? (j | split_image(a, s, i, j) << SP_IMG) : j;
+        };
+#pragma unroll 1
+        for (int e = 2 * gq;; e += 2 * LQ) {
+          const int p = entry(e);
+          if (p < 0) break;
+          ele_pair(kind, i, p, pi, qci, pmf_row, ax, ay, az);
+          const int q = entry(e + 1);
+          if (q < 0) break;
+          ele_pair(kind, i, q, pi, qci, pmf_row, bx, by, bz);
         }
       }
       fx = (double)ax + (double)bx; fy = (double)ay + (double)by; fz = (double)az + (double)bz;

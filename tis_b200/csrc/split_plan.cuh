@@ -37,7 +37,7 @@ inline SplitPlan split_plan(const TopDesc &T, int nq, int row, int nr, bool peri
   const unsigned n = p.np, o = p.own, W = (N + 31) / 32, R = real;
   unsigned b = 0;
   auto take = [&](unsigned bytes) { const unsigned at = b; b = (b + bytes + 15u) & ~15u; return at; };
-  p.tcu = take(4 * n);                    // type | class << 8 | unit << 16
+  p.tcu = take(4 * n);                    // type | class << 4 | unit << 8 (and the kernel's periodic cell << 16)
   p.RE = take(2 * R * n);                 // exv radius, sqrt(eps)
   p.qb = take(4 * nq);
   p.base = take(4 * (SPLIT_MAX + 1));
@@ -56,7 +56,6 @@ inline SplitPlan split_plan(const TopDesc &T, int nq, int row, int nr, bool peri
   p.X = take(24 * n);
   p.P = periodic ? take(24 * n) : p.X;
   p.Q = periodic ? take(24 * n) : p.X;
-  p.box = periodic ? take(4 * n) : 0;     // periodic cell of each bead
   p.A4 = take(4 * R * (n + 4));           // and a bead far away without charge (entry np)
   p.L3 = real == 4 ? take(12 * n) : 0;
   p.V = take((skin ? 72 : 48) * o);       // v, a, [dxyz]
