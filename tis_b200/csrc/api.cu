@@ -16,6 +16,7 @@
 #include <cstddef>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -909,12 +910,13 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const bool mixed = p.precision == TIS_PREC_MIXED;
     const bool pair_ok = !c->bdhi && mixed && !periodic && p.i_ele != TIS_ELE_EWALD && minN >= 64 && pair_fits;
+    const int nall = lad ? lad->nall : nlane;   // a ladder's ranks choose alike
     LaunchCfg cfg;
     int source = 0;
     {
       const std::string path = p.launch_table ? std::string(p.launch_table) : library_dir() + "/tuned_launch.tsv";
       const std::vector<TuneRow> rows = read_tune_table(path);
-      if (!c->bdhi && tune_lookup(rows, maxN, nlane, mixed ? 1 : 0, p.i_ele, periodic ? 1 : 0, skin ? 1 : 0, cfg))
+      if (!c->bdhi && tune_lookup(rows, maxN, nall, mixed ? 1 : 0, p.i_ele, periodic ? 1 : 0, skin ? 1 : 0, cfg))
         source = 1;
     }
     const int env_t = env_int("TIS_THREADS"), env_g = env_int("TIS_GROUP");
@@ -930,7 +932,7 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     if (p.launch_order) { cfg.order = p.launch_order; source = 2; }
     if (p.launch_sweep) { cfg.sweep = p.launch_sweep; source = 2; }
     const int asked = cfg.ctas;
-    if (cfg.ctas == 0) cfg.ctas = (pair_ok && nsm > 0 && 2 * nlane <= nsm) ? 2 : 1;
+    if (cfg.ctas == 0) cfg.ctas = (pair_ok && nsm > 0 && 2 * nall <= nsm) ? 2 : 1;
     if (cfg.ctas == 2 && !pair_ok) cfg.ctas = 1;
     if (cfg.ctas == 2) cfg.threads = 512;   // the cluster kernel runs 512 threads per CTA
     if (cfg.threads == 0) cfg.threads = maxN <= 96 ? 128 : (maxN <= 160 ? 256 : 512);
@@ -1020,37 +1022,69 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
         // The split with the least estimated time of a step of the whole
         // context: nr CTAs for every lane, or for the lanes of a batch that
         // have at least `least` beads, the others on one CTA beside them.
-        // From timings on B200 (chains of 26 to 1,199 beads, 1 to 64 lanes),
-        // microseconds: a lane on one CTA takes t1(N), on nr CTAs c + w(N) /
-        // nr, and lanes that do not fit at once take turns.  A ladder context
-        // decides for the whole ladder, so a replica moves the same whichever
-        // ranks hold it.
+        // A ladder context decides for the whole ladder, so a replica moves the
+        // same whichever ranks hold it.
+        //
+        // Fits to event times on B200 (chains of 23 to 1,199 beads, 1 to 64
+        // lanes, at most 8 % off from 90 beads on), microseconds: a step on one
+        // CTA (t1), on the pair of CTAs that each hold the lane (t2) and on nr
+        // CTAs (tn), and a list rebuild (r1, r2, rn), paid every n_step_neighbor
+        // steps (a skin lasts too long to count).  The split tests every pair
+        // from both sides: 64 lanes of 227 beads 9.8 us a step and 42 a rebuild
+        // against 10.8 and 14 for pairs of CTAs; 599 beads, 4 CTAs 15.5 and 121
+        // against 41 and 58.  Without electrostatics the quadratic terms shrink;
+        // in a box one CTA takes 1.7 and a split 1.2 times as long.  With Ewald
+        // sums the reciprocal part weighs more and wants the SMs that the lanes
+        // leave: a dearer split (8 CTAs rather than 16 for 2 lanes of 165 charges:
+        // 14.5 against 17.2 us a step).  Lanes that do not fit at once take turns.
+        const double every = p.n_step_neighbor > 0 ? 1.0 / p.n_step_neighbor : 0.0;
+        const bool es = p.i_ele != TIS_ELE_NONE, ewald = p.i_ele == TIS_ELE_EWALD;
+        const double quad = es ? 1.0 : 0.4, test = es ? 1.0 : 0.7;
         auto t1 = [&](double n) {
-          return mixed ? 6.0 + 0.010 * n + (cfg.threads >= 1024 ? 0.8e-4 : 1.3e-4) * n * n : 10.0 + 0.02 * n + 1.9e-4 * n * n;
+          if (ewald) return mixed ? 6.0 + 0.010 * n + (cfg.threads >= 1024 ? 0.8e-4 : 1.3e-4) * n * n : 10.0 + 0.02 * n + 1.9e-4 * n * n;
+          const double t = mixed ? 6.0 + 0.005 * n + (cfg.threads >= 1024 ? 0.75e-4 : 1.15e-4) * quad * n * n
+                                 : 8.0 + 0.025 * n + 1.95e-4 * quad * n * n;
+          return t * (periodic ? 1.7 : 1.0) + every * test * (5.0 + 3.0e-4 * n * n) * (periodic ? 2.0 : 1.0);
+        };
+        auto t2 = [&](double n) {
+          const double z = std::max(0.0, n - 240.0);
+          return 6.4 + (es ? 0.020 : 0.014) * n + quad * z * (0.041 + 6.0e-5 * z) + every * test * (4.0 + 0.01 * n + 1.4e-4 * n * n);
         };
         auto tn = [&](double n, int nr) {
-          const double w = mixed ? 0.010 * n + 1.1e-4 * n * n : 0.02 * n + 1.6e-4 * n * n;
-          return (nr == 16 ? 7.0 : 6.0) + n / 300.0 + w / nr;
+          if (ewald) return (nr == 16 ? 7.0 : 6.0) + n / 300.0 + (mixed ? 0.010 * n + 1.1e-4 * n * n : 0.02 * n + 1.6e-4 * n * n) / nr;
+          const double wide = nr == 16 ? 0.45 : 0.0;   // (barriers of more than 8 CTAs)
+          const double t = wide + (mixed ? 3.49 + 0.073 * nr + (0.041 * n + (es ? 5.2e-5 : 0.0) * n * n) / nr
+                                 : 3.43 + 0.068 * nr + 0.0017 * n + (0.0447 * n + (es ? 9.3e-5 : 0.0) * n * n) / nr);
+          return t * (periodic ? 1.2 : 1.0) + every * test * (5.0 + 0.02 * n + 1.2e-3 * n * n / nr) * (periodic ? 1.5 : 1.0);
         };
-        const int nall = lad ? lad->nall : nlane, sms = std::max(nsm, 1);
-        const double scale = (double)nall / nlane;
-        auto total = [&](int nr, int least, int places) {   // nr 0: every lane on one CTA
-          double work = 0.0, longest = 0.0;
-          int n_split = 0;
-          for (int l = 0; l < nlane; ++l) {
-            const double n = c->lane_nmp[l];
-            const bool sp = nr && c->lane_nmp[l] >= least;
-            const double t = sp ? tn(n, nr) : t1(n);
-            work += t * (sp ? nr : 1);
-            longest = std::max(longest, t);
-            n_split += sp;
-          }
-          const int room = nr ? places : sms;
-          if (c->ntop == 1) return longest * ((nall + room - 1) / room);   // equal lanes: whole rounds
-          const double turns = n_split > places || nlane > sms ? 0.25 * longest : 0.0;
-          return std::max(longest, std::max(work * scale / sms, n_split ? work * n_split / nlane / (places * nr) : 0.0) + turns);
+        // lanes in the order of their launch
+        std::vector<int> size(c->lane_nmp.begin(), c->lane_nmp.end());
+        if (cfg.order == 2) std::stable_sort(size.begin(), size.end(), std::greater<int>());
+        const int sms = std::max(nsm, 1);
+        auto total = [&](int nr, int least, int places) {   // nr 0: the launch without a split
+          const int wide = nr ? nr : (c->pair ? 2 : 1);
+          auto time_of = [&](int n, bool sp) { return sp ? tn(n, nr) : (c->pair && !nr ? t2(n) : t1(n)); };
+          const int groups = std::min(nr ? places : sms, sms / wide);   // of SMs that take a cluster
+          if (groups < 1) return 1.0e300;
+          if (c->ntop == 1) return time_of(size[0], nr > 0) * ((nall + groups - 1) / groups);   // equal lanes: whole rounds
+          std::vector<double> free(sms, 0.0);   // when each SM is free
+          for (int pass = 0; pass < 2; ++pass)   // the split lanes, then the others
+            for (int n : size) {
+              const bool sp = nr && n >= least;
+              if (sp != (pass == 0)) continue;
+              const int w = sp || !nr ? wide : 1, m = sp || !nr ? groups : sms;
+              int at = 0;
+              double from = 1.0e300;
+              for (int g = 0; g < m; ++g) {
+                const double f = *std::max_element(&free[g * w], &free[g * w] + w);
+                if (f < from) { from = f; at = g; }
+              }
+              std::fill_n(&free[at * w], w, from + time_of(n, sp));
+            }
+          return *std::max_element(free.begin(), free.end());
         };
-        const double time = total(0, 0, 0);
+        // what runs without a split stands where the estimates are closer than they are right
+        const double time = total(0, 0, 0) / (ewald ? 1.0 : 1.0654);
         std::vector<int> from{0};
         if (c->ntop > 1 && p.i_ele != TIS_ELE_EWALD)
           for (int n : {150, 240, 320, 450, 600, 800, 1000})
@@ -1069,10 +1103,6 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
           const double x = total(o.nr, o.least, clusters);
           if (x < least_time) { least_time = x; best = o.nr; best_least = o.least; }
         }
-        // Lists rebuilt every few steps: the two-CTA kernel rebuilds in 14 us
-        // (64 chains of 227 beads; each pair tested once), the split in 36,
-        // and a step takes 10.75 against 10.25 us: even at one in 44
-        if (best == 2 && !best_least && c->pair && p.n_step_neighbor > 0 && p.n_step_neighbor < 44) best = 0;
       }
       c->nsplit = 0;
       if (best) {
