@@ -194,6 +194,7 @@ struct tis_ctx {
   DBuf<char4> ew_col;
   DBuf<double> ew_w, ew_S, f_ext;
   int ew_nb = 0;
+  int ew_polls = EW_POLLS;
   int ew_work = 0;                  // worker CTAs of the reciprocal sum in the split lanes' launch (0: its own kernels)
   DBuf<unsigned> ew_sync;
   DBuf<double2> ew_E;
@@ -1612,7 +1613,7 @@ KArgs make_args(tis_ctx *c, int mode, int nsteps, int only_lane) {
     a.hmax = c->hmax; a.ew_ncol = c->ew_ncol;
     a.two_pi_L = 2.0 * F_PI / p.psize[0];
     a.ew_col = c->ew_col.p; a.ew_w = c->ew_w.p; a.ew_S = c->ew_S.p;
-    a.ew_sync = c->ew_sync.p; a.ew_E = c->ew_E.p; a.ew_nqmax = c->nq_max;
+    a.ew_sync = c->ew_sync.p; a.ew_polls = c->ew_polls; a.ew_E = c->ew_E.p; a.ew_nqmax = c->nq_max;
     a.ew_nb = c->ew_nb;
   }
   a.f_ext = nullptr;
@@ -2141,6 +2142,14 @@ extern "C" int tis_get_launch(tis_ctx *c, int32_t irep, int32_t *layout, int32_t
   if (ctas) *ctas = c->bdhi ? 0 : (split ? c->nsplit : (c->pair ? 2 : 1));
   if (threads) *threads = c->bdhi ? 0 : (split ? c->split_nt : (c->pair ? 512 : c->threads));
   if (row_lists) *row_lists = lists;
+  return TIS_OK;
+}
+
+// Not part of the interface: the polls of this context's waits for the
+// reciprocal sum, so that a test can make one run out.
+extern "C" int tis_test_ewald_polls(tis_ctx *c, int32_t polls) {
+  if (!c || polls < 1 || polls > EW_POLLS) return TIS_E_ARG;
+  c->ew_polls = polls;
   return TIS_OK;
 }
 

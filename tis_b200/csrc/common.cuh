@@ -21,6 +21,8 @@ constexpr int N_ETYPE = 25;   // E_TYPE%MAX
 constexpr int CHMAX = 1024;   // electrostatic row chunks per lane (at least one per charged bead)
 constexpr int EW_H = 12;      // Ewald: hz = 0 .. 11 of a column (hx, hy) of reciprocal vectors
 enum { EWS_READY = 0, EWS_BARRIER = 32, EWS_DONE = 64, EWS_ABORT = 96, EWS_ARRIVED = 128, EWS_WORDS = 160 };   // words of ew_sync
+constexpr int EW_POLLS = 4000000;     // polls of a wait for the reciprocal sum before it gives up: about 2 s,
+constexpr int EW_START_WAIT = 30;     // and this many times that while a CTA has not started (other work holds its SM)
 constexpr int EW_COLS = 192;  // columns of the half space at most (189 for |h| <= 11)
 // HI_TENSOR (const_index.F90:39-45)
 constexpr int TIS_HI_RPY_DEV = 1, TIS_HI_RPY_OVER_DEV = 2, TIS_HI_ERMAK_OVER_DEV = 3, TIS_HI_ZUK_RPY_DEV = 4;
@@ -153,6 +155,7 @@ struct KArgs {
   // reciprocal sum inside the launch of the split lanes (split_ewald.cuh); ew_nwork 0: separate kernels
   int ew_nwork, ew_nqmax;         // worker CTAs behind the lanes'; largest charge count of a lane
   unsigned *ew_sync;              // counters
+  int ew_polls;                   // EW_POLLS
   int ew_nb;                      // beads of the context
   double2 *ew_E;                  // (EW_H, 3, ew_nb) powers e^{i 2 pi h x_d / L}
   double *f_ext;                  // (3, nbead_total) force added to each bead's sum, or null

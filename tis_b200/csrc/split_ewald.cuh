@@ -31,8 +31,6 @@
 
 namespace tis {
 
-constexpr int EW_WAIT_POLLS = 4000000;   // about 2 s; 30 times that while a CTA has not started (other work holds its SM)
-
 // By a whole warp: after a loop that one thread takes alone the warp stayed in
 // two parts, up to the next shuffle (4 k cycles of a lane's update).
 __device__ __forceinline__ void ew_wait(const KArgs &a, int word, unsigned target) {
@@ -43,9 +41,9 @@ __device__ __forceinline__ void ew_wait(const KArgs &a, int word, unsigned targe
     if ((int)(v - target) >= 0) break;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(ab) : "l"(a.ew_sync + EWS_ABORT) : "memory");
     if (ab) break;
-    if (i >= EW_WAIT_POLLS) {
+    if (i >= a.ew_polls) {
       asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.ew_sync + EWS_ARRIVED) : "memory");
-      if (v >= gridDim.x || i >= 30 * EW_WAIT_POLLS) {
+      if (v >= gridDim.x || i >= EW_START_WAIT * a.ew_polls) {
         atomicExch(a.ew_sync + EWS_ABORT, 1u);
         break;
       }
