@@ -53,6 +53,7 @@ cudaError_t vscale_launch(cudaStream_t st, const KArgs &a, const double *scale, 
 cudaError_t rex_exchange_launch(cudaStream_t st, const KArgs &a, RexState *rex, int *rep2lab, int *lab2rep,
                                 const double *e_own, const double *e_opp, const double *u, double *scale,
                                 double *velo);
+cudaError_t pivot_rcp_launch(const double *p, int n, double *own, double *cuda);
 cudaError_t ewald_recip_launch(cudaStream_t st, const KArgs &a, int nq_max, bool forces);
 cudaError_t ewald_energy_launch(cudaStream_t st, const KArgs &a);
 cudaError_t bd_refactor_launch(cudaStream_t st, KArgs a, int max_nmp, const int *items, const int *koff,
@@ -2143,6 +2144,21 @@ extern "C" int tis_get_launch(tis_ctx *c, int32_t irep, int32_t *layout, int32_t
   if (threads) *threads = c->bdhi ? 0 : (split ? c->split_nt : (c->pair ? 512 : c->threads));
   if (row_lists) *row_lists = lists;
   return TIS_OK;
+}
+
+// Not part of the interface: the Cholesky pivots' reciprocals of p[n] beside
+// CUDA's own, for a test.
+extern "C" int tis_test_pivot_rcp(const double *p, int32_t n, double *own, double *cuda) {
+  if (!p || !own || !cuda || n < 1) return TIS_E_ARG;
+  const size_t nb = n * sizeof(double);
+  double *d = nullptr;
+  cudaError_t e = cudaMalloc((void **)&d, 3 * nb);
+  if (e == cudaSuccess) e = cudaMemcpy(d, p, nb, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = pivot_rcp_launch(d, n, d + n, d + 2 * (size_t)n);
+  if (e == cudaSuccess) e = cudaMemcpy(own, d + n, nb, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(cuda, d + 2 * (size_t)n, nb, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? TIS_OK : TIS_E_CUDA;
 }
 
 // Not part of the interface: the polls of this context's waits for the

@@ -224,20 +224,25 @@ constexpr int FD_X = (CT + FB) * FBP + 2 * FB + 4;   // a block: rows, the block
 constexpr int FD_VEC = CT / FB * FD_X + CT * FBP;
 static_assert(FD_VEC * (int)sizeof(double) <= U64_SMEM, "the factor's work space reuses the operand tiles");
 
-// 1 / p to within an ulp for a normal p: the hardware's approximation y with
-// e = 1 - p y, then Chebyshev's third-order step y (1 + e + e^2).  Without the
-// division's branch the updates of one pivot fill the wait of the next.
+// 1 / p for 2^-1021 <= p <= 2^1021: the instruction's approximation (20 bits
+// or more) and two Newton-Raphson steps y += y (1 - p y), each doubling its
+// bits; at most 1 ulp off (the test takes CUDA's own reciprocal for reference).
+// Without the division's branch the updates of one pivot fill the wait of the
+// next: 821 us for four steps of 150 beads with a refresh each, 856 with
+// __drcp_rn.
+constexpr double PIVOT_MIN = 0x1p-1021, PIVOT_MAX = 0x1p1021;
 __device__ __forceinline__ double pivot_rcp(double p) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(p));
-  const double e = fma(-p, y, 1.0);
-  return fma(y, fma(e, e, e), y);
+  y = fma(y, fma(-p, y, 1.0), y);
+  return fma(y, fma(-p, y, 1.0), y);
 }
 
 // Factor the 8 x 8 block at xin + c0 FBP and solve the thread's row v against
-// it; d = pivots, ip = their reciprocals.  Returns true if a pivot is not > 0:
-// the values are then of no use without guard, which replaces such a pivot by
-// 1 (its compare and selects are on the chain of every pivot: 742 against 574
+// it; d = pivots, ip = their reciprocals.  Returns true if a pivot is outside
+// pivot_rcp's range: the values are then of no use without guard, which divides
+// and replaces a pivot that is not > 0 by 1, and returns true if there is one
+// (its compare and selects are on the chain of every pivot: 742 against 574
 // cycles).
 template <bool guard>
 __device__ __forceinline__ bool diag_block(const double *xin, const double *row, int own, double (&v)[FB],
@@ -260,8 +265,8 @@ __device__ __forceinline__ bool diag_block(const double *xin, const double *row,
   bool bad = false;
 #pragma unroll
   for (int j = 0; j < FB; ++j) {
-    double p = b[j][j], r = pivot_rcp(p);
-    const bool ok = p > 0.0;
+    double p = b[j][j], r = guard ? 1.0 / p : pivot_rcp(p);
+    const bool ok = guard ? p > 0.0 : p >= PIVOT_MIN && p <= PIVOT_MAX;
     bad |= !ok;
     if (guard && !ok) p = r = 1.0;
     d[j] = p;
@@ -331,8 +336,7 @@ __device__ void factor_diag_tile(const KArgs &a, int lane, double *Lm, int n, in
       const double *row = xin + (tid < CT ? tid : FB * s + (tid & 7)) * FBP;
       double v[FB], d[FB], ip[FB];
       if (diag_block<false>(xin + FB * s * FBP, row, own, v, d, ip)) {   // the same in every thread
-        bad = true;
-        diag_block<true>(xin + FB * s * FBP, row, own, v, d, ip);
+        bad |= diag_block<true>(xin + FB * s * FBP, row, own, v, d, ip);
       }
       if (tid < CT + FB) {
 #pragma unroll
@@ -353,7 +357,7 @@ __device__ void factor_diag_tile(const KArgs &a, int lane, double *Lm, int n, in
   // block's column is unscaled: L_ic = x / sqrt(p_c)
   const int c = tid & 63, q = c & 7;
   const double *X = vec + (c >> 3) * FD_X;
-  const double d = sqrt(X[(CT + FB) * FBP + q]), ri = pivot_rcp(d);
+  const double d = sqrt(X[(CT + FB) * FBP + q]), ri = 1.0 / d;
   const int i0 = tid >> 6, c8 = c & ~7;
   double u[CT / 4];
 #pragma unroll
@@ -1237,6 +1241,16 @@ __global__ void __launch_bounds__(256) bd_force_kernel(KArgs a) {
     F[0] = fx; F[1] = fy; F[2] = fz;
     if (nclamp) atomicAdd((unsigned long long *)&a.lstate[lane].nclamp, (unsigned long long)nclamp);
   }
+}
+
+// pivot_rcp and CUDA's reciprocal of n numbers, for its test
+__global__ void pivot_rcp_kernel(const double *p, int n, double *own, double *cuda) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) { own[i] = pivot_rcp(p[i]); cuda[i] = __drcp_rn(p[i]); }
+}
+cudaError_t pivot_rcp_launch(const double *p, int n, double *own, double *cuda) {
+  pivot_rcp_kernel<<<(n + 255) / 256, 256>>>(p, n, own, cuda);
+  return cudaGetLastError();
 }
 
 // ------------------------------------------------------------ launches
