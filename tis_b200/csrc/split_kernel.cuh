@@ -192,6 +192,21 @@ template <typename Real> __device__ __forceinline__ Real sdot(R3<Real> a, R3<Rea
 template <typename Real> __device__ __forceinline__ R3<Real> cross(R3<Real> a, R3<Real> b) {
   return R3<Real>{det2(a.y, b.z, a.z, b.y), det2(a.z, b.x, a.x, b.z), det2(a.x, b.y, a.y, b.x)};
 }
+// n / d from an inverse of d that is off by a few ulp
+__device__ __forceinline__ double quot(double n, double d, double inv) {
+  const double q = n * inv;
+  return fma(fma(-q, d, n), inv, q);
+}
+// a vector's length and its inverse.  FP64: without the corrections by the
+// residuals the length is off by 1.5 ulp, which the difference to the native
+// length magnifies (forces of the chains 24 % further off than with sqrt)
+__device__ __forceinline__ void length(float d2, float &d, float &r) { d = sqrtf(d2); r = __fdividef(1.0f, d); }
+__device__ __forceinline__ void length(double d2, double &d, double &r) {
+  r = rsqrt(d2);
+  const double e = d2 * r;
+  d = fma(fma(-e, e, d2), 0.5 * r, e);
+  r = fma(fma(-d, r, 1.0), r, r);
+}
 template <typename Real> struct Dih { R3<Real> a, b, c, d; Real e; bool straight; };
 template <typename Real, bool CAP>
 __device__ __forceinline__ Dih<Real> dihedral(R3<Real> u, R3<Real> w, R3<Real> z, Real nat, Real k, Real maxc) {
@@ -212,9 +227,13 @@ __device__ __forceinline__ Dih<Real> dihedral(R3<Real> u, R3<Real> w, R3<Real> z
   Real aw, ou, oz, im2, in2;   // |w|, uw / w2, zw / w2, 1 / m2, 1 / n2
   if constexpr (sizeof(Real) == 8) {
     // FP64 divisions are long dependent chains: one reciprocal square root
-    // and one reciprocal stand for a square root and four divisions
-    const Real rw = rsqrt(w2), iw2 = rw * rw, imn = (Real)1 / (m2 * n2);
-    aw = w2 * rw; ou = uw * iw2; oz = zw * iw2; im2 = n2 * imn; in2 = m2 * imn;
+    // and one reciprocal stand for a square root and four divisions, each
+    // result corrected by its residual to the rounding of the operation
+    Real rw;
+    length(w2, aw, rw);
+    const Real iw2 = rw * rw, imn = (Real)1 / (m2 * n2);
+    ou = quot(uw, w2, iw2); oz = quot(zw, w2, iw2);
+    im2 = quot((Real)1, m2, n2 * imn); in2 = quot((Real)1, n2, m2 * imn);
   } else {
     aw = sqrt(w2); ou = fdiv(uw, w2); oz = fdiv(zw, w2); im2 = fdiv((Real)1, m2); in2 = fdiv((Real)1, n2);
   }
@@ -230,9 +249,6 @@ __device__ __forceinline__ Dih<Real> dihedral(R3<Real> u, R3<Real> w, R3<Real> z
 }
 __device__ __forceinline__ float invsqrt(float x) { return rsqrtf(x); }
 __device__ __forceinline__ double invsqrt(double x) { return rsqrt(x); }
-// a vector's length and its inverse
-__device__ __forceinline__ void length(float d2, float &d, float &r) { d = sqrtf(d2); r = __fdividef(1.0f, d); }
-__device__ __forceinline__ void length(double d2, double &d, double &r) { r = rsqrt(d2); d = d2 * r; }
 template <typename Real> __device__ __forceinline__ R3<Real> add3(R3<Real> a, R3<Real> b) {
   return R3<Real>{a.x + b.x, a.y + b.y, a.z + b.z};
 }
@@ -265,7 +281,7 @@ __device__ __forceinline__ void split_angle(R3<Real> v21, R3<Real> v32, Real nat
   if (t3 <= (Real)1) t3 = 1;
   const Real f = cf < (Real)1.0e-6 ? (Real)0 : (Real)2 * cf * (th - nat) * invsqrt(t3);
   Real a1, a2;
-  if constexpr (sizeof(Real) == 8) { const Real r2 = rs * rs; a1 = c21 * c22 * r2; a2 = c21 * c11 * r2; }
+  if constexpr (sizeof(Real) == 8) { const Real r2 = rs * rs; a1 = quot(c21, c11, c22 * r2); a2 = quot(c21, c22, c11 * r2); }
   else { a1 = fdiv(c21, c11); a2 = fdiv(c21, c22); }
   const R3<Real> A{fma(v21.x, a1, -v32.x), fma(v21.y, a1, -v32.y), fma(v21.z, a1, -v32.z)};
   const R3<Real> B{fma(v32.x, a2, -v21.x), fma(v32.y, a2, -v21.y), fma(v32.z, a2, -v21.z)};
@@ -1133,8 +1149,10 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
           const Real p2 = sdot(p, p), q2 = sdot(q, q), pq = sdot(p, q);
           Real apq, co, cp, cq;   // |p| |q|, the cosine, pq / p2, pq / q2
           if constexpr (sizeof(Real) == 8) {
-            const Real r = rsqrt(p2 * q2), r2 = r * r;
-            apq = p2 * q2 * r; co = pq * r; cp = pq * q2 * r2; cq = pq * p2 * r2;
+            Real r;
+            length(p2 * q2, apq, r);
+            const Real r2 = r * r;
+            co = quot(pq, apq, r); cp = quot(pq, p2, q2 * r2); cq = quot(pq, q2, p2 * r2);
           } else {
             apq = sqrt(p2) * sqrt(q2); co = fdiv(pq, apq); cp = fdiv(pq, p2); cq = fdiv(pq, q2);
           }
