@@ -99,22 +99,26 @@ struct SplitSmem {
                            // lane's bead, 5 bits a dimension, changed by list builds only
 };
 
-// pxyz of any bead from the copies that every step refreshes
+// FP64 coordinate of any bead during a sweep: the FP64 path's own copy; mixed,
+// where a step sends FP32 hi and lo parts (2^-48), the owner's through
+// distributed shared memory (nothing writes it between a step's barriers).
+// For the terms that stay FP64 in both paths, few or rare
 template <typename Real>
 struct SplitCoord {
-  const Real *A4;          // component d of bead i at 4 i
-  const float *L3;
+  const Real *A4;          // component of bead i at 4 i
+  const double *X;         // the same component in its owner's copy
+  unsigned magic;          // bead / own = mulhi(bead, magic)
   __device__ double operator[](int i) const {
-    if constexpr (sizeof(Real) == 4) return (double)A4[4 * i] + (double)L3[3 * i];
+    if constexpr (sizeof(Real) == 4) return cg::this_cluster().map_shared_rank(X, (int)__umulhi((unsigned)i, magic))[i];
     else return A4[4 * i];
   }
 };
 template <typename Real>
 struct SplitView { SplitCoord<Real> PX, PY, PZ; };
 template <typename Real>
-__device__ __forceinline__ SplitView<Real> split_view(const SplitSmem<Real> &s) {
+__device__ __forceinline__ SplitView<Real> split_view(const SplitSmem<Real> &s, unsigned magic) {
   const Real *A = (const Real *)s.A4;
-  return SplitView<Real>{{A, s.L3}, {A + 1, s.L3 + 1}, {A + 2, s.L3 + 2}};
+  return SplitView<Real>{{A, s.PX, magic}, {A + 1, s.PY, magic}, {A + 2, s.PZ, magic}};
 }
 
 template <typename Real>
@@ -443,7 +447,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   const bool ewald = a.i_ele == 2, coul = a.i_ele == 3;
   const int LQ = split_row_lanes(NQ, ewald), RW = 32 / LQ;
   // x_j - x_i of the bonded terms in W, in FP32 from the hi and lo parts,
-  // rounded once.  Periodic: of the unwrapped positions (bonds, angles,
+  // rounded once (FP64 terms of the mixed path: from the FP64 positions).  Periodic: of the unwrapped positions (bonds, angles,
   // stacks), i.e. of the wrapped ones and the beads' cells, or the nearest
   // image (hydrogen bonds).  Across the box the two coordinates are ~L apart,
   // so the rounding error of their difference is kept (TwoSum)
@@ -466,12 +470,14 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
       };
       return R3<Wt>{d1(p.x, q.x, l[0], m[0], 0), d1(p.y, q.y, l[1], m[1], 1), d1(p.z, q.z, l[2], m[2], 2)};
     } else {
-      double px = (double)p.x, py = (double)p.y, pz = (double)p.z, qx = (double)q.x, qy = (double)q.y, qz = (double)q.z;
-      if constexpr (sizeof(Real) == 4) {
-        const float *l = s.L3 + 3 * i, *m = s.L3 + 3 * j;
-        px += (double)l[0]; py += (double)l[1]; pz += (double)l[2];
-        qx += (double)m[0]; qy += (double)m[1]; qz += (double)m[2];
+      if constexpr (sizeof(Real) == 4) {   // the owners' unwrapped FP64 positions (see SplitCoord)
+        static_assert(!NEAREST, "");
+        const double *xi = cl.map_shared_rank(s.X, (int)__umulhi((unsigned)i, magic)) + i;
+        const double *xj = cl.map_shared_rank(s.X, (int)__umulhi((unsigned)j, magic)) + j;
+        return R3<Wt>{xj[0] - xi[0], xj[np] - xi[np], xj[2 * np] - xi[2 * np]};
       }
+      const double px = (double)p.x, py = (double)p.y, pz = (double)p.z;
+      const double qx = (double)q.x, qy = (double)q.y, qz = (double)q.z;
       if (PER && !NEAREST) {
         auto d1 = [&](double x, double y, int d) SPLIT_INL {
           const double t = y - x, bb = t - y, e = (y - (t - bb)) + (-x - bb);
@@ -1054,7 +1060,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
         const int m[7] = {(int)(ix.x & 0xffff), (int)(ix.x >> 16), (int)(ix.y & 0xffff), (int)(ix.y >> 16),
                           (int)(ix.z & 0xffff), (int)(ix.z >> 16), (int)(ix.w & 0xffff)};
         const double u0 = u0s[k];
-        const bool off = T.ntst > 0 && stack_excluded<Real>(a, T, split_view(s), stk[k]), live = k0 < nst;
+        const bool off = T.ntst > 0 && stack_excluded<Real>(a, T, split_view(s, magic), stk[k]), live = k0 < nst;
         // the stack in W (nat and coef of its distance, then of this thread's
         // dihedral): forces of beads 0 / 1, 2 / 6, 3 / 5 and (thread 0) 4;
         // true when a triple is too straight for FP32
@@ -1215,7 +1221,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
       } else {
         const int k = ((c - c_ts) << 5) + lid;
         if (k < nts) {
-          const SplitView<Real> s2 = split_view(s);   // copies: the values used elsewhere stay in registers
+          const SplitView<Real> s2 = split_view(s, magic);   // copies: the values used elsewhere stay in registers
           const TopDesc T2 = T;
           const SplitDst<Real> d2 = dst;
           term_tstack<Real>(a, T2, s2, d2, tsk[k]);
