@@ -18,6 +18,7 @@
 #include <cstring>
 #include <functional>
 #include <mutex>
+#include <queue>
 #include <string>
 #include <vector>
 
@@ -204,11 +205,14 @@ struct tis_ctx {
   int max_nmp = 0;
   long long bd_istep = 0;
   // pinned staging of the state's and the replicas' copies; null: the caller's
-  // memory is copied directly
+  // memory is copied directly.  A state that does not fit goes through its two
+  // halves in turn, each copied to or from the caller while the other is on
+  // its way
   unsigned char *stage = nullptr;
-  size_t stage_state = 0;             // bytes for three state arrays; the replicas' states and flags follow
-  cudaEvent_t stage_ev = nullptr;     // the last copy out of it
-  bool stage_busy = false;
+  size_t stage_state = 0;             // bytes for the state; the replicas' states and flags follow
+  size_t stage_half = 0;              // 0: three state arrays fit
+  cudaEvent_t stage_ev[2] = {nullptr, nullptr};   // the last copy out of (set_state) or into (get_state) a half
+  bool stage_busy[2] = {false, false};
   DBuf<int> fene_idx, wca_idx, bd_ptr, d_not_spd;
   DBuf<int2> bd_ent;
   DBuf<double> fene_cls, wca_cls, b_hrad;
@@ -393,27 +397,27 @@ void ewald_columns(double L, double alpha, double hmax, std::vector<char4> &col,
 
 // --------------------------------------------------------------------- init
 namespace {
-// How many clusters of nr CTAs of the split kernel the GPU holds at once (0:
-// none); asked once per process, device and kernel variant (its registers
-// allow one CTA per SM, so neither the threads nor the shared memory of a
-// context change it).
-int split_clusters(int nr, bool mixed, bool periodic) {
+// How many clusters of nr CTAs of nt threads of the split kernel the GPU holds
+// at once (0: none); asked once per process, device and kernel variant (its
+// registers allow one CTA per SM, so the shared memory of a context does not
+// change it).  Asking loads the variant: about 4 ms each.
+int split_clusters(int nr, int nt, bool mixed, bool periodic) {
   static std::mutex mu;
-  static std::map<std::array<int, 4>, int> known;
+  static std::map<std::array<int, 5>, int> known;
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
-  const std::array<int, 4> key{dev, nr, mixed, periodic};
+  const std::array<int, 5> key{dev, nr, nt, mixed, periodic};
   const auto it = known.find(key);
   if (it != known.end()) return it->second;
   auto setup = periodic ? (mixed ? split_setup_mixed_box : split_setup_fp64_box)
                         : (mixed ? split_setup_mixed : split_setup_fp64);
-  int n = 0, m = 0;
-  if (setup(nr, 256, 227 * 1024, &n) != cudaSuccess || setup(nr, 512, 227 * 1024, &m) != cudaSuccess) {
+  int n = 0;
+  if (setup(nr, nt, 227 * 1024, &n) != cudaSuccess) {
     cudaGetLastError();
-    n = m = 0;
+    n = 0;
   }
-  return known[key] = std::min(n, m);
+  return known[key] = n;
 }
 
 // the whole ladder of a context that holds only some of its replicas
@@ -750,14 +754,9 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
       for (int q2 = 0; q2 < 6; ++q2) inc[t.idtrna_hb2mp[6 * b + q2] - 1].push_back(d.slot_hb + 6 * b + q2);
     int ip = (int)inc_slot.size();
     const int ip0 = ip;
-    d.sp0 = (int)slot_pos.size();
-    slot_pos.resize(slot_pos.size() + d.nslot, 0);
     for (int i = 0; i < t.nmp; ++i) {
       inc_ptr.push_back(ip);
-      for (size_t q = 0; q < inc[i].size(); ++q) {
-        inc_slot.push_back(inc[i][q]);
-        slot_pos[d.sp0 + inc[i][q]] = ip - ip0 + (int)q;
-      }
+      for (int sl : inc[i]) inc_slot.push_back(sl);
       ip += (int)inc[i].size();
     }
     inc_ptr.push_back(ip);
@@ -1005,10 +1004,8 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
       const SplitPlan sp = split_plan(mx, mq, row, nr, periodic, skin, ewald, real_size, 227 * 1024);
       // (without room for the lists the kernel reads the rows' bits, ~4x slower)
       if (sp.total > 227 * 1024 || (lists && sp.ecap < (unsigned)sp.rows * row)) return false;
-      // 256 threads (with twice the registers) while a CTA's warps have a
-      // few work items each, 512 above
-      const int nt = sp.own <= 32 ? 256 : 512;
-      clusters = split_clusters(nr, mixed, periodic);
+      const int nt = split_threads(mx.nmp, nr);
+      clusters = split_clusters(nr, nt, mixed, periodic);
       if (clusters < 1) return false;
       c->nsplit = nr;
       c->split_nt = nt;
@@ -1069,21 +1066,27 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
           const int groups = std::min(nr ? places : sms, sms / wide);   // of SMs that take a cluster
           if (groups < 1) return 1.0e300;
           if (c->ntop == 1) return time_of(size[0], nr > 0) * ((nall + groups - 1) / groups);   // equal lanes: whole rounds
-          std::vector<double> free(sms, 0.0);   // when each SM is free
-          for (int pass = 0; pass < 2; ++pass)   // the split lanes, then the others
+          // when each group of SMs, then each SM, is free: the split lanes, then the others
+          typedef std::priority_queue<double, std::vector<double>, std::greater<double>> Queue;
+          double last = 0.0;
+          auto run = [&](Queue &q, bool sp) {
             for (int n : size) {
-              const bool sp = nr && n >= least;
-              if (sp != (pass == 0)) continue;
-              const int w = sp || !nr ? wide : 1, m = sp || !nr ? groups : sms;
-              int at = 0;
-              double from = 1.0e300;
-              for (int g = 0; g < m; ++g) {
-                const double f = *std::max_element(&free[g * w], &free[g * w] + w);
-                if (f < from) { from = f; at = g; }
-              }
-              std::fill_n(&free[at * w], w, from + time_of(n, sp));
+              if ((nr && n >= least) != sp) continue;
+              const double end = q.top() + time_of(n, sp);
+              q.pop();
+              q.push(end);
+              last = std::max(last, end);
             }
-          return *std::max_element(free.begin(), free.end());
+          };
+          Queue group, sm;
+          for (int g = 0; g < groups; ++g) group.push(0.0);
+          run(group, nr > 0);
+          if (!nr || least == 0) return last;
+          for (int k = groups * wide; k < sms; ++k) sm.push(0.0);
+          for (; !group.empty(); group.pop())
+            for (int k = 0; k < wide; ++k) sm.push(group.top());
+          run(sm, false);
+          return last;
         };
         // what runs without a split stands where the estimates are closer than they are right
         const double time = total(0, 0, 0) / (ewald ? 1.0 : 1.0654);
@@ -1101,9 +1104,11 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
         double least_time = time;
         for (const Option &o : options) {
           if (o.time >= least_time) break;
-          if (!try_split(o.nr, o.least, true, clusters)) continue;
-          const double x = total(o.nr, o.least, clusters);
-          if (x < least_time) { least_time = x; best = o.nr; best_least = o.least; }
+          const double x = total(o.nr, o.least, split_clusters(o.nr, split_threads(maxN, o.nr), mixed, periodic));
+          if (x >= least_time || !try_split(o.nr, o.least, true, clusters)) continue;
+          least_time = x;
+          best = o.nr;
+          best_least = o.least;
         }
       }
       c->nsplit = 0;
@@ -1129,6 +1134,13 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
   std::vector<unsigned char> split_blob;
   if (c->nsplit) {
     const int nr = c->nsplit;
+    for (auto &d : c->tops) {   // place of each slot in the incidence lists
+      d.sp0 = (int)slot_pos.size();
+      if (d.nmp < c->split_least) continue;
+      slot_pos.resize(slot_pos.size() + d.nslot, 0);
+      const int first = inc_ptr[d.inc0];
+      for (int k = first; k < inc_ptr[d.inc0 + d.nmp]; ++k) slot_pos[d.sp0 + inc_slot[k]] = k - first;
+    }
     auto build = [&](auto real) {
       typedef decltype(real) Real;
       for (auto &d : c->tops) {
@@ -1358,7 +1370,7 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
     // whole ladder
     if (c->nsplit && c->n_split == nlane && c->nq_max > 0) {
       const int nall = lad ? lad->nall : nlane;
-      const int clusters = split_clusters(c->nsplit, p.precision == TIS_PREC_MIXED, true);
+      const int clusters = split_clusters(c->nsplit, c->split_nt, p.precision == TIS_PREC_MIXED, true);
       if ((clusters - nall) * c->nsplit >= 48 && ew_smem(nall, c->nq_max, c->ew_ncol).total <= 227 * 1024) {
         c->ew_work = (clusters - nlane) * c->nsplit;
         c->ew_nb = (int)(n3 / 3);
@@ -1371,11 +1383,15 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
   }
   c->clamp_seen.assign(nlane, 0);
   {
-    // up to 64 MB of the host's memory stay pinned while the context lives
-    const size_t state = 3 * n3 * sizeof(double), all = state + nlane * (sizeof(LaneState) + sizeof(int));
-    if (all <= ((size_t)64 << 20) && cudaHostAlloc((void **)&c->stage, all, cudaHostAllocDefault) == cudaSuccess) {
-      c->stage_state = state;
-      CK(cudaEventCreateWithFlags(&c->stage_ev, cudaEventDisableTiming));
+    // at most 1 MB pinned while the context lives: that much comes from memory
+    // that the driver keeps pinned, in microseconds; 2 MB took 3 ms and 8 MB 9 ms,
+    // more than the copies of many calls gain
+    const size_t most = (size_t)1 << 20, state = 3 * n3 * sizeof(double), rest = nlane * (sizeof(LaneState) + sizeof(int));
+    const size_t half = state + rest <= most ? 0 : (rest <= most / 2 ? (most - rest) / 2 / 4096 * 4096 : 1);
+    if (half != 1 && cudaHostAlloc((void **)&c->stage, half ? most : state + rest, cudaHostAllocDefault) == cudaSuccess) {
+      c->stage_state = half ? 2 * half : state;
+      c->stage_half = half;
+      for (auto &e : c->stage_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     } else {
       c->stage = nullptr;
       cudaGetLastError();
@@ -1411,7 +1427,8 @@ extern "C" void tis_destroy(tis_ctx *c) {
   if (!c) return;
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->stage) cudaFreeHost(c->stage);
-  if (c->stage_ev) cudaEventDestroy(c->stage_ev);
+  for (auto &e : c->stage_ev)
+    if (e) cudaEventDestroy(e);
   c->d_tops.free(); c->d_lanes.free(); c->d_lstate.free();
   c->b_type.free(); c->b_class.free(); c->b_unit.free();
   c->b_rcmass.free(); c->b_cmass.free(); c->b_fric.free(); c->b_radius.free(); c->b_eps.free(); c->b_charge.free();
@@ -1468,34 +1485,54 @@ __global__ void set_istep_kernel(LaneState *ls, int n, long long istep) {
   for (int l = threadIdx.x; l < n; l += blockDim.x) ls[l].istep = istep;
 }
 
-// Waits until the staging memory may be overwritten.
-cudaError_t stage_free(tis_ctx *c) {
-  if (!c->stage_busy) return cudaSuccess;
-  c->stage_busy = false;
-  return cudaEventSynchronize(c->stage_ev);
+// Waits until half h of the staging memory may be overwritten or read (whole
+// states use the event of half 0).
+cudaError_t stage_free(tis_ctx *c, int h) {
+  if (!c->stage_busy[h]) return cudaSuccess;
+  c->stage_busy[h] = false;
+  return cudaEventSynchronize(c->stage_ev[h]);
+}
+cudaError_t stage_mark(tis_ctx *c, int h) {
+  c->stage_busy[h] = true;
+  return cudaEventRecord(c->stage_ev[h], c->stream);
+}
+
+// A state array to the device through the two halves in turn.
+cudaError_t stage_put(tis_ctx *c, double *dst, const double *src, size_t n, int &h) {
+  for (size_t at = 0; at < n; at += c->stage_half, h ^= 1) {
+    const size_t m = std::min(c->stage_half, n - at);
+    unsigned char *part = c->stage + h * c->stage_half;
+    cudaError_t e = stage_free(c, h);
+    if (e != cudaSuccess) return e;
+    std::memcpy(part, (const unsigned char *)src + at, m);
+    e = cudaMemcpyAsync((unsigned char *)dst + at, part, m, cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = stage_mark(c, h);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 }  // namespace
 
 // The caller's arrays are copied to pinned memory and queued from there, so
 // that the call does not wait for the device (one copy of the positions; the
-// wrapped ones start as a device copy).
+// wrapped ones start as a device copy); a state beyond the staging memory waits
+// for all but its last two parts.
 extern "C" int tis_set_state(tis_ctx *c, const double *xyz, const double *velo, const double *accel) {
   if (!c || !xyz) return TIS_E_ARG;
   size_t n = 3 * (size_t)c->nbead_total * sizeof(double);
-  CK(stage_free(c));
+  int h = 0;
+  if (!c->stage_half) CK(stage_free(c, 0));
   auto put = [&](double *dst, const double *src, int part) {
     if (!src) return cudaMemsetAsync(dst, 0, n, c->stream);
     if (!c->stage) return cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, c->stream);
+    if (c->stage_half) return stage_put(c, dst, src, n, h);
     std::memcpy(c->stage + part * n, src, n);
     return cudaMemcpyAsync(dst, c->stage + part * n, n, cudaMemcpyHostToDevice, c->stream);
   };
   CK(put(c->xyz.p, xyz, 0));
   CK(put(c->velo.p, velo, 1));
   CK(put(c->accel.p, accel, 2));
-  if (c->stage) {
-    CK(cudaEventRecord(c->stage_ev, c->stream));
-    c->stage_busy = true;
-  }
+  if (c->stage && !c->stage_half) CK(stage_mark(c, 0));
   CK(cudaMemcpyAsync(c->pxyz.p, c->xyz.p, n, cudaMemcpyDeviceToDevice, c->stream));
   CK(cudaMemsetAsync(c->dxyz.p, 0, n, c->stream));
   if (!c->stage) CK(cudaStreamSynchronize(c->stream));
@@ -1505,9 +1542,34 @@ extern "C" int tis_set_state(tis_ctx *c, const double *xyz, const double *velo, 
 extern "C" int tis_get_state(tis_ctx *c, double *xyz, double *velo, double *accel) {
   if (!c) return TIS_E_ARG;
   size_t n = 3 * (size_t)c->nbead_total * sizeof(double);
-  CK(stage_free(c));
   double *const out[3] = {xyz, velo, accel};
   const double *const dev[3] = {c->xyz.p, c->velo.p, c->accel.p};
+  for (int h = 0; h < 2; ++h) CK(stage_free(c, h));
+  if (c->stage_half) {
+    // part p is queued into half p % 2, then part p - 1 copied to the caller
+    const size_t part = c->stage_half, np = (n + part - 1) / part;
+    unsigned char *to = nullptr;
+    size_t bytes = 0;
+    int h = 0;
+    auto take = [&](int half) {   // the part waiting there
+      if (!to) return cudaSuccess;
+      const cudaError_t e = stage_free(c, half);
+      if (e == cudaSuccess) std::memcpy(to, c->stage + half * part, bytes);
+      return e;
+    };
+    for (int k = 0; k < 3; ++k)
+      for (size_t p = 0; out[k] && p < np; ++p, h ^= 1) {
+        const size_t at = p * part, m = std::min(part, n - at);
+        CK(cudaMemcpyAsync(c->stage + h * part, (const unsigned char *)dev[k] + at, m, cudaMemcpyDeviceToHost, c->stream));
+        CK(stage_mark(c, h));
+        CK(take(h ^ 1));
+        to = (unsigned char *)out[k] + at;
+        bytes = m;
+      }
+    CK(take(h ^ 1));
+    CK(cudaStreamSynchronize(c->stream));
+    return TIS_OK;
+  }
   for (int k = 0; k < 3; ++k)
     if (out[k])
       CK(cudaMemcpyAsync(c->stage ? (void *)(c->stage + k * n) : out[k], dev[k], n, cudaMemcpyDeviceToHost, c->stream));

@@ -24,6 +24,10 @@ __host__ __device__ inline int split_row_lanes(int nq, bool ewald) {
 // own beads of a CTA for a lane of N beads
 __host__ __device__ inline int split_own(int N, int nr) { return ((N + nr - 1) / nr + 3) & ~3; }
 
+// threads of a CTA: 256 (with twice the registers) while its warps have a few
+// work items each, 512 above
+inline int split_threads(int N, int nr) { return split_own(N, nr) <= 32 ? 256 : 512; }
+
 // T: the largest counts of the context's topologies; bonded items: of a CTA
 // row: partners of a charged row to make room for (on average over a CTA's rows)
 inline SplitPlan split_plan(const TopDesc &T, int nq, int row, int nr, bool periodic, bool skin, bool ewald, int real,
