@@ -85,3 +85,24 @@ def test_brownian_hi_has_no_lane_kernel(tis_lib):
     eng = Engine([synth.bead_chain(24, 7)], synth.bdhi_params(), [300.0])
     assert eng.launch() == dict(layout=0, ctas=0, threads=0, row_lists=0)
     eng.close()
+
+
+def test_a_recorded_period_of_a_batch_with_both_kernels(tis_lib):
+    """tis_run records the two kernels' launches on two streams: the same
+    steps as tis_step, bit for bit, also when replayed."""
+    systems = [chain(k) for k in [300] * 12 + [20] * 150]
+    par = synth.dt15_params(ionic_strength=0.15, n_step_neighbor=0, precision=0)
+    out = []
+    for recorded in (False, True):
+        eng = Engine(systems, par, [300.0] * len(systems), nrep=[1] * len(systems))
+        assert eng.launch(1)["layout"] == 3 and eng.launch(162)["layout"] == 1
+        eng.set_state(np.vstack([s["xyz"] for s in systems]))
+        eng.time_integral_pre()
+        for _ in range(2):
+            if recorded:
+                eng.run(2, 4, exchange=False)
+            else:
+                eng.step(8)
+        out.append(eng.get_state())
+        eng.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))

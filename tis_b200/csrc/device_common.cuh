@@ -18,16 +18,10 @@ static __device__ unsigned long long g_phase[128];
 #else
 #define PHASE_ALL(k, t0) do { if (blockIdx.x == 0) { atomicAdd(&g_phase[k], (unsigned long long)(clock64() - (t0))); atomicAdd(&g_phase[(k) + 16], 1ull); } } while (0)
 #endif
-// per-warp spans by kind of work of CTA 0: total at 32 + k, count at 48 + k
-#define PHASE_KIND(k, t0) do { if (blockIdx.x == 0 && (threadIdx.x & 31) == 0) { const int k_ = (k); atomicAdd(&g_phase[32 + k_], (unsigned long long)(clock64() - (t0))); atomicAdd(&g_phase[48 + k_], 1ull); } } while (0)
-// spans of thread 0 of the first 16 CTAs
-#define PHASE_CTA(base, t0) do { if (threadIdx.x == 0 && blockIdx.x < 16) atomicAdd(&g_phase[(base) + blockIdx.x], (unsigned long long)(clock64() - (t0))); } while (0)
 // per-warp spans of the first two CTAs: slots base + 16 blockIdx.x + warp
 #define PHASE_WARP(base, t0) do { if (blockIdx.x < 2 && (threadIdx.x & 31) == 0) atomicAdd(&g_phase[(base) + 16 * blockIdx.x + (threadIdx.x >> 5)], (unsigned long long)(clock64() - (t0))); } while (0)
 #else
 #define PHASE_WARP(base, t0) do {} while (0)
-#define PHASE_KIND(k, t0) do {} while (0)
-#define PHASE_CTA(base, t0) do {} while (0)
 #define PHASE_ALL(k, t0) do {} while (0)
 #define PHASE_T0(v) do {} while (0)
 #define PHASE_ADD(k, t0) do {} while (0)

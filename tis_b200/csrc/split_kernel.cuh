@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   // this CTA's copy; send() then hands the block to the other CTAs
   const int g = tid & (SG - 1), grp = tid / SG;
   constexpr int NG = NT / SG;
-  auto xmove = [&](int li, bool valid, int par, bool fire) SPLIT_INL {
+  auto xmove = [&](int li, bool valid, bool fire) SPLIT_INL {
     const int i = lo + li;
     if (valid && g < 3) {
       const int q = g * OS + li;
@@ -805,9 +805,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   // 16 bytes per thread, whole warps per CTA: scattered stores of single
   // values cost ~2 cycles each on the SM-to-SM network
   auto send = [&](int par) SPLIT_INL {
-    PHASE_T0(t_y);
     __syncthreads();
-    PHASE_ADD(13, t_y);
     constexpr int PV = sizeof(V) / 16;
     const int avail = max(((N + 3) & ~3) - lo, 0);   // beads from lo on: the last block is shorter
     const int nA = min(own, avail) * PV, nL = sizeof(Real) == 4 ? min(own, avail) * 3 / 4 : 0;
@@ -988,9 +986,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     if (tid == 0) misc[MISC_EXCESS + (par ^ 1)] = 0;
     const int c_end = c_nz + (noise_step >= 0 ? n_nz : 0);
     int c = warp;
-    PHASE_T0(t_s);
     while (c < c_end) {
-      PHASE_T0(t_c);
       int cn = 0;   // the next chunk, requested before this one is processed
       if (lid == 0) cn = atomicAdd(&misc[MISC_CHUNK], 1);
       if (c >= c_ex && c < c_ba) {
@@ -1227,21 +1223,11 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
           term_tstack<Real>(a, T2, s2, d2, tsk[k]);
         }
       }
-      PHASE_KIND(c < c_ts ? 1 : c < c_st ? 0 : c < c_dh ? 2 : c < c_ex ? 3 : c < c_ba ? 4 : c < c_bd ? 5 : c < c_nz ? 6 : 7, t_c);
       c = __shfl_sync(0xffffffffu, cn, 0);
     }
-    PHASE_ADD(1, t_s);
-#ifdef TIS_PHASE_TIMING
-    if (lid == 0) atomicMax(&misc[15], (int)(clock64() - t_s));
-    __syncthreads();
-    if (tid == 0) { atomicAdd(&g_phase[64 + blockIdx.x % 16], (unsigned long long)misc[15]); misc[15] = 0; }
-#endif
-    PHASE_T0(t_b);
     if constexpr (PER)
       if (a.ew_nwork && warp == 0) ew_wait(a, EWS_DONE, ew_done);   // this step's reciprocal forces
     cl.sync();
-    PHASE_ADD(2, t_b);
-    PHASE_CTA(80, t_b);
     if (tid == 0) {
       misc[MISC_CHUNK] = NW;   // every warp has taken its last chunk
       misc[MISC_NEAR_BAD] = 0;
@@ -1278,11 +1264,9 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
   bool do_build = lists_new || (first_x && fire), do_x = first_x;
   for (int step = 0;; ++step) {
     const int par = (int)(istep & 1);
-    PHASE_T0(t_l);
     if (do_build) build(istep, step == 0);
-    PHASE_ADD(5, t_l);
     if (do_x) {
-      for (int l0 = 0; l0 < nown; l0 += NG) xmove(l0 + grp, l0 + grp < nown, par, fire);
+      for (int l0 = 0; l0 < nown; l0 += NG) xmove(l0 + grp, l0 + grp < nown, fire);
       send(par);
     }
     if (step >= nloop) break;
@@ -1293,9 +1277,7 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
         ew_done = (unsigned)(step + 1) * (unsigned)a.ew_nwork;
         ew_publish(a, s.PX, np, lo, nown, L.state0, tid, NT);
       }
-    PHASE_T0(t_a);
     cl.sync();   // the positions of this step are complete
-    PHASE_ADD(3, t_a);
     if constexpr (PER)
       if (a.ew_nwork && tid == 0) ew_signal(a, EWS_READY);
     const bool next = a.mode == KM_STEP ? step + 1 < nloop
@@ -1314,7 +1296,6 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
     const bool rec = misc[MISC_NEAR_BAD] != 0 || __int_as_float(far) > SP_SKIN_DISP * SP_SKIN_DISP;
     sweep(istep, stepping ? a.noise_base + step : (a.mode == KM_PRE ? a.noise_base : -1), par, rec);
     const bool move = next && !fire;
-    PHASE_T0(t_u);
     for (int l0 = 0; l0 < nown; l0 += NG) {
       const int li = l0 + grp, i = lo + li;
       const bool valid = li < nown;
@@ -1326,7 +1307,6 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
           fx += (double)slots[3 * p]; fy += (double)slots[3 * p + 1]; fz += (double)slots[3 * p + 2];
         }
       group_reduce<Real>(fx, fy, fz, SG);
-      PHASE_ADD(10, t_u);
       if (valid && g < 3) {
         double f = (g == 0 ? fx : (g == 1 ? fy : fz)) + exF[3 * li + g] + dhF[3 * li + g];
         if (PER) f += fe;
@@ -1342,12 +1322,9 @@ __global__ void __launch_bounds__(NT) split_kernel(const __grid_constant__ KArgs
         }
       }
       __syncwarp();
-      PHASE_ADD(11, t_u);
-      if (move) xmove(li, valid, par ^ 1, false);
-      PHASE_ADD(12, t_u);
+      if (move) xmove(li, valid, false);
     }
     if (move) send(par ^ 1);
-    PHASE_ADD(4, t_u);
     // hbond-site counters of the next sweep (read behind this one's barriers)
     if (rank == 0) for (int k = tid; k < T.nsite; k += NT) exc[k] = 0;
     if (!next) break;
