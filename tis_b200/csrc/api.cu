@@ -1397,6 +1397,9 @@ int init_impl(int32_t ntop, const tis_topology *tops, const tis_params *par, con
       cudaGetLastError();
     }
   }
+  // the zeros above were queued on the default stream, which the context's
+  // stream does not wait for (set_state returns before its copies are done)
+  CK(cudaStreamSynchronize(nullptr));
   *out = c;
   return TIS_OK;
 }
