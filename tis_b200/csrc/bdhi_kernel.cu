@@ -208,7 +208,7 @@ __device__ __forceinline__ void load_diag_tile(const double *Lm, int n, int td, 
 // row of the matrix below the block or a row of the identity above.
 // In one launch of its own, cold (ncu): 36.8 us when one warp factored 16
 // columns for all rows, pivots and columns passed by shuffles, and the inverse
-// followed in 64 more steps; 11.6 us this way.
+// followed in 64 more steps; 11.9 us this way.
 //
 // The results are written at the end: with the idle warps writing a block's
 // while the next is factored, a block took 900 + 1050 cycles (factor, update)
@@ -242,8 +242,7 @@ __device__ __forceinline__ double pivot_rcp(double p) {
 // it; d = pivots, ip = their reciprocals.  Returns true if a pivot is outside
 // pivot_rcp's range: the values are then of no use without guard, which divides
 // and replaces a pivot that is not > 0 by 1, and returns true if there is one
-// (its compare and selects are on the chain of every pivot: 742 against 574
-// cycles).
+// (its division, compare and selects are on the chain of every pivot).
 template <bool guard>
 __device__ __forceinline__ bool diag_block(const double *xin, const double *row, int own, double (&v)[FB],
                                            double (&d)[FB], double (&ip)[FB]) {
@@ -869,7 +868,7 @@ __global__ void __launch_bounds__(128) bd_noise_kernel(KArgs a) {
 // doubles per lane, 32 bytes apart), so with one row per warp L1 was the bound
 // (640 MB in 187 us, 3.4 TB/s; 32 lanes of 100 to 1000 beads).  R = 4 rows share
 // the loads of F and xi, and the matrices stream past L1 with 16 float4 in flight
-// per lane: 116 us (5.6 TB/s; more rows, warps or bytes in flight, or rows
+// per lane: 111 us (5.8 TB/s; more rows, warps or bytes in flight, or rows
 // staged by bulk copies, were no faster).  Every row's sum has the same order
 // for either R (columns by lane, then a butterfly).
 struct Rows64 {
@@ -1409,7 +1408,7 @@ cudaError_t bd_step_launch(cudaStream_t st, const KArgs &a, int max_nmp) {
     refine_trsv_kernel<<<a.nlane, TRSV_THREADS, sm, st>>>(a);
   }
   // four rows per warp once that still gives every SM two CTAs (64 rows): 32
-  // chains of 100 to 1,000 beads 110 us against 187 with one row; below, the
+  // chains of 100 to 1,000 beads 111 us against 187 with one row; below, the
   // rows of one warp would queue up behind one another on idle SMs
   if ((long long)3 * max_nmp * a.nlane >= 64LL * BD_SMS)
     bd_update_kernel<4><<<dim3((3 * max_nmp + 31) / 32, a.nlane), 256, 0, st>>>(a);

@@ -4,7 +4,7 @@
 // lane keeps one of 148 SMs busy for 121 us a step, and what bounds it is that
 // SM's issue rate and the latency of its longest items, not memory.  Split
 // over 16 CTAs the same step takes 12.2 us; 599 beads in FP64 82 -> 9.5 us,
-// 227 beads mixed 10.3 -> 5.8 us (8 CTAs), 65 beads FP64 11.2 -> 6.2 us (B200,
+// 227 beads mixed 10.3 -> 5.8 us (8 CTAs), 65 beads FP64 11.2 -> 6.3 us (B200,
 // event time of the step kernel).  Every mode of the lane kernel (KM_*) runs
 // here, for both precisions, with or without a periodic box.
 //
@@ -24,7 +24,8 @@
 //           reads every position, writes slots and row sums.  The longest
 //           serial chains are cut: a stack's two dihedrals run on two
 //           threads, a hydrogen bond's three on four (14.3 k -> 5.3 k cycles
-//           for one in FP64, with one reciprocal in place of five divisions);
+//           for one in FP64, with one reciprocal and corrections in place of five
+//           divisions);
 //   update  8 threads per own bead sum its slots (stored in incidence order,
 //           so the reads are contiguous and need no index), add the row sums
 //           and update v / a and x; then whole warps copy the block's new
@@ -35,8 +36,8 @@
 // A step whose lists must be rebuilt first does so from the old positions
 // between its two halves, with one more barrier.
 //
-// Every bead's sums run in an order that depends on the lane's topology
-// only, so the results do not depend on the number of CTAs.
+// Every bead's sums run in an order that depends on the lane's topology and
+// lists only, so the results do not depend on the number of CTAs.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_pipeline.h>
